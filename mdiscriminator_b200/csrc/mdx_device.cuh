@@ -56,26 +56,32 @@ struct DiscrMask {
     }
 };
 
-// class = key % m: Mod<N> (x % N).  The remainder uses the direct-remainder
-// method of Lemire, Kaser and Kurz, "Faster Remainder by Direct Computation"
-// (2019): with c = floor((2^64 - 1) / m) + 1, key % m = hi64((c * key mod 2^64) * m),
-// exact for every 32-bit key and m >= 1 (c wraps to 0 for m = 1, giving 0).
+// class = key % m: Mod<N> (x % N), by a reciprocal in 32-bit arithmetic.  With
+// c = floor((2^32 - 1) / m) the quotient estimate floor(key * c / 2^32) is the
+// quotient or one less: m * c lies in [2^32 - m, 2^32), so key * c / 2^32 falls
+// short of key / m by key * (2^32 - m * c) / (m * 2^32) <= key / 2^32 < 1.  The
+// remainder it leaves is r or r + m, and the unsigned minimum of that and that
+// minus m (which wraps when it is below m) is r.  Four instructions and no 64-bit
+// product: the 64-bit remainder it replaces (Lemire, Kaser and Kurz's direct
+// form) was most of what the count kernel executed (see plain_count_kernel).
 struct DiscrMod {
-    uint64_t c;
+    uint32_t c;
     uint32_t m;
     __host__ __device__ static DiscrMod make(uint32_t m_) {
         DiscrMod d;
         d.m = m_;
-        d.c = ~0ull / m_ + 1ull;
+        d.c = 0xffffffffu / m_;
         return d;
     }
     template <class V>
     __host__ __device__ __forceinline__ uint32_t operator()(const V& v) const {
-        const uint64_t low = c * static_cast<uint64_t>(key_of(v));
+        const uint32_t k = key_of(v);
 #ifdef __CUDA_ARCH__
-        return static_cast<uint32_t>(__umul64hi(low, static_cast<uint64_t>(m)));
+        const uint32_t r = k - __umulhi(k, c) * m;
+        return min(r, r - m);
 #else
-        return static_cast<uint32_t>((static_cast<unsigned __int128>(low) * m) >> 64);
+        const uint32_t r = k - static_cast<uint32_t>((static_cast<uint64_t>(k) * c) >> 32) * m;
+        return r < r - m ? r : r - m;
 #endif
     }
 };

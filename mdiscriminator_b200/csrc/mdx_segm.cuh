@@ -466,7 +466,7 @@ struct GroupPrefetch {
 // The discriminator of a group's segment with class count m: per-segment
 // remainders use the precomputed constants cmod[m] (DiscrMod::make).
 template <class D>
-__device__ __forceinline__ D group_discr(const SegArgs& a, const D& d, const uint64_t* cmod,
+__device__ __forceinline__ D group_discr(const SegArgs& a, const D& d, const uint32_t* cmod,
                                          uint32_t m) {
     if constexpr (std::is_same<D, DiscrMod>::value) {
         if (a.seg_m != nullptr) {
@@ -497,7 +497,7 @@ __device__ __forceinline__ D group_discr(const SegArgs& a, const D& d, const uin
 //       closed with the scanned counts plus its part in the range;
 //   P4  every element goes to head + base[class] + its rank in the segment.
 template <class V, class D, int M, int THREADS>
-__device__ void seg_group_cta(const SegArgs& a, const D& d, const uint64_t* cmod, uint32_t h,
+__device__ void seg_group_cta(const SegArgs& a, const D& d, const uint32_t* cmod, uint32_t h,
                               uint32_t he, uint64_t r0, uint32_t L, const V* src, V* dst,
                               GroupScratch<M, THREADS>& gs, GroupPrefetch& pf,
                               const uint32_t* next_h, const uint32_t* next_he) {
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(THREADS, 3)
     __shared__ GroupScratch<M, THREADS> gs;
     __shared__ uint32_t gb_h[kMaxGroupBatch], gb_he[kMaxGroupBatch];  // the batch's groups
     __shared__ uint64_t gb_r0[kMaxGroupBatch], gb_r1[kMaxGroupBatch];
-    __shared__ uint64_t cmod[17];  // DiscrMod constants for m = 1 .. 16
+    __shared__ uint32_t cmod[17];  // DiscrMod constants for m = 1 .. 16
 
     const int tid = threadIdx.x;
     const V* in = static_cast<const V*>(a.in);

@@ -9,8 +9,7 @@
 // after their own part, at the end of each phase:
 //
 //   count phase   own part [t0 + q, t1) through the CTA's TMA ring
-//                 (cp.async.bulk.tensor, 128-byte swizzle -- none for more
-//                 than 16 classes -- no multicast),
+//                 (cp.async.bulk.tensor, 128-byte swizzle, no multicast),
 //                 counted from shared memory with 4-bit packed counters; then
 //                 pool tiles by ticket (tile idx of chunk j for ticket
 //                 idx * G + j, so concurrent tiles lie far apart), each reduced
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* ring = reinterpret_cast<V*>(base);
     V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint16_t* cnt_sm = reinterpret_cast<uint16_t*>(base + L::kRingBytes + L::G::kStageBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + L::G::kStageBytes);
     // count-phase tables in the (still unused) stage: chunk reduction [W][M];
     // pool-tile counts by tile parity, M <= 16: [2][W][HW] pairs, else [2][W][M]
     uint32_t* red = reinterpret_cast<uint32_t*>(stage);
@@ -246,10 +245,7 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
             const uint32_t valid = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - ts));
             V v[ITEMS];
             if (tma_tile) {
-                // counts do not depend on the order within a tile: for more
-                // than 16 classes the tile is unswizzled and read striped
-                if constexpr (M <= 16) take_swizzled<V, ITEMS>(ring + slot * TILE, v);
-                else take_striped<V, ITEMS>(ring + slot * TILE, v);
+                take_swizzled<V, ITEMS>(ring + slot * TILE, v);
             } else {
 #pragma unroll
                 for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j < valid) ? in[ts + e0 + j] : V();
@@ -532,30 +528,22 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
         };
         const bool tma_tile = in_map(tile);
         bool done;
-        if constexpr (M <= 16) {
-            if (tma_tile) {
-                take_swizzled<V, ITEMS>(ring + slot * TILE, v);
-            } else {
-#pragma unroll
-                for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j < valid) ? in[ts + e0 + j] : V();
-            }
-            // m = 2 keeps the nibble step here: tile_filter measured 1 % slower
-            // in this kernel (N = 2^28 u32: 0.544 against 0.538 ms per call)
-            done = tile_scatter<V, D, M, THREADS, false>(d, v, 0u, valid, full, stage, cnt_sm, sh, tp,
-                                                         out, ok, refill);
+        if (tma_tile) {
+            take_swizzled<V, ITEMS>(ring + slot * TILE, v);
         } else {
-            const uint32_t w0 = static_cast<uint32_t>(tid >> 5) * 32u * ITEMS + (tid & 31);
-            if (tma_tile) {
-                take_striped<V, ITEMS>(ring + slot * TILE, v);
-            } else {
 #pragma unroll
-                for (int j = 0; j < ITEMS; j++)
-                    v[j] = (w0 + j * 32u < valid) ? in[ts + w0 + j * 32u] : V();
-            }
-            done = tile_scatter_wide<V, D, M, THREADS, false>(
-                d, v, 0u, valid, full, stage, reinterpret_cast<uint32_t*>(cnt_sm), sh, tp, out, ok,
-                refill);
+            for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j < valid) ? in[ts + e0 + j] : V();
         }
+        if constexpr (M == 2)
+            done = tile_filter<V, D, THREADS, false>(d, v, 0u, valid, full, stage, cnt_sm, sh, tp, out,
+                                                     ok, refill);
+        else if constexpr (M > 16)
+            done = tile_scatter_bytes<V, D, M, THREADS, false, false>(
+                d, v, 0u, valid, full, stage, reinterpret_cast<unsigned char*>(cnt_sm), sh, tp, out,
+                ok, refill);
+        else
+            done = tile_scatter<V, D, M, THREADS, false, false>(d, v, 0u, valid, full, stage, cnt_sm, sh, tp,
+                                                         out, ok, refill);
         if (!done) {  // a copy did not land or a chunk never got ready: nothing of this tile written
             if (tid == 0) {
                 atomicOr(a.error, kErrTimeout);

@@ -22,7 +22,13 @@ namespace host {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kMaxChunks = 4096;
-constexpr int kStages = 2;
+constexpr int kStages = 2;  // TMA ring of the one-kernel path and of the segmented run scatter
+// The plain scatter's ring has one slot: a tile is taken into registers at
+// once, so the next copy overlaps all but the take.  A second slot per CTA was
+// slower at every class count (N = 2^28 u32, 256 threads: scatter at m = 2, 8,
+// 16: 383, 370, 465 us with two slots, 346, 358, 440 with one): the reads in
+// flight beyond what covers the latency only compete with the writes.
+constexpr int kScatterStages = 1;
 constexpr size_t kHeaderBytes = 256;  // done, error, ... (see WsHeader)
 constexpr size_t kAlign = 256;
 
@@ -148,7 +154,7 @@ inline cudaError_t occupancy(const void* fn, size_t dyn_smem, int* blocks, int* 
                 return cudaSuccess;
             }
     }
-    if (dyn_smem > 48 * 1024) {
+    if (dyn_smem > 0) {  // the 48 KB a kernel has without asking hold its static part too
         err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(dyn_smem));
         if (err != cudaSuccess) return err;
@@ -188,13 +194,9 @@ inline EncodeTiledFn tensor_map_encoder() {
 }
 
 // The n elements viewed as rows of 128 bytes (n * sizeof(V) / 128 whole rows),
-// boxes of `box_rows` rows, 128-byte swizzle (thread-contiguous tile steps
-// read 16-byte chunks of every row) or none (the warp-rank step of more than
-// 16 classes reads the tile striped, one word per lane).  False if TMA
-// cannot be used (unaligned base, fewer rows than one box, encoder
-// unavailable).
-inline bool make_row_map(CUtensorMap* map, const void* base, uint64_t n, size_t elem, uint32_t box_rows,
-                         bool swizzle = true) {
+// boxes of `box_rows` rows, 128-byte swizzle.  False if TMA cannot be used
+// (unaligned base, fewer rows than one box, encoder unavailable).
+inline bool make_row_map(CUtensorMap* map, const void* base, uint64_t n, size_t elem, uint32_t box_rows) {
     std::memset(map, 0, sizeof(*map));
     if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
     const uint64_t rows = n * elem / 128;  // whole 128-byte rows
@@ -209,8 +211,7 @@ inline bool make_row_map(CUtensorMap* map, const void* base, uint64_t n, size_t 
     const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_UINT32;
     return enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE,
-               swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // ------------------------------------------------------------------ tuning --
@@ -290,14 +291,14 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     constexpr int TILE = TS * ITEMS;
     constexpr bool kBase = BPT == 64 && TS == kThreads;  // the geometry of every path
     static_assert(BPT != 64 || ITEMS == ElemCfg<V>::kItems, "64-byte tiles");
-    auto count = plain_count_kernel<V, D, M, kThreads, TILE>;
+    auto count = plain_count_kernel<V, D, M, TS, TILE>;
     const void* scatter_fn;
     size_t smem;
     {
-        using SL = ScatterTmaSmem<V, TS, kStages, M, BPT>;
+        using SL = ScatterTmaSmem<V, TS, kScatterStages, M, BPT>;
         static_assert(SL::kTile == TILE, "both kernels use the same tiles");
         scatter_fn = reinterpret_cast<const void*>(
-            plain_scatter_tma_kernel<V, D, M, TS, kStages, OutFlat<V>, BPT>);
+            plain_scatter_tma_kernel<V, D, M, TS, kScatterStages, OutFlat<V>, BPT>);
         smem = SL::kBytes;
     }
     int blocks = 0, sms = 0;
@@ -349,10 +350,10 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             // one cooperative kernel: count, grid barrier, scatter (mdx_fused.cuh)
             using SL = ScatterTmaSmem<V, kThreads, kStages, M>;
             CUtensorMap map;
-            if (make_row_map(&map, d_in, n, sizeof(V), SL::kRows, M <= 16)) {
+            if (make_row_map(&map, d_in, n, sizeof(V), SL::kRows)) {
                 auto fused = plain_fused_kernel<V, D, M, kThreads, kStages>;
                 int fb = 0, fs = 0;
-                if (occupancy(reinterpret_cast<const void*>(fused), smem, &fb, &fs) != cudaSuccess)
+                if (occupancy(reinterpret_cast<const void*>(fused), SL::kBytes, &fb, &fs) != cudaSuccess)
                     return MDX_ERR_CUDA;
                 if (tun.plain_ctas_per_sm > 0 && static_cast<int>(tun.plain_ctas_per_sm) < fb)
                     fb = static_cast<int>(tun.plain_ctas_per_sm);
@@ -392,7 +393,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(FG);
                 cfg.blockDim = dim3(kThreads);
-                cfg.dynamicSmemBytes = smem;
+                cfg.dynamicSmemBytes = SL::kBytes;
                 cfg.stream = stream;
                 cudaLaunchAttribute attr[1];
                 attr[0].id = cudaLaunchAttributeCooperative;
@@ -410,19 +411,19 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
         if (d_headflags != nullptr &&
             cudaMemsetAsync(d_headflags, 0, n * sizeof(uint32_t), stream) != cudaSuccess)
             return MDX_ERR_CUDA;
-        count<<<G, kThreads, 0, stream>>>(a, d);
+        count<<<G, TS, 0, stream>>>(a, d);
         if (ev_mid != nullptr && cudaEventRecord(ev_mid, stream) != cudaSuccess) return MDX_ERR_CUDA;
     }
     if (step == PlainStep::kCount) return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
     {
-        using SL = ScatterTmaSmem<V, TS, kStages, M, BPT>;
+        using SL = ScatterTmaSmem<V, TS, kScatterStages, M, BPT>;
         CUtensorMap map;
-        a.use_tma = make_row_map(&map, d_in, n, sizeof(V), SL::kRows, M <= 16) ? 1 : 0;
+        a.use_tma = make_row_map(&map, d_in, n, sizeof(V), SL::kRows) ? 1 : 0;
         if (dist == nullptr) {
             const OutFlat<V> o{static_cast<V*>(d_out),
                                static_cast<uint32_t>((reinterpret_cast<uintptr_t>(d_out) / sizeof(V)) &
                                                      (16u / sizeof(V) - 1u))};
-            auto scatter = plain_scatter_tma_kernel<V, D, M, TS, kStages, OutFlat<V>, BPT>;
+            auto scatter = plain_scatter_tma_kernel<V, D, M, TS, kScatterStages, OutFlat<V>, BPT>;
             if (step == PlainStep::kBoth && ev_mid == nullptr) {
                 // programmatic dependent launch: scheduled while the count grid
                 // drains, it starts its first tile copies before waiting for it
@@ -448,7 +449,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             // chunks of both steps must match)
             int b2 = 0, s2 = 0;
             if (occupancy(reinterpret_cast<const void*>(
-                              plain_scatter_tma_kernel<V, D, M, kThreads, kStages, OutSharded<V>>),
+                              plain_scatter_tma_kernel<V, D, M, kThreads, kScatterStages, OutSharded<V>>),
                           smem, &b2, &s2) != cudaSuccess)
                 return MDX_ERR_CUDA;
             uint32_t* skip = reinterpret_cast<uint32_t*>(ws + kDistSkipOffset);
@@ -461,7 +462,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             for (uint32_t q = dist->R; q < static_cast<uint32_t>(kMaxRanks); q++) o.chunks[q] = nullptr;
             o.chunk = static_cast<uint32_t>(dist->chunk);
             o.R = dist->R;
-            plain_scatter_tma_kernel<V, D, M, kThreads, kStages, OutSharded<V>>
+            plain_scatter_tma_kernel<V, D, M, kThreads, kScatterStages, OutSharded<V>>
                 <<<G, kThreads, smem, stream>>>(a, d, map, o);
         }
     }
@@ -476,12 +477,9 @@ mdx_status run_plain(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
     if constexpr (sizeof(V) <= 8) {
         const Tuning tun = tuning_for(sizeof(V) == 8 ? MDX_ELEM_REC8 : MDX_ELEM_U32, M, n);
         if (dist == nullptr && step == PlainStep::kBoth) {
-            if constexpr (M <= 16) {  // the warp-rank step spills at 512 threads
-                if (tun.tile_threads == 512)
-                    return run_plain_g<V, D, M, 64, 512>(d_in, d_out, n, d, m, d_sizes, d_headflags,
-                                                         ws, L, stream, ev_mid, step, dist,
-                                                         allow_fused);
-            }
+            if (tun.tile_threads == 512)
+                return run_plain_g<V, D, M, 64, 512>(d_in, d_out, n, d, m, d_sizes, d_headflags, ws,
+                                                     L, stream, ev_mid, step, dist, allow_fused);
             if (tun.tile_bytes == 32)
                 return run_plain_g<V, D, M, 32, kThreads>(d_in, d_out, n, d, m, d_sizes,
                                                           d_headflags, ws, L, stream, ev_mid, step,

@@ -46,7 +46,7 @@ namespace noalloc {
 
 constexpr size_t kNoAllocScratchBytes = 525312;  // 2052 * 256
 constexpr int kThreadsN = 256;
-constexpr int kStagesN = 2;
+constexpr int kStagesN = 1;
 constexpr uint32_t kMaxChunksN = 4096;
 constexpr size_t kHeaderN = 256;
 constexpr int kMaxDevices = 64;
@@ -85,7 +85,7 @@ cudaError_t occupancy_n(const void* fn, size_t smem, int* blocks, int* sms) {
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(g_mu);
     if (s_blocks[dev] == 0) {
-        if (smem > 48 * 1024) {
+        if (smem > 0) {
             err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
             if (err != cudaSuccess) return err;

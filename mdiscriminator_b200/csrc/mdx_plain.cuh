@@ -14,10 +14,9 @@
 //                        `offsets` of SeqMdiscr.h:34-38) and the class sizes.
 //   plain_scatter_tma_kernel
 //                        re-reads each element (4 B) and writes it once (4 B):
-//                        per tile, element ranks (m <= 16: thread-local
-//                        nibble counters and a block scan, mdx_tile.cuh
-//                        tile_scatter; more classes: warp ranks from ballots
-//                        of the class bits + __popc, tile_scatter_wide), a
+//                        per tile, element ranks (mdx_tile.cuh: thread-private
+//                        counters, in registers for m <= 16 and in shared
+//                        memory above, and a block scan), a
 //                        shared-memory staged scatter so every class run
 //                        leaves the SM as bulk stores.  Tiles are staged into
 //                        shared memory by TMA (cp.async.bulk.tensor, no
@@ -216,7 +215,7 @@ __device__ void plain_finish_scan(const PlainArgs& a, uint32_t* tot_sh) {
 }
 
 template <class V, class D, int M, int THREADS, int TILE>
-__global__ void __launch_bounds__(THREADS, 4) plain_count_kernel(PlainArgs a, D d) {
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(PlainArgs a, D d) {
     constexpr int W = THREADS / 32;
     constexpr int VEC = 16 / static_cast<int>(sizeof(V));
     constexpr int UNROLL = M <= 8 ? 8 : 4;  // 16-byte loads in flight per thread (registers allowing)
@@ -344,14 +343,17 @@ struct ScatterTmaSmem {
 // Scatter kernel: CTA k re-reads chunk k (tiles in reverse order) and writes
 // every element at class_base[c] + chunk_pre[c][k] + its rank in the chunk.
 // Tiles arrive by tensor TMA (one 2-D box of 128-byte rows per tile, 128-byte
-// swizzle for m <= 16 and none above, STAGES-deep mbarrier ring) and go
-// through tile_filter (m = 2), tile_scatter (m <= 16:
-// thread-local nibble ranks, a block scan over the [class][thread] count
-// matrix) or tile_scatter_wide (17..64 classes: warp ranks from ballots),
+// swizzle, STAGES-deep mbarrier ring) and go through tile_filter (m = 2),
+// tile_scatter (m <= 16) or tile_scatter_bytes (17..64 classes),
 // then a shared-memory stage at the destination's 16-byte phase and bulk
 // stores of every class run (mdx_tile.cuh).  OUT: one output array, or the
 // output chunks of several ranks (distributed partition).  BPT: bytes of a
-// tile per thread (64, or 32 for tiles half as long).
+// tile per thread (64, or 32 for tiles half as long).  Two CTAs of 512 threads
+// beat four of 256 for large inputs at every class count: the class runs of a
+// tile are twice as long, so the bulk stores are half as many and the block scan
+// is shared by twice the elements (N = 2^28 u32, m = 2, 4, 8, 16, 64: scatter
+// 346, 359, 367, 404, 707 us with 256 threads, 335, 343, 353, 391, 597 with 512;
+// a device copy of the same bytes takes 337).
 template <class V, class D, int M, int THREADS, int STAGES, class OUT = OutFlat<V>, int BPT = 64>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: <= 64 registers
     plain_scatter_tma_kernel(PlainArgs a, D d, const __grid_constant__ CUtensorMap tmap,
@@ -367,11 +369,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* ring = reinterpret_cast<V*>(base);
     V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint16_t* cnt_sm = reinterpret_cast<uint16_t*>(base + L::kRingBytes + L::G::kStageBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + L::G::kStageBytes);
 
     __shared__ __align__(8) uint64_t bars[STAGES];
     __shared__ TileShared<M> sh;
     __shared__ uint32_t tot_sh[M], pre_sh[M];
+    __shared__ int clustered_sh;  // two classes hold nearly all of this chunk
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t G = a.num_chunks, k = blockIdx.x;
@@ -389,6 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
 #pragma unroll
         for (int s = 0; s < STAGES; s++) mbar_init(&bars[s], 1);
         mbar_fence_init();
+        clustered_sh = 0;
     }
     if (tid < M) {
         tot_sh[tid] = 0u;
@@ -444,7 +448,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
         }
         __syncthreads();
         if (warp == 0) {  // class bases: exclusive scan of the totals
-            uint32_t carry = 0;
+            uint32_t carry = 0, sum = 0, max1 = 0, max2 = 0;
 #pragma unroll
             for (int h = 0; h < (M + 31) / 32; h++) {
                 const uint32_t cc = static_cast<uint32_t>(lane + 32 * h);
@@ -452,7 +456,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
                 const uint32_t incl = warp_incl_scan(x);
                 const uint32_t bc = carry + incl - x;
                 if (cc < static_cast<uint32_t>(M)) {
-                    sh.cursor[0][cc] = bc + pre_sh[cc] + __ldcg(a.chunk_cnt + static_cast<uint64_t>(cc) * stride + k);
+                    const uint32_t own = __ldcg(a.chunk_cnt + static_cast<uint64_t>(cc) * stride + k);
+                    sh.cursor[0][cc] = bc + pre_sh[cc] + own;
+                    sum += own;
+                    max2 = max(max2, min(max1, own));
+                    max1 = max(max1, own);
                     if (k == 0) {
                         a.class_base[cc] = bc;
                         a.class_tot[cc] = x;
@@ -463,6 +471,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
                 }
                 carry += __shfl_sync(0xffffffffu, incl, 31);
             }
+            if constexpr (M > 2) {
+                const uint32_t all = __reduce_add_sync(0xffffffffu, sum);
+                const uint32_t top = __reduce_max_sync(0xffffffffu, max1);
+                const uint32_t at = __ballot_sync(0xffffffffu, max1 == top);
+                const uint32_t rest = lane == __ffs(at) - 1 ? max2 : max1;
+                const uint32_t second = __reduce_max_sync(0xffffffffu, rest);
+                if (lane == 0) clustered_sh = all - top - second <= all / 8u;
+            }
         }
     } else if (tid < M) {
         const uint64_t o = static_cast<uint64_t>(tid) * stride + k;
@@ -471,19 +487,20 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     __syncthreads();
 
     const uint32_t e0 = tid * ITEMS;
-    for (uint32_t i = 0; i < cnt; i++) {
-        const uint32_t tile = t1 - 1u - i;
-        const uint64_t ts = static_cast<uint64_t>(tile) * TILE;
-        const uint32_t valid = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - ts));
-        const bool full = valid == TILE;
-        const bool ok = mbar_wait_bounded(&bars[i % STAGES], (i / STAGES) & 1u);
-        V v[ITEMS];
-        // the ring slot is consumed (values are in registers): refill it
-        auto refill = [&] {
-            if (tid == 0 && i + STAGES < cnt) issue(i + STAGES);
-        };
-        bool done;
-        if constexpr (M <= 16) {  // thread-contiguous elements
+    auto place_tiles = [&](auto clustered) {
+        constexpr bool CLUSTERED = decltype(clustered)::value;
+        for (uint32_t i = 0; i < cnt; i++) {
+            const uint32_t tile = t1 - 1u - i;
+            const uint64_t ts = static_cast<uint64_t>(tile) * TILE;
+            const uint32_t valid = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - ts));
+            const bool full = valid == TILE;
+            const bool ok = mbar_wait_bounded(&bars[i % STAGES], (i / STAGES) & 1u);
+            V v[ITEMS];
+            // the ring slot is consumed (values are in registers): refill it
+            auto refill = [&] {
+                if (tid == 0 && i + STAGES < cnt) issue(i + STAGES);
+            };
+            bool done;
             if (tma_ok && full) {
                 take_swizzled<V, ITEMS>(ring + (i % STAGES) * TILE, v);
             } else if (full) {
@@ -494,33 +511,33 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
                 for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j < valid) ? in[ts + e0 + j] : V();
             }
             if constexpr (M == 2)
-                done = tile_filter<V, D, THREADS, false>(d, v, 0u, valid, full, stage,
-                                                         reinterpret_cast<uint32_t*>(cnt_sm), sh,
-                                                         i & 1u, out, ok, refill);
+                done = tile_filter<V, D, THREADS, false>(d, v, 0u, valid, full, stage, cnt_sm, sh, i & 1u,
+                                                         out, ok, refill);
+            else if constexpr (M > 16)
+                done = tile_scatter_bytes<V, D, M, THREADS, false, CLUSTERED>(
+                    d, v, 0u, valid, full, stage, reinterpret_cast<unsigned char*>(cnt_sm), sh, i & 1u,
+                    out, ok, refill);
             else
-                done = tile_scatter<V, D, M, THREADS, false>(d, v, 0u, valid, full, stage, cnt_sm,
-                                                             sh, i & 1u, out, ok, refill);
-        } else {  // striped elements (warp ranks)
-            const uint32_t w0 = static_cast<uint32_t>(tid >> 5) * 32u * ITEMS + (tid & 31);
-            if (tma_ok && full) {
-                take_striped<V, ITEMS>(ring + (i % STAGES) * TILE, v);
-            } else {
-#pragma unroll
-                for (int j = 0; j < ITEMS; j++)
-                    v[j] = (w0 + j * 32u < valid) ? in[ts + w0 + j * 32u] : V();
+                done = tile_scatter<V, D, M, THREADS, false, CLUSTERED>(d, v, 0u, valid, full, stage, cnt_sm, sh,
+                                                             i & 1u, out, ok, refill);
+            if (!done) {
+                if (tid == 0) {
+                    atomicOr(a.error, kErrTimeout);
+                    for (uint32_t q = i; q < cnt && q < i + STAGES; q++)
+                        (void)mbar_wait_bounded(&bars[q % STAGES], (q / STAGES) & 1u);
+                }
+                break;
             }
-            done = tile_scatter_wide<V, D, M, THREADS, false>(
-                d, v, 0u, valid, full, stage, reinterpret_cast<uint32_t*>(cnt_sm), sh, i & 1u, out,
-                ok, refill);
         }
-        if (!done) {
-            if (tid == 0) {
-                atomicOr(a.error, kErrTimeout);
-                for (uint32_t q = i; q < cnt && q < i + STAGES; q++)
-                    (void)mbar_wait_bounded(&bars[q % STAGES], (q / STAGES) & 1u);
-            }
-            break;
-        }
+    };
+    // Sorted or clustered input (two classes hold 7/8 of the chunk): the tile
+    // step that also looks for warps of one class, a loop of its own because the
+    // look alone costs the other chunks 2 to 5 % of the scatter.
+    if constexpr (M > 2 && std::is_same<OUT, OutFlat<V>>::value) {
+        if (clustered_sh) place_tiles(std::true_type{});
+        else place_tiles(std::false_type{});
+    } else {
+        place_tiles(std::false_type{});
     }
     if (tid < M) bulk_wait_all();
     if constexpr (!std::is_same<OUT, OutFlat<V>>::value) {

@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* ring = reinterpret_cast<V*>(base);
     V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint16_t* cnt_sm = reinterpret_cast<uint16_t*>(base + L::kRingBytes + TG::kStageBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + TG::kStageBytes);
 
     __shared__ __align__(8) uint64_t bars[STAGES];
     __shared__ TileShared<M> sh;
@@ -1130,10 +1130,17 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
                 for (int q = 0; q < ITEMS; q++)
                     v[q] = (e0 + q >= lo && e0 + q < hi) ? in[ts + e0 + q] : V();
             }
-            const bool done = tile_scatter<V, D, M, THREADS, true>(
-                dj, v, lo, hi, full, stage, cnt_sm, sh, i & 1u, OutFlat<V>{out, out_phase}, ok, [&] {
-                    if (tid == 0 && i + STAGES < ntiles) issue(i + STAGES);
-                });
+            auto refill = [&] {
+                if (tid == 0 && i + STAGES < ntiles) issue(i + STAGES);
+            };
+            bool done;
+            if constexpr (M == 2)
+                done = tile_filter<V, D, THREADS, true>(dj, v, lo, hi, full, stage, cnt_sm, sh, i & 1u,
+                                                        OutFlat<V>{out, out_phase}, ok, refill);
+            else
+                done = tile_scatter<V, D, M, THREADS, true, false>(dj, v, lo, hi, full, stage, cnt_sm, sh,
+                                                            i & 1u, OutFlat<V>{out, out_phase}, ok,
+                                                            refill);
             if (!done) {
                 failed = true;
                 if (tid == 0) {
@@ -1201,7 +1208,7 @@ __global__ void __launch_bounds__(THREADS, 4)
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* slab = reinterpret_cast<V*>(base);
     V* stage = reinterpret_cast<V*>(base + L::kSlabBytes);
-    uint16_t* cnt_sm = reinterpret_cast<uint16_t*>(base + L::kSlabBytes + TG::kStageBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kSlabBytes + TG::kStageBytes);
 
     __shared__ __align__(8) uint64_t bars[KMAX];
     __shared__ TileShared<M> sh;
@@ -1364,11 +1371,16 @@ __global__ void __launch_bounds__(THREADS, 4)
             const bool full = lo == 0u && hi == static_cast<uint32_t>(P);
             V v[ITEMS];
             take(cur, i, lo, hi, v);
-            (void)tile_scatter<V, D, M, THREADS, true>(
-                dj, v, lo, hi, full, stage, cnt_sm, sh, i & 1u, OutFlat<V>{out, out_phase}, true,
-                [&] {
-                    if (tid == 0 && has_next && i < nxt.ntiles) issue(nxt, i);
-                });
+            auto refill = [&] {
+                if (tid == 0 && has_next && i < nxt.ntiles) issue(nxt, i);
+            };
+            if constexpr (M == 2)
+                (void)tile_filter<V, D, THREADS, true>(dj, v, lo, hi, full, stage, cnt_sm, sh, i & 1u,
+                                                       OutFlat<V>{out, out_phase}, true, refill);
+            else
+                (void)tile_scatter<V, D, M, THREADS, true, false>(dj, v, lo, hi, full, stage, cnt_sm, sh,
+                                                           i & 1u, OutFlat<V>{out, out_phase}, true,
+                                                           refill);
         }
         cur = nxt;
         s_next = s_after;

@@ -4,15 +4,18 @@
 // A tile is THREADS * ITEMS elements (BPT = 64 or 32 contiguous bytes per
 // thread: two tile geometries, chosen per call by the tuning table).  For
 // the elements of tile-local range [lo, hi):
-//  * pass 1: each thread ranks its own consecutive elements with 4-bit
-//    counters in a register (local rank = number of its earlier elements of
-//    the same class; the 16th element is kept aside so no lane can reach 16)
-//    and publishes its per-class counts to a [class][thread] u16 matrix;
-//  * row scans: warp w < m/2 scans rows w and w + m/2 of the matrix at once,
-//    packed in u16 pairs (exclusive prefix over threads = stable order); those
-//    warps derive the tile's class runs (lanes = classes) and fold each run's
-//    stage slot into their rows;
-//  * pass 2: element -> stage slot = row prefix + local rank;
+//  * pass 1: each thread counts its own consecutive elements per class with
+//    4-bit counters in a register (the 16th element is kept aside so no lane can
+//    reach 16) and publishes the counts to a matrix of 16-bit pairs;
+//  * row scans: warp w < m/2 scans word row w of the matrix, two classes at once
+//    (exclusive prefix over threads = stable order); those warps derive the
+//    tile's class runs (lanes = classes) and fold each run's stage slot into
+//    their rows;
+//  * pass 2: element -> stage slot = row prefix + local rank; m < 16 keeps the
+//    ranks of pass 1 in registers, m = 16 lets the thread's entry of the matrix
+//    move on with every element (a 64-bit shift less per element, against a
+//    store: N = 2^28 u32, 512 threads: scatter 391 against 444 us, but 383
+//    against 353 at m = 8, where the shifts are cheap and the chain is not);
 //  * write-out: each class run sits in the stage at the same 16-byte phase as
 //    its destination, so its aligned interior leaves by one bulk store
 //    (cp.async.bulk shared -> global) and threads store the < 16-byte head and
@@ -81,10 +84,12 @@ struct TileGeom {
     // every class run gets kAU slots of slack for its 16-byte phase
     static constexpr int kStageElems = kTile + static_cast<int>(kAU) * M;
     static constexpr size_t kStageBytes = static_cast<size_t>(kStageElems) * sizeof(V);
-    // m <= 16: [class][thread] u16 counts; more classes: [warp][class] u32
-    // counts, then stage bases (tile_scatter_wide)
-    static constexpr size_t kCntBytes = M <= 16 ? static_cast<size_t>(M) * THREADS * 2
-                                                : static_cast<size_t>(THREADS / 32) * M * 4;
+    // m <= 16: [class pair][thread] words of two 16-bit counts; more classes:
+    // [class / 4][thread] words of four byte counts and a table of up to 32 rows
+    // (tile_scatter_bytes)
+    static constexpr size_t kCntBytes = M > 16
+                                            ? static_cast<size_t>(M) * THREADS + 32 * (M + 4) * 2
+                                            : static_cast<size_t>(M) * THREADS * 2;
     static_assert(kStageElems < 65536, "stage slots are kept in 16 bits");
 };
 
@@ -92,7 +97,8 @@ struct TileGeom {
 template <int M>
 struct TileShared {
     uint32_t cursor[2][M];  // ping-pong by tile parity
-    uint32_t run_start[M], run_cnt[M], run_dst[M], rowtot[M];
+    uint32_t run_start[M], run_cnt[M], run_dst[M];
+    alignas(16) uint32_t rowtot[M];
 };
 
 // Where a tile's class runs go.  `idx` is an element's position in the whole
@@ -155,88 +161,181 @@ __device__ __forceinline__ void take_swizzled(const V* tile, V (&v)[ITEMS]) {
     }
 }
 
+// A warp whose elements all belong to one class (sorted or clustered input)
+// fills 32 * ITEMS consecutive stage slots from `run` on, ITEMS from each lane.
+// Stored lane by lane, the lanes would be ITEMS slots apart and hit two banks in
+// all; so each lane stores its slots in an order of its own (slot j ^ lane / 2),
+// which spreads a store over the banks, and the warp then puts the slots of
+// every 32 in order.  Three conflict-free accesses an element instead of one that
+// is repeated for each of 16 lanes (4-byte elements) of a bank: N = 2^28 u32
+// sorted by class, scatter at m = 2, 8, 16: 601, 652, 733 us before, 333, 349,
+// 365 with it.
+template <class V, int ITEMS>
+__device__ __forceinline__ void place_warp_run(V* run, const V (&v)[ITEMS]) {
+    const uint32_t lane = threadIdx.x & 31u;
+    constexpr uint32_t I = ITEMS;
+#pragma unroll
+    for (uint32_t j = 0; j < I; j++) run[I * lane + (j ^ ((lane >> 1) & (I - 1u)))] = v[j];
+    __syncwarp();
+#pragma unroll 4
+    for (uint32_t k = 0; k < I; k++) {  // slots 32 k ..: in order; they stay among themselves
+        const uint32_t l = 32u / I * k + lane / I;  // the lane slot 32 k + lane came from
+        const V x = run[I * l + ((lane % I) ^ ((l >> 1) & (I - 1u)))];
+        __syncwarp();
+        run[32u * k + lane] = x;
+    }
+}
+
+// Whether the warp's lanes all have `one` (their elements share a class) and the
+// same class c.
+__device__ __forceinline__ bool warp_of_one_class(bool one, uint32_t c) {
+    const uint32_t c0 = __shfl_sync(0xffffffffu, c, 0);  // by every lane, whatever `one` says
+    return __all_sync(0xffffffffu, one && c == c0);
+}
+
+// Count matrix of the nibble step: a 32-bit word holds the 16-bit counts of two
+// classes and a row one word of every thread, so a warp's words of a row lie in
+// 32 banks whatever classes its lanes look up (16-bit entries side by side put
+// two threads in a bank and cost two wavefronts a lookup).  Thread t = PER g +
+// 4 h + i (PER = threads a scan lane takes) has column 128 h + ((4 g + i) ^ X h):
+// a scan lane's PER words are then 16-byte loads that are consecutive over the
+// lanes.
+template <int THREADS>
+struct CountColumns {
+    static constexpr uint32_t kPer = THREADS / 32;
+    static constexpr uint32_t kX = 128u / kPer;  // 32 banks over the kPer / 4 loads
+    static_assert(kPer == 8 || kPer == 16, "row scans load 8 or 16 words per lane");
+    static __device__ __forceinline__ uint32_t column(uint32_t t) {
+        const uint32_t g = t / kPer, h = (t / 4u) % (kPer / 4u), i = t % 4u;
+        return 128u * h + ((4u * g + i) ^ (kX * h));
+    }
+    // first word of scan lane l's load h
+    static __device__ __forceinline__ uint32_t chunk(uint32_t l, uint32_t h) {
+        return 128u * h + ((4u * l) ^ (kX * h));
+    }
+};
+
+// Per-thread class counts of the nibble step and where class c's 16-bit count
+// lies: classes k and k + M / 2 share word k.
+template <int M>
+struct ThreadCounts {
+    static_assert(M == 4 || M == 8 || M == 16, "class bound");
+    static constexpr int kRows = M / 2;
+    static constexpr uint32_t kHalf = M / 2;
+    // four classes: 8-bit counters, which hold the 16th element too
+    static constexpr bool kNibbles = M > 4;
+    uint32_t w[2];
+    __device__ __forceinline__ void init() { w[0] = w[1] = 0; }
+    __device__ __forceinline__ uint32_t get(uint32_t c) const {
+        if constexpr (M == 4) return (w[0] >> (c << 3)) & 0xffu;
+        else if constexpr (M == 8) return (w[0] >> (c << 2)) & 15u;
+        else return static_cast<uint32_t>(((static_cast<uint64_t>(w[1]) << 32) | w[0]) >> (c << 2)) & 15u;
+    }
+    __device__ __forceinline__ void inc(uint32_t c) {
+        if constexpr (M == 4) {
+            w[0] += 1u << (c << 3);
+        } else if constexpr (M == 8) {
+            w[0] += 1u << (c << 2);
+        } else {  // sixteen nibbles: one 64-bit shift
+            uint64_t x = (static_cast<uint64_t>(w[1]) << 32) | w[0];
+            x += 1ull << (c << 2);
+            w[0] = static_cast<uint32_t>(x);
+            w[1] = static_cast<uint32_t>(x >> 32);
+        }
+    }
+    // the counts of classes r (low half) and r + M / 2
+    __device__ __forceinline__ uint32_t word(int r) const {
+        if constexpr (M == 4) return (w[0] >> (8 * r)) & 0x00ff00ffu;
+        else if constexpr (M == 8) return (w[0] >> (4 * r)) & 0x000f000fu;
+        else return (__byte_perm(w[0], w[1], r < 4 ? 0x5410 : 0x7632) >> (4 * (r & 3))) & 0x000f000fu;
+    }
+    // byte offset of class c's count from the thread's column
+    template <int THREADS>
+    static __device__ __forceinline__ uint32_t offset(uint32_t c) {
+        constexpr uint32_t kRow = 4u * THREADS;
+        return c * kRow - c / kHalf * (kHalf * kRow - 2u);
+    }
+};
+
 // One tile: see the file comment.  `full` means lo == 0 and hi == TILE (no
 // bounds checks).  FORWARD: run c of this tile starts at cursor[par][c] and
 // the cursor advances; otherwise it ends there and the cursor moves back.
 // `after_counts` runs right after the first barrier (the input ring slot is
 // consumed by then).  Returns false, having written nothing, when `ok` is
 // false on any thread.
-template <class V, class D, int M, int THREADS, bool FORWARD, class OUT, class AfterCounts,
-          int ITEMS>
+template <class V, class D, int M, int THREADS, bool FORWARD, bool CLUSTERED, class OUT,
+          class AfterCounts, int ITEMS>
 __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], uint32_t lo,
-                                             uint32_t hi, bool full, V* stage, uint16_t* cnt_sm,
+                                             uint32_t hi, bool full, V* stage, uint32_t* cnt_sm,
                                              TileShared<M>& sh, uint32_t par, const OUT& out,
                                              bool ok, AfterCounts after_counts) {
     using G = TileGeom<V, THREADS, M, ITEMS * static_cast<int>(sizeof(V))>;
     static_assert(G::kItems == ITEMS, "geometry");
+    using CC = CountColumns<THREADS>;
+    using TC = ThreadCounts<M>;
     constexpr uint32_t AU = G::kAU;
     constexpr int W = THREADS / 32;
-    constexpr int PER = THREADS / 32;
-    constexpr int LR = (ITEMS + 7) / 8;
-    static_assert(M <= 16 && M >= 2, "class bound");
-    static_assert(M <= 2 * W, "each warp scans at most two rows");
-    static_assert((M & (M - 1)) == 0, "rows paired as w and w + M/2");
+    constexpr int PER = static_cast<int>(CC::kPer);
+    static_assert(TC::kRows <= W, "a warp per row");
     static_assert(ITEMS == 16 || ITEMS == 8 || ITEMS == 4 || ITEMS == 2, "thread elements");
-    static_assert(PER == 8 || PER == 16, "row scans load 8 or 16 entries per lane");
+    // a nibble holds 15: the 16th element is kept out of them
+    constexpr int kIn = TC::kNibbles && ITEMS > 15 ? 15 : ITEMS;
+    constexpr bool kRanks = M < 16;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t e0 = tid * ITEMS;
-    uint16_t* my_cnt = cnt_sm + tid;  // this thread's column: my_cnt[c * THREADS]
+    unsigned char* my_cnt = reinterpret_cast<unsigned char*>(cnt_sm + CC::column(tid));
+    auto count_at = [&](uint32_t c) -> uint16_t& {
+        return *reinterpret_cast<uint16_t*>(my_cnt + TC::template offset<THREADS>(c));
+    };
 
     // ---- pass 1
-    NibbleCounts<M> nc;
-    nc.init();
-    uint32_t lr[LR];
+    TC tc;
+    tc.init();
+    uint32_t last_c = M;  // class of the element kept out of the nibbles
+    uint32_t lr[kRanks ? (ITEMS + 7) / 8 : 1];  // local ranks, four bits each
+    if constexpr (kRanks) {
 #pragma unroll
-    for (int q = 0; q < LR; q++) lr[q] = 0;
-    uint32_t last_c = M;  // class of element 15 (kept out of the nibbles)
+        for (int q = 0; q < (ITEMS + 7) / 8; q++) lr[q] = 0;
+    }
+    auto count = [&](int j) {
+        const uint32_t c = d(v[j]);
+        if constexpr (kRanks) lr[j >> 3] += tc.get(c) << (4 * (j & 7));
+        if (j < kIn) tc.inc(c); else last_c = c;
+    };
     if (full) {
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            const uint32_t c = d(v[j]);
-            lr[j >> 3] += nc.get(c) << (4 * (j & 7));
-            if (j < 15) nc.inc(c); else last_c = c;
-        }
+        for (int j = 0; j < ITEMS; j++) count(j);
     } else {
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            if (e0 + j >= lo && e0 + j < hi) {
-                const uint32_t c = d(v[j]);
-                lr[j >> 3] += nc.get(c) << (4 * (j & 7));
-                if (j < 15) nc.inc(c); else last_c = c;
-            }
-        }
+        for (int j = 0; j < ITEMS; j++)
+            if (e0 + j >= lo && e0 + j < hi) count(j);
     }
+    const uint32_t c_last = d(v[ITEMS - 1]);
+    bool one_class = false;  // the warp's elements
+    if constexpr (CLUSTERED) one_class = full && warp_of_one_class(tc.get(c_last) == kIn, c_last);
 #pragma unroll
-    for (int c = 0; c < M; c++) my_cnt[c * THREADS] = static_cast<uint16_t>(nc.get(c));
-    if (last_c < static_cast<uint32_t>(M)) my_cnt[last_c * THREADS] += 1;
+    for (int r = 0; r < TC::kRows; r++)
+        *reinterpret_cast<uint32_t*>(my_cnt + r * 4 * THREADS) = tc.word(r);
+    if constexpr (kIn < ITEMS)
+        if (last_c < static_cast<uint32_t>(M)) count_at(last_c) += 1;
     if (__syncthreads_or(!ok)) return false;  // (A)
     after_counts();
 
-    // ---- row scans: warp w < M/2 scans rows w and w + M/2 at once, the two
-    // rows' u16 counts packed in one word (row w low, row w + M/2 high; a
-    // row's sum is at most the tile, < 2^16); the other warps idle here.  A
-    // lane holds PER consecutive threads' entries (8 at 256 threads, 16 at 512)
-    constexpr int H = M / 2;
-    constexpr int NV = PER / 8;  // 16-byte loads per row and lane
-    const bool scans = warp < H;
+    // ---- row scans: warp w < M/2 scans row w, two classes at once (a class's
+    // sum is at most the tile, < 2^16); the other warps idle here
+    const bool scans = warp < TC::kRows;
+    uint32_t* row = cnt_sm + warp * THREADS;
     uint32_t pre[PER];  // packed exclusive prefixes of this lane's threads
     if (scans) {
         uint32_t x[PER];
 #pragma unroll
-        for (int u = 0; u < NV; u++) {
-            const uint4 xa =
-                *reinterpret_cast<const uint4*>(cnt_sm + warp * THREADS + lane * PER + 8 * u);
-            const uint4 xb =
-                *reinterpret_cast<const uint4*>(cnt_sm + (warp + H) * THREADS + lane * PER + 8 * u);
-            x[8 * u + 0] = __byte_perm(xa.x, xb.x, 0x5410);
-            x[8 * u + 1] = __byte_perm(xa.x, xb.x, 0x7632);
-            x[8 * u + 2] = __byte_perm(xa.y, xb.y, 0x5410);
-            x[8 * u + 3] = __byte_perm(xa.y, xb.y, 0x7632);
-            x[8 * u + 4] = __byte_perm(xa.z, xb.z, 0x5410);
-            x[8 * u + 5] = __byte_perm(xa.z, xb.z, 0x7632);
-            x[8 * u + 6] = __byte_perm(xa.w, xb.w, 0x5410);
-            x[8 * u + 7] = __byte_perm(xa.w, xb.w, 0x7632);
+        for (int u = 0; u < PER / 4; u++) {
+            const uint4 a = *reinterpret_cast<const uint4*>(row + CC::chunk(lane, u));
+            x[4 * u + 0] = a.x;
+            x[4 * u + 1] = a.y;
+            x[4 * u + 2] = a.z;
+            x[4 * u + 3] = a.w;
         }
         uint32_t tot = 0;
 #pragma unroll
@@ -250,14 +349,14 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
         }
         if (lane == 31) {
             sh.rowtot[warp] = incl & 0xffffu;
-            sh.rowtot[warp + H] = incl >> 16;
+            sh.rowtot[warp + TC::kHalf] = incl >> 16;
         }
     }
     __syncthreads();  // (B)
 
     // ---- class runs (the scanning warps, lanes = classes): destination of
     // run c and its stage slot, at the destination's 16-byte phase within kAU
-    // slots of slack per run; each scanning warp folds the slots into its rows
+    // slots of slack per run; each scanning warp folds the slots into its row
     if (scans) {
         const uint32_t c = static_cast<uint32_t>(lane);
         const bool cls = c < static_cast<uint32_t>(M);
@@ -267,21 +366,14 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
         const uint32_t room = cc + (cls ? AU : 0u);
         const uint32_t q0 = warp_incl_scan(room) - room;
         const uint32_t st = q0 + (((out.phase() + dst) - q0) & (AU - 1u));
-        // slots < kStageElems < 2^16: the two rows' slots stay packed
+        // slots < kStageElems < 2^16: the two classes' slots stay packed
         const uint32_t add = __shfl_sync(0xffffffffu, st, warp) |
-                             (__shfl_sync(0xffffffffu, st, warp + H) << 16);
+                             (__shfl_sync(0xffffffffu, st, warp + TC::kHalf) << 16);
 #pragma unroll
-        for (int u = 0; u < NV; u++) {
-            uint32_t p[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) p[q] = pre[8 * u + q] + add;
-            *reinterpret_cast<uint4*>(cnt_sm + warp * THREADS + lane * PER + 8 * u) =
-                make_uint4(__byte_perm(p[0], p[1], 0x5410), __byte_perm(p[2], p[3], 0x5410),
-                           __byte_perm(p[4], p[5], 0x5410), __byte_perm(p[6], p[7], 0x5410));
-            *reinterpret_cast<uint4*>(cnt_sm + (warp + H) * THREADS + lane * PER + 8 * u) =
-                make_uint4(__byte_perm(p[0], p[1], 0x7632), __byte_perm(p[2], p[3], 0x7632),
-                           __byte_perm(p[4], p[5], 0x7632), __byte_perm(p[6], p[7], 0x7632));
-        }
+        for (int u = 0; u < PER / 4; u++)
+            *reinterpret_cast<uint4*>(row + CC::chunk(lane, u)) =
+                make_uint4(pre[4 * u] + add, pre[4 * u + 1] + add, pre[4 * u + 2] + add,
+                           pre[4 * u + 3] + add);
         if (warp == 0 && cls) {
             sh.cursor[par ^ 1u][c] = FORWARD ? cur + cc : dst;
             sh.run_start[c] = st;
@@ -295,20 +387,25 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
     __syncthreads();  // (C)
 
     // ---- pass 2: scatter into the class-sorted stage
-    if (full) {
-#pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            const uint32_t c = d(v[j]);
-            stage[my_cnt[c * THREADS] + ((lr[j >> 3] >> (4 * (j & 7))) & 15u)] = v[j];
+    auto place = [&](int j) {
+        uint16_t& next = count_at(d(v[j]));
+        if constexpr (kRanks) {
+            stage[next + ((lr[j >> 3] >> (4 * (j & 7))) & 15u)] = v[j];
+        } else {  // the thread's slot of a class moves on with every element of it
+            const uint32_t slot = next;
+            next = static_cast<uint16_t>(slot + 1u);
+            stage[slot] = v[j];
         }
+    };
+    if (CLUSTERED && one_class) {
+        place_warp_run(stage + (count_at(c_last) - ITEMS * lane), v);
+    } else if (full) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; j++) place(j);
     } else {
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            if (e0 + j >= lo && e0 + j < hi) {
-                const uint32_t c = d(v[j]);
-                stage[my_cnt[c * THREADS] + ((lr[j >> 3] >> (4 * (j & 7))) & 15u)] = v[j];
-            }
-        }
+        for (int j = 0; j < ITEMS; j++)
+            if (e0 + j >= lo && e0 + j < hi) place(j);
     }
     fence_proxy_async_smem();
     __syncthreads();  // (D)
@@ -395,6 +492,7 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
         }
     }
     const uint32_t n1 = static_cast<uint32_t>(__popc(m1));
+    const bool one_class = full && warp_of_one_class(n1 == 0u || n1 == ITEMS, n1);
     const uint32_t x = (static_cast<uint32_t>(__popc(mv)) - n1) | (n1 << 16);
     const uint32_t incl = warp_incl_scan(x);
     if (lane == 31) wsum[warp] = incl;
@@ -431,12 +529,17 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
         const uint32_t b0 = sh.run_start[0] + (pre & 0xffffu);
         const uint32_t b1 = sh.run_start[1] + (pre >> 16);
         const uint32_t m0 = mv & ~m1;
+        if (one_class) {
+            place_warp_run(stage + ((m1 ? b1 : b0) - ITEMS * lane), v);
+        } else {
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            const uint32_t below = (1u << j) - 1u;
-            const uint32_t slot = ((m1 >> j) & 1u) ? b1 + static_cast<uint32_t>(__popc(m1 & below))
-                                                   : b0 + static_cast<uint32_t>(__popc(m0 & below));
-            if ((mv >> j) & 1u) stage[slot] = v[j];
+            for (int j = 0; j < ITEMS; j++) {
+                const uint32_t below = (1u << j) - 1u;
+                const uint32_t slot = ((m1 >> j) & 1u)
+                                          ? b1 + static_cast<uint32_t>(__popc(m1 & below))
+                                          : b0 + static_cast<uint32_t>(__popc(m0 & below));
+                if ((mv >> j) & 1u) stage[slot] = v[j];
+            }
         }
     }
     fence_proxy_async_smem();
@@ -475,145 +578,225 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
 }
 
 // ------------------------------------------------------------ 17..64 classes --
-// With more than 16 classes the per-thread nibble counters no longer fit in a
-// register pair, so ranks come from the warp instead (striped layout):
-//  * in round j lane l of warp w holds tile element w*32*ITEMS + j*32 + l, so
-//    (warp, round, lane) is input order; TMA places these tiles without
-//    swizzle, so a round is one conflict-free shared load per lane;
-//  * the lanes of a round that share a class are found from log2(M) ballots
-//    of the class bits (peers = AND over bits of ballot or ~ballot), the rank
-//    in the round is popc(peers & lanemask_lt);
-//  * lane k keeps the warp's running count of class k (and k + 32 when M = 64)
-//    in a register, read by one shuffle per element and advanced by a popcount
-//    of the lanes of class k (the same AND over bits with k's own bits);
-//  * warp 0 turns the [warp][class] counts into class runs at the
-//    destination's 16-byte phase and stage bases per (warp, class), which pass
-//    2 reads from shared memory; the write-out is that of tile_scatter.
-// The step is bound by the ALU pipe (ncu, m = 64: 72 % of peak), so full
-// tiles take a path without the bounds tests and selects.
+// With this many classes a thread's counters no longer fit in a register pair.
+// They lie in shared memory instead, one byte per class, and are private to the
+// thread, so no ranks have to be agreed on within a warp:
+//  * pass 1: an element's local rank is the thread's counter of its class, read
+//    and incremented.  A 32-bit word holds four classes, a row holds one word of
+//    every thread, and a warp's 32 words of a row lie in 32 banks, so whatever
+//    classes the lanes hold, a load or a store is one wavefront;
+//  * scan: a warp takes a row (four classes), a lane the words of 8 or 16
+//    threads; exclusive prefixes in the packed bytes, over as many lanes as keep
+//    them within a byte (a group of 16 threads of 16 elements), are written back;
+//    the lanes' totals, widened to 16 bits, are scanned over the warp and, with
+//    the class's stage slot added, go to a [group][class] table;
+//  * pass 2: stage slot = group table + thread prefix + local rank;
+//  * the write-out is that of tile_scatter.
+// The words lie in the columns of CountColumns; a row of the group table is
+// padded by 8 bytes so that its 8-byte stores spread over the banks.
+//
+// What bounds it: the shared-memory pipe, about 15 wavefronts per 32 elements at
+// m = 64 (a byte load and store, the two table lookups and the stage store of
+// which the lookup and the store conflict at random), 70 % busy.  The ballots per
+// class bit and shuffles that this replaces took 79 instructions an element and
+// were bound by the ALU.  N = 2^28 u32, scatter at m = 32 and 64: 814 and 1050 us
+// before, 528 and 707 with 256 threads, 506 and 597 with 512; 2^27 records of 8
+// bytes: 521 and 632 before, 442 and 587, 443 and 501.
+template <int M>
+constexpr int kGroupRow = M + 4;  // u16 entries of a row of the group table
 
-// A warp's striped elements of a tile that TMA placed in shared memory
-// without swizzle (element e at tile[e]).
-template <class V, int ITEMS>
-__device__ __forceinline__ void take_striped(const V* tile, V (&v)[ITEMS]) {
-    const V* p = tile + (threadIdx.x >> 5) * 32u * ITEMS + (threadIdx.x & 31u);
-#pragma unroll
-    for (int j = 0; j < ITEMS; j++) v[j] = p[j * 32];
+// Scan lanes (PER threads each) whose threads share a row of the group table:
+// as many as keep a thread's prefix in the group within a byte, a warp at most.
+__host__ __device__ constexpr int byte_group_lanes(int per, int items) {
+    int l = 1;
+    while (2 * l * per <= 32 && 2 * l * per * items <= 256) l *= 2;
+    return l;
 }
 
-template <class V, class D, int M, int THREADS, bool FORWARD, bool FULL, class OUT,
+template <class V, class D, int M, int THREADS, bool FORWARD, bool CLUSTERED, class OUT,
           class AfterCounts, int ITEMS>
-__device__ __forceinline__ bool tile_scatter_wide_impl(const D& d, const V (&v)[ITEMS],
-                                                       uint32_t lo, uint32_t hi, V* stage,
-                                                       uint32_t* wtab, TileShared<M>& sh,
-                                                       uint32_t par, const OUT& out, bool ok,
-                                                       AfterCounts after_counts) {
+__device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEMS], uint32_t lo,
+                                                   uint32_t hi, bool full, V* stage,
+                                                   unsigned char* cnt, TileShared<M>& sh,
+                                                   uint32_t par, const OUT& out, bool ok,
+                                                   AfterCounts after_counts) {
     using G = TileGeom<V, THREADS, M, ITEMS * static_cast<int>(sizeof(V))>;
+    using CC = CountColumns<THREADS>;
+    static_assert(G::kItems == ITEMS, "geometry");
+    static_assert(M == 32 || M == 64, "class bound");
     constexpr uint32_t AU = G::kAU;
     constexpr int W = THREADS / 32;
-    constexpr int B = M == 32 ? 5 : 6;
-    static_assert(M == 32 || M == 64, "17..64 classes (class bound 32 or 64)");
-    static_assert(32 * ITEMS <= 512, "warp ranks < 512 fit the packed 16-bit slots");
+    constexpr int PER = static_cast<int>(CC::kPer);
+    constexpr int ROWS = M / 4;
+    constexpr int RPW = (ROWS + W - 1) / W;  // rows a warp scans
+    constexpr int LPG = byte_group_lanes(PER, ITEMS);
+    static_assert((PER * LPG - 1) * ITEMS <= 255, "byte prefixes");
+    static_assert(LPG == 1 || PER * ITEMS <= 255, "a lane's totals fit bytes when lanes share a group");
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t lt = lanemask_lt();
-    const uint32_t ew = static_cast<uint32_t>(warp) * 32u * ITEMS + static_cast<uint32_t>(lane);
+    const uint32_t e0 = tid * ITEMS;
+    unsigned char* my = cnt + 4u * CC::column(tid);  // class c at my[(c / 4) * 4 * THREADS + c % 4]
+    uint16_t* grp = reinterpret_cast<uint16_t*>(cnt + M * THREADS);
+    auto at = [&](uint32_t c) -> unsigned char& {
+        return my[(c >> 2) * (4u * THREADS) + (c & 3u)];
+    };
 
-    // ---- pass 1: warp ranks.  Lane k builds the mask of the lanes holding
-    // class k (and k + 32): one LOP3 per class bit against its own bits; an
-    // element's peers are then lane (c mod 32)'s mask, fetched by a shuffle.
-    uint32_t inv[5];  // bit i of the lane id set: ballot as is, else its complement
+    // ---- pass 1: local ranks, a byte each
 #pragma unroll
-    for (int i = 0; i < 5; i++) inv[i] = ((lane >> i) & 1) ? 0u : 0xffffffffu;
-    uint32_t runs = 0;       // warp's running count of class lane (low 16 bits), lane + 32 (high)
-    uint32_t rk[ITEMS / 2];  // ranks, two per word
+    for (int r = 0; r < ROWS; r++) *reinterpret_cast<uint32_t*>(my + r * 4 * THREADS) = 0u;
+    uint32_t lr[(ITEMS + 3) / 4];
 #pragma unroll
-    for (int q = 0; q < ITEMS / 2; q++) rk[q] = 0;
+    for (int q = 0; q < (ITEMS + 3) / 4; q++) lr[q] = 0;
+    auto count = [&](int j) {
+        unsigned char& x = at(d(v[j]));
+        const uint32_t r = x;
+        x = static_cast<unsigned char>(r + 1u);
+        lr[j >> 2] += r << (8 * (j & 3));
+    };
+    if (full) {
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        bool valid = true;
-        if constexpr (!FULL) {
-            const uint32_t e = ew + j * 32u;
-            valid = e >= lo && e < hi;
-        }
-        const uint32_t c = valid ? d(v[j]) : 0u;
-        uint32_t com = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
+        for (int j = 0; j < ITEMS; j++) count(j);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 5; i++) com &= __ballot_sync(0xffffffffu, (c >> i) & 1u) ^ inv[i];
-        uint32_t peers, base;
-        // a shuffle's source lane is taken mod 32: c selects lane c mod 32
-        const uint32_t x = __shfl_sync(0xffffffffu, runs, c);
-        if constexpr (B == 6) {
-            const uint32_t hi = (c >> 5) & 1u;
-            const uint32_t b5 = __ballot_sync(0xffffffffu, hi);
-            const uint32_t com1 = com & b5;
-            // lanes of class (c mod 32) with the same sixth bit as c
-            const uint32_t p = __shfl_sync(0xffffffffu, com, c);
-            peers = p & (b5 ^ (hi - 1u));
-            base = __byte_perm(x, 0u, 0x4410u + hi * 0x22u);  // low or high 16 bits
-            const uint32_t n1 = static_cast<uint32_t>(__popc(com1));
-            runs += (static_cast<uint32_t>(__popc(com)) - n1) + (n1 << 16);
-        } else {
-            peers = __shfl_sync(0xffffffffu, com, c);
-            base = x;
-            runs += static_cast<uint32_t>(__popc(com));
-        }
-        const uint32_t r = base + __popc(peers & lt);
-        rk[j >> 1] |= r << (16 * (j & 1));
+        for (int j = 0; j < ITEMS; j++)
+            if (e0 + j >= lo && e0 + j < hi) count(j);
     }
-    wtab[warp * M + lane] = runs & 0xffffu;
-    if constexpr (M == 64) wtab[warp * M + lane + 32] = runs >> 16;
+    const uint32_t c_last = d(v[ITEMS - 1]);
+    bool one_class = false;  // the warp's elements
+    if constexpr (CLUSTERED)
+        one_class = full && warp_of_one_class(
+                                (lr[(ITEMS - 1) >> 2] >> (8 * ((ITEMS - 1) & 3))) == ITEMS - 1, c_last);
     if (__syncthreads_or(!ok)) return false;  // (A)
     after_counts();
 
-    // ---- class runs (warp 0, lane = classes lane and lane + 32): totals over
-    // warps, runs at the destination's 16-byte phase, stage base per (warp, class)
-    if (warp == 0) {
-        constexpr int KL = M / 32;
-        uint32_t st_prev = 0;  // end of the rooms of the classes scanned so far
+    // ---- scan: warp w takes rows w, w + W, ...; a lane PER threads
+    uint32_t ev[RPW], od[RPW];  // classes 4 r, 4 r + 2 and 4 r + 1, 4 r + 3: exclusive over lanes
 #pragma unroll
-        for (int h = 0; h < KL; h++) {
-            const uint32_t c = static_cast<uint32_t>(lane + 32 * h);
-            uint32_t pre[W];
-            uint32_t cc = 0;
+    for (int u = 0; u < RPW; u++) {
+        const int r = warp + u * W;
+        if (ROWS % W != 0 && r >= ROWS) break;
+        unsigned char* row = cnt + 4 * r * THREADS;
+        uint32_t x[PER];
 #pragma unroll
-            for (int w = 0; w < W; w++) {
-                pre[w] = cc;
-                cc += wtab[w * M + c];
+        for (int q = 0; q < PER / 4; q++) {
+            const uint4 a = *reinterpret_cast<const uint4*>(row + 4u * CC::chunk(lane, q));
+            x[4 * q + 0] = a.x;
+            x[4 * q + 1] = a.y;
+            x[4 * q + 2] = a.z;
+            x[4 * q + 3] = a.w;
+        }
+        uint32_t p = 0;  // the lane's threads but the last
+#pragma unroll
+        for (int q = 0; q + 1 < PER; q++) p += x[q];
+        const uint32_t te = (p & 0x00ff00ffu) + (x[PER - 1] & 0x00ff00ffu);
+        const uint32_t to = ((p >> 8) & 0x00ff00ffu) + ((x[PER - 1] >> 8) & 0x00ff00ffu);
+        uint32_t run = 0;
+        if constexpr (LPG > 1) {  // the threads of the group's lanes before this one
+            const uint32_t own = p + x[PER - 1];
+            uint32_t in = own;
+#pragma unroll
+            for (int dd = 1; dd < LPG; dd <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, in, dd, LPG);
+                if (lane % LPG >= dd) in += up;
             }
-            const uint32_t cur = sh.cursor[par][c];
-            const uint32_t dst = FORWARD ? cur : cur - cc;
-            const uint32_t room = cc + AU;
-            const uint32_t incl = warp_incl_scan(room);
-            const uint32_t q0 = st_prev + incl - room;
-            st_prev += __shfl_sync(0xffffffffu, incl, 31);
-            const uint32_t st = q0 + (((out.phase() + dst) - q0) & (AU - 1u));
+            run = in - own;
+        }
 #pragma unroll
-            for (int w = 0; w < W; w++) wtab[w * M + c] = st + pre[w];
-            sh.cursor[par ^ 1u][c] = FORWARD ? cur + cc : dst;
-            sh.run_start[c] = st;
-            sh.run_cnt[c] = cc;
-            sh.run_dst[c] = dst;
+        for (int q = 0; q < PER; q++) {
+            const uint32_t t = x[q];
+            x[q] = run;
+            run += t;
+        }
+#pragma unroll
+        for (int q = 0; q < PER / 4; q++)
+            *reinterpret_cast<uint4*>(row + 4u * CC::chunk(lane, q)) =
+                make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        const uint32_t ie = warp_incl_scan(te), io = warp_incl_scan(to);
+        ev[u] = ie - te;
+        od[u] = io - to;
+        if (lane == 31) {
+            *reinterpret_cast<uint4*>(&sh.rowtot[4 * r]) =
+                make_uint4(ie & 0xffffu, io & 0xffffu, ie >> 16, io >> 16);
+        }
+    }
+    __syncthreads();  // (B)
+
+    // ---- class runs: destination of run c and its stage slot, at the
+    // destination's 16-byte phase (every scanning warp, lanes = classes, two
+    // consecutive classes a lane when M = 64)
+    if (ROWS >= W || warp < ROWS) {
+        constexpr int CPL = M > 32 ? 2 : 1;
+        uint32_t cc[CPL], dst[CPL], st[CPL];
+        uint32_t room = 0;
+        const bool cls = lane * CPL < M;
+#pragma unroll
+        for (int q = 0; q < CPL; q++) {
+            const int c = lane * CPL + q;
+            cc[q] = cls ? sh.rowtot[c] : 0u;
+            const uint32_t cur = cls ? sh.cursor[par][c] : 0u;
+            dst[q] = FORWARD ? cur : cur - cc[q];
+            room += cc[q] + (cls ? AU : 0u);
+        }
+        uint32_t q0 = warp_incl_scan(room) - room;
+#pragma unroll
+        for (int q = 0; q < CPL; q++) {
+            st[q] = q0 + (((out.phase() + dst[q]) - q0) & (AU - 1u));
+            q0 += cc[q] + AU;
+        }
+        if (warp == 0 && cls) {
+#pragma unroll
+            for (int q = 0; q < CPL; q++) {
+                const int c = lane * CPL + q;
+                sh.cursor[par ^ 1u][c] = FORWARD ? dst[q] + cc[q] : dst[q];
+                sh.run_start[c] = st[q];
+                sh.run_cnt[c] = cc[q];
+                sh.run_dst[c] = dst[q];
+            }
+        }
+        const uint32_t st2 = CPL == 2 ? st[0] | (st[CPL - 1] << 16) : st[0];  // slots < 2^16
+#pragma unroll
+        for (int u = 0; u < RPW; u++) {
+            const int r = warp + u * W;
+            if (ROWS % W != 0 && r >= ROWS) break;
+            uint32_t s01, s23;  // the slots of classes 4 r, 4 r + 1 and 4 r + 2, 4 r + 3
+            if (CPL == 2) {
+                s01 = __shfl_sync(0xffffffffu, st2, 2 * r);
+                s23 = __shfl_sync(0xffffffffu, st2, 2 * r + 1);
+            } else {
+                s01 = __shfl_sync(0xffffffffu, st2, 4 * r) |
+                      (__shfl_sync(0xffffffffu, st2, 4 * r + 1) << 16);
+                s23 = __shfl_sync(0xffffffffu, st2, 4 * r + 2) |
+                      (__shfl_sync(0xffffffffu, st2, 4 * r + 3) << 16);
+            }
+            if (lane % LPG == 0)
+                *reinterpret_cast<uint2*>(grp + (lane / LPG) * kGroupRow<M> + 4 * r) =
+                    make_uint2(__byte_perm(ev[u], od[u], 0x5410) + s01,
+                               __byte_perm(ev[u], od[u], 0x7632) + s23);
         }
     }
     // the stage is about to be rewritten: the previous tile's bulk stores
     // must have finished reading it
     if (tid < M) bulk_wait_read<0>();
-    __syncthreads();  // (B)
+    __syncthreads();  // (C)
 
-    // ---- pass 2: stage slot = base of (warp, class) + warp rank
-    const uint32_t* wb = wtab + warp * M;
+    // ---- pass 2: scatter into the class-sorted stage
+    const uint16_t* gb = grp + tid / (PER * LPG) * kGroupRow<M>;
+    auto place = [&](int j) {
+        const uint32_t c = d(v[j]);
+        stage[gb[c] + at(c) + __byte_perm(lr[j >> 2], 0u, 0x4440 + (j & 3))] = v[j];
+    };
+    if (CLUSTERED && one_class) {
+        place_warp_run(stage + (gb[c_last] + at(c_last) - ITEMS * lane), v);
+    } else if (full) {
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        bool valid = true;
-        if constexpr (!FULL) {
-            const uint32_t e = ew + j * 32u;
-            valid = e >= lo && e < hi;
-        }
-        if (valid) stage[wb[d(v[j])] + ((rk[j >> 1] >> (16 * (j & 1))) & 0xffffu)] = v[j];
+        for (int j = 0; j < ITEMS; j++) place(j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < ITEMS; j++)
+            if (e0 + j >= lo && e0 + j < hi) place(j);
     }
     fence_proxy_async_smem();
-    __syncthreads();  // (C)
+    __syncthreads();  // (D)
 
     // ---- write-out: bulk store of each run's aligned interior; all threads
     // store the unaligned heads and tails
@@ -624,7 +807,7 @@ __device__ __forceinline__ bool tile_scatter_wide_impl(const D& d, const V (&v)[
         const uint32_t body = ((cc - head) / AU) * AU;
         uint32_t a0 = sh.run_dst[tid] + head, sl = s + head;
         const uint32_t a1 = a0 + body;
-        while (a0 < a1) {
+        while (a0 < a1) {  // one piece per destination buffer
             const uint32_t b = out.piece_end(a0, a1);
             bulk_store_s2g(out.at(a0), stage + sl, (b - a0) * sizeof(V));
             sl += b - a0;
@@ -632,35 +815,24 @@ __device__ __forceinline__ bool tile_scatter_wide_impl(const D& d, const V (&v)[
         }
         bulk_commit();
     }
-    for (int t = tid; t < M * 2 * static_cast<int>(AU); t += THREADS) {
-        const uint32_t c = static_cast<uint32_t>(t) / (2 * AU), q = static_cast<uint32_t>(t) % (2 * AU);
-        const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t off = 0xffffffffu;
-        if (q < AU) {
-            if (q < head) off = q;
-        } else if (head + body + (q - AU) < cc) {
-            off = head + body + (q - AU);
+    if constexpr (AU > 1) {
+#pragma unroll
+        for (int t = tid; t < M * 2 * static_cast<int>(AU); t += THREADS) {
+            const uint32_t c = static_cast<uint32_t>(t) / (2 * AU), q = static_cast<uint32_t>(t) % (2 * AU);
+            const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
+            uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
+            if (head > cc) head = cc;
+            const uint32_t body = ((cc - head) / AU) * AU;
+            uint32_t off = 0xffffffffu;
+            if (q < AU) {
+                if (q < head) off = q;
+            } else if (head + body + (q - AU) < cc) {
+                off = head + body + (q - AU);
+            }
+            if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
         }
-        if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
     }
     return true;
-}
-
-template <class V, class D, int M, int THREADS, bool FORWARD, class OUT, class AfterCounts,
-          int ITEMS>
-__device__ __forceinline__ bool tile_scatter_wide(const D& d, const V (&v)[ITEMS],
-                                                  uint32_t lo, uint32_t hi, bool full, V* stage,
-                                                  uint32_t* wtab, TileShared<M>& sh, uint32_t par,
-                                                  const OUT& out, bool ok,
-                                                  AfterCounts after_counts) {
-    if (full)
-        return tile_scatter_wide_impl<V, D, M, THREADS, FORWARD, true>(d, v, lo, hi, stage, wtab, sh,
-                                                                     par, out, ok, after_counts);
-    return tile_scatter_wide_impl<V, D, M, THREADS, FORWARD, false>(d, v, lo, hi, stage, wtab, sh,
-                                                                  par, out, ok, after_counts);
 }
 
 }  // namespace mdx

@@ -1,5 +1,7 @@
 """The plain path's tile steps where they can go wrong, bit-exact against the
-oracle: remainders over the whole range of 32-bit keys."""
+oracle: remainders over the whole range of 32-bit keys, sorted and clustered
+inputs (warps of one class next to mixed ones), and every tile geometry at the
+edges of its tiles."""
 import numpy as np
 import pytest
 
@@ -37,3 +39,54 @@ def test_remainders_of_every_class_count(cuda_ready):
         x = k[k < (1 << 32)].astype(np.uint32)
         x[-1] = 0xffffffff
         check(cuda_ready, x, m)
+
+
+def clustered(n, m, form, seed):
+    rng = np.random.default_rng(seed)
+    if form == "sorted":
+        cls = np.sort(rng.integers(0, m, n))
+    elif form == "one":
+        cls = np.full(n, m - 1)
+    elif form == "runs":  # lengths around a warp's and a thread's elements
+        lengths = rng.choice([1, 15, 16, 17, 127, 128, 255, 256, 511, 512, 513, 2000, 9000], n)
+        cls = np.repeat(rng.integers(0, m, n), lengths)[:n]
+    else:  # two classes hold nearly all
+        cls = np.where(rng.random(n) < 0.02, rng.integers(0, m, n), (np.arange(n) // 3000) % 2)
+    return (rng.integers(0, 1 << 24, n) * m + cls).astype(np.uint32)
+
+
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("threads", [256, 512])
+@pytest.mark.parametrize("m", [2, 3, 8, 13, 32, 64])
+def test_clustered_inputs(cuda_ready, m, threads, rec):
+    elem = mdx.ELEM_REC8 if rec else mdx.ELEM_U32
+    tile = threads * (8 if rec else 16)
+    try:
+        mdx.set_tuning(elem, m, 0, 33, plain_two_kernel=1, tile_bytes=64, tile_threads=threads)
+        for form in ("sorted", "one", "runs", "two"):
+            for n in (tile - 1, tile, 3 * tile + 1, 700_001):
+                x = clustered(n, m, form, m + n)
+                if rec:
+                    x = x.astype(np.uint64) | (np.arange(n, dtype=np.uint64) << np.uint64(32))
+                check(cuda_ready, x, m)
+    finally:
+        mdx.set_tuning(elem, m, 0, 33)
+        mdx.load_tuning(mdx.TUNING_PATH, missing_ok=True)
+
+
+@pytest.mark.parametrize("m", [5, 16, 32, 64])
+def test_records_of_16_bytes(cuda_ready, m):
+    """Four records a thread: the count columns and byte groups at their smallest."""
+    torch = cuda_ready
+    for n in (1023, 1024, 4097, 300_001):
+        for form in ("sorted", "runs"):
+            keys = clustered(n, m, form, n)
+            rows = np.empty((n, 4), dtype=np.uint32)
+            rows[:, 0] = keys
+            rows[:, 1:] = np.random.default_rng(n).integers(0, 1 << 32, (n, 3))
+            order = np.argsort(keys % m, kind="stable")
+            d = torch.from_numpy(rows.view(np.int32)).cuda()
+            out, sizes = mdx.partition_records(d, 16, ("mod", m))
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy().view(np.uint32), rows[order])
+            assert np.array_equal(sizes.cpu().numpy(), np.bincount(keys % m, minlength=m))

@@ -340,6 +340,79 @@ struct ScatterTmaSmem {
     static constexpr size_t kBytes = 1024 + kRingBytes + G::kStageBytes + G::kCntBytes;
 };
 
+// Where chunk k's class runs end in the output, from the [class][chunk] counts
+// (a scatter CTA, every thread): cursor[c] = class base + the chunk's exclusive
+// prefix + its own count.  CTA 0 writes the class bases, totals, sizes and head
+// flags.  tot_sh and pre_sh are zero on entry; *clustered: two classes hold 7/8 of
+// the chunk.  The caller synchronises before it uses the results.
+template <int M, int THREADS>
+__device__ __forceinline__ void scatter_cursors(const PlainArgs& a, uint32_t k, uint32_t* tot_sh,
+                                                uint32_t* pre_sh, uint32_t* cursor, int* clustered) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t G = a.num_chunks, stride = a.chunk_stride;
+    // this chunk's exclusive class prefix and the class totals from the
+    // [class][chunk] counts (TPC threads per class, 16-byte loads)
+    constexpr int TPC = THREADS / M;
+    constexpr int RW = TPC < 32 ? TPC : 32;
+    const uint32_t c = static_cast<uint32_t>(tid / TPC), l = static_cast<uint32_t>(tid % TPC);
+    const uint4* row = reinterpret_cast<const uint4*>(a.chunk_cnt + static_cast<uint64_t>(c) * stride);
+    uint32_t tot = 0, pre = 0;
+    for (uint32_t q4 = l; q4 < stride / 4u; q4 += TPC) {
+        const uint4 x = __ldcg(row + q4);
+        const uint32_t j = 4u * q4;
+        const uint32_t xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const uint32_t v = (j + u < G) ? xv[u] : 0u;
+            tot += v;
+            pre += (j + u < k) ? v : 0u;
+        }
+    }
+#pragma unroll
+    for (int off = RW / 2; off > 0; off >>= 1) {
+        tot += __shfl_xor_sync(0xffffffffu, tot, off);
+        pre += __shfl_xor_sync(0xffffffffu, pre, off);
+    }
+    if ((lane % RW) == 0) {
+        atomicAdd(&tot_sh[c], tot);
+        atomicAdd(&pre_sh[c], pre);
+    }
+    __syncthreads();
+    if (warp == 0) {  // class bases: exclusive scan of the totals
+        uint32_t carry = 0, sum = 0, max1 = 0, max2 = 0;
+#pragma unroll
+        for (int h = 0; h < (M + 31) / 32; h++) {
+            const uint32_t cc = static_cast<uint32_t>(lane + 32 * h);
+            const uint32_t x = cc < static_cast<uint32_t>(M) ? tot_sh[cc] : 0u;
+            const uint32_t incl = warp_incl_scan(x);
+            const uint32_t bc = carry + incl - x;
+            if (cc < static_cast<uint32_t>(M)) {
+                const uint32_t own = __ldcg(a.chunk_cnt + static_cast<uint64_t>(cc) * stride + k);
+                cursor[cc] = bc + pre_sh[cc] + own;
+                sum += own;
+                max2 = max(max2, min(max1, own));
+                max1 = max(max1, own);
+                if (k == 0) {
+                    a.class_base[cc] = bc;
+                    a.class_tot[cc] = x;
+                    if (a.sizes != nullptr && cc < a.m) a.sizes[cc] = x;
+                    // head-flag form (SeqMdiscr.h:47-49); zeroed before the count kernel
+                    if (a.headflags != nullptr && x > 0) a.headflags[bc] = x;
+                }
+            }
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if constexpr (M > 2) {
+            const uint32_t all = __reduce_add_sync(0xffffffffu, sum);
+            const uint32_t top = __reduce_max_sync(0xffffffffu, max1);
+            const uint32_t at = __ballot_sync(0xffffffffu, max1 == top);
+            const uint32_t rest = lane == __ffs(at) - 1 ? max2 : max1;
+            const uint32_t second = __reduce_max_sync(0xffffffffu, rest);
+            if (lane == 0) *clustered = all - top - second <= all / 8u;
+        }
+    }
+}
+
 // Scatter kernel: CTA k re-reads chunk k (tiles in reverse order) and writes
 // every element at class_base[c] + chunk_pre[c][k] + its rank in the chunk.
 // Tiles arrive by tensor TMA (one 2-D box of 128-byte rows per tile, 128-byte
@@ -419,67 +492,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     pdl_wait();
     const uint32_t stride = a.chunk_stride;
     if (a.prefix_in_scatter) {
-        // this chunk's exclusive class prefix and the class totals from the
-        // [class][chunk] counts (TPC threads per class, 16-byte loads)
-        constexpr int TPC = THREADS / M;
-        constexpr int RW = TPC < 32 ? TPC : 32;
-        const uint32_t c = static_cast<uint32_t>(tid / TPC), l = static_cast<uint32_t>(tid % TPC);
-        const uint4* row = reinterpret_cast<const uint4*>(a.chunk_cnt + static_cast<uint64_t>(c) * stride);
-        uint32_t tot = 0, pre = 0;
-        for (uint32_t q4 = l; q4 < stride / 4u; q4 += TPC) {
-            const uint4 x = __ldcg(row + q4);
-            const uint32_t j = 4u * q4;
-            const uint32_t xv[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (uint32_t u = 0; u < 4; u++) {
-                const uint32_t v = (j + u < G) ? xv[u] : 0u;
-                tot += v;
-                pre += (j + u < k) ? v : 0u;
-            }
-        }
-#pragma unroll
-        for (int off = RW / 2; off > 0; off >>= 1) {
-            tot += __shfl_xor_sync(0xffffffffu, tot, off);
-            pre += __shfl_xor_sync(0xffffffffu, pre, off);
-        }
-        if ((lane % RW) == 0) {
-            atomicAdd(&tot_sh[c], tot);
-            atomicAdd(&pre_sh[c], pre);
-        }
-        __syncthreads();
-        if (warp == 0) {  // class bases: exclusive scan of the totals
-            uint32_t carry = 0, sum = 0, max1 = 0, max2 = 0;
-#pragma unroll
-            for (int h = 0; h < (M + 31) / 32; h++) {
-                const uint32_t cc = static_cast<uint32_t>(lane + 32 * h);
-                const uint32_t x = cc < static_cast<uint32_t>(M) ? tot_sh[cc] : 0u;
-                const uint32_t incl = warp_incl_scan(x);
-                const uint32_t bc = carry + incl - x;
-                if (cc < static_cast<uint32_t>(M)) {
-                    const uint32_t own = __ldcg(a.chunk_cnt + static_cast<uint64_t>(cc) * stride + k);
-                    sh.cursor[0][cc] = bc + pre_sh[cc] + own;
-                    sum += own;
-                    max2 = max(max2, min(max1, own));
-                    max1 = max(max1, own);
-                    if (k == 0) {
-                        a.class_base[cc] = bc;
-                        a.class_tot[cc] = x;
-                        if (a.sizes != nullptr && cc < a.m) a.sizes[cc] = x;
-                        // head-flag form (SeqMdiscr.h:47-49); zeroed before the count kernel
-                        if (a.headflags != nullptr && x > 0) a.headflags[bc] = x;
-                    }
-                }
-                carry += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            if constexpr (M > 2) {
-                const uint32_t all = __reduce_add_sync(0xffffffffu, sum);
-                const uint32_t top = __reduce_max_sync(0xffffffffu, max1);
-                const uint32_t at = __ballot_sync(0xffffffffu, max1 == top);
-                const uint32_t rest = lane == __ffs(at) - 1 ? max2 : max1;
-                const uint32_t second = __reduce_max_sync(0xffffffffu, rest);
-                if (lane == 0) clustered_sh = all - top - second <= all / 8u;
-            }
-        }
+        scatter_cursors<M, THREADS>(a, k, tot_sh, pre_sh, sh.cursor[0], &clustered_sh);
     } else if (tid < M) {
         const uint64_t o = static_cast<uint64_t>(tid) * stride + k;
         sh.cursor[0][tid] = a.class_base[tid] + a.chunk_pre[o] + a.chunk_cnt[o];

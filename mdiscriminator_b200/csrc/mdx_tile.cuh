@@ -23,6 +23,8 @@
 //    read it (cp.async.bulk.wait_group.read).
 #pragma once
 
+#include <type_traits>
+
 #include "mdx_device.cuh"
 
 namespace mdx {
@@ -76,7 +78,7 @@ __device__ __forceinline__ void unpack16_to<Rec16>(const uint4& r, Rec16* e) {
 
 template <class V, int THREADS, int M, int BPT = 64>
 struct TileGeom {
-    static_assert(BPT == 64 || BPT == 32, "64 or 32 bytes per thread");
+    static_assert(BPT == 64 || BPT == 32 || BPT == 16, "64, 32 or 16 bytes per thread");
     static constexpr int kItems = BPT / static_cast<int>(sizeof(V));  // BPT bytes per thread
     static constexpr int kTile = THREADS * kItems;
     static constexpr int kRows = kTile * static_cast<int>(sizeof(V)) / 128;  // 128-byte rows
@@ -107,6 +109,7 @@ struct TileShared {
 // OutFlat: one array.  phase = (out / sizeof(V)) mod (16 / sizeof(V)).
 template <class V>
 struct OutFlat {
+    static constexpr uint32_t kAU = 16 / sizeof(V);  // elements a bulk store is aligned to
     V* out;
     uint32_t phase_;
     __device__ __forceinline__ uint32_t phase() const { return phase_; }
@@ -126,6 +129,7 @@ struct OutFlat {
 constexpr int kMaxRanks = 128;
 template <class V>
 struct OutSharded {
+    static constexpr uint32_t kAU = 16 / sizeof(V);
     V* chunks[kMaxRanks];
     uint32_t chunk;
     uint32_t R;
@@ -140,6 +144,14 @@ struct OutSharded {
         const uint64_t b = static_cast<uint64_t>(q + 1u) * chunk;
         return b < end ? static_cast<uint32_t>(b) : end;
     }
+};
+
+// OutRows: the tile's order is wanted, not its elements: runs lie in the stage one
+// after another without room for a 16-byte phase, and run_dst holds what has to be
+// added to a slot to give its position in the output (mdx_rows.cuh).
+struct OutRows {
+    static constexpr uint32_t kAU = 1;
+    __device__ __forceinline__ uint32_t phase() const { return 0u; }
 };
 
 // Take a thread's ITEMS * sizeof(V) (64 or 32) bytes of a tile that TMA
@@ -257,6 +269,59 @@ struct ThreadCounts {
     }
 };
 
+// What run_dst of a run says: its position in the output, or (OutRows) the
+// distance from its stage slots to it.
+template <class OUT>
+__device__ __forceinline__ uint32_t run_position(uint32_t dst, uint32_t st) {
+    return std::is_same<OUT, OutRows>::value ? dst - st : dst;
+}
+
+// Write-out of a tile whose class runs lie in the stage, each at its destination's
+// 16-byte phase: a bulk store of each run's aligned interior; threads store the
+// unaligned heads and tails (those of warp 0, which issue the bulk stores, only
+// when the others do not suffice).
+template <class V, int M, int THREADS, class OUT>
+__device__ __forceinline__ void write_runs(const V* stage, const TileShared<M>& sh, const OUT& out) {
+    constexpr uint32_t AU = OUT::kAU;
+    constexpr int kEdges = M * 2 * static_cast<int>(AU);  // head and tail elements at most
+    constexpr int kFirst = M <= 32 && 32 + kEdges <= THREADS ? 32 : 0;
+    const int tid = threadIdx.x;
+    if (tid < M) {
+        const uint32_t s = sh.run_start[tid], cc = sh.run_cnt[tid];
+        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
+        if (head > cc) head = cc;
+        const uint32_t body = ((cc - head) / AU) * AU;
+        uint32_t a0 = sh.run_dst[tid] + head, sl = s + head;
+        const uint32_t a1 = a0 + body;
+        while (a0 < a1) {  // one piece per destination buffer
+            const uint32_t b = out.piece_end(a0, a1);
+            bulk_store_s2g(out.at(a0), stage + sl, (b - a0) * sizeof(V));
+            sl += b - a0;
+            a0 = b;
+        }
+        bulk_commit();
+    }
+    if constexpr (AU > 1) {
+#pragma unroll
+        for (int t0 = 0; t0 < kEdges; t0 += THREADS) {
+            const int t = tid - kFirst + t0;
+            if (t < 0 || t >= kEdges) continue;
+            const uint32_t c = static_cast<uint32_t>(t) / (2 * AU), q = static_cast<uint32_t>(t) % (2 * AU);
+            const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
+            uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
+            if (head > cc) head = cc;
+            const uint32_t body = ((cc - head) / AU) * AU;
+            uint32_t off = 0xffffffffu;
+            if (q < AU) {
+                if (q < head) off = q;
+            } else if (head + body + (q - AU) < cc) {
+                off = head + body + (q - AU);
+            }
+            if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
+        }
+    }
+}
+
 // One tile: see the file comment.  `full` means lo == 0 and hi == TILE (no
 // bounds checks).  FORWARD: run c of this tile starts at cursor[par][c] and
 // the cursor advances; otherwise it ends there and the cursor moves back.
@@ -273,7 +338,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
     static_assert(G::kItems == ITEMS, "geometry");
     using CC = CountColumns<THREADS>;
     using TC = ThreadCounts<M>;
-    constexpr uint32_t AU = G::kAU;
+    constexpr uint32_t AU = OUT::kAU;
     constexpr int W = THREADS / 32;
     constexpr int PER = static_cast<int>(CC::kPer);
     static_assert(TC::kRows <= W, "a warp per row");
@@ -355,7 +420,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
     __syncthreads();  // (B)
 
     // ---- class runs (the scanning warps, lanes = classes): destination of
-    // run c and its stage slot, at the destination's 16-byte phase within kAU
+    // run c and its stage slot, at the destination's 16-byte phase within AU - 1
     // slots of slack per run; each scanning warp folds the slots into its row
     if (scans) {
         const uint32_t c = static_cast<uint32_t>(lane);
@@ -363,7 +428,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
         const uint32_t cc = cls ? sh.rowtot[c] : 0u;
         const uint32_t cur = cls ? sh.cursor[par][c] : 0u;
         const uint32_t dst = FORWARD ? cur : cur - cc;
-        const uint32_t room = cc + (cls ? AU : 0u);
+        const uint32_t room = cc + (cls ? AU - 1u : 0u);
         const uint32_t q0 = warp_incl_scan(room) - room;
         const uint32_t st = q0 + (((out.phase() + dst) - q0) & (AU - 1u));
         // slots < kStageElems < 2^16: the two classes' slots stay packed
@@ -378,7 +443,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
             sh.cursor[par ^ 1u][c] = FORWARD ? cur + cc : dst;
             sh.run_start[c] = st;
             sh.run_cnt[c] = cc;
-            sh.run_dst[c] = dst;
+            sh.run_dst[c] = run_position<OUT>(dst, st);
         }
     }
     // the stage is about to be rewritten: the previous tile's bulk stores
@@ -410,36 +475,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
     fence_proxy_async_smem();
     __syncthreads();  // (D)
 
-    // ---- write-out: bulk store of each run's aligned interior; threads store
-    // the unaligned head and tail elements
-    if (tid < M) {
-        const uint32_t s = sh.run_start[tid], cc = sh.run_cnt[tid];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t a0 = sh.run_dst[tid] + head, sl = s + head;
-        const uint32_t a1 = a0 + body;
-        while (a0 < a1) {  // one piece per destination buffer
-            const uint32_t b = out.piece_end(a0, a1);
-            bulk_store_s2g(out.at(a0), stage + sl, (b - a0) * sizeof(V));
-            sl += b - a0;
-            a0 = b;
-        }
-        bulk_commit();
-    } else if (tid >= 32 && tid < 32 + M * 2 * static_cast<int>(AU)) {
-        const uint32_t c = (tid - 32) / (2 * AU), q = (tid - 32) % (2 * AU);
-        const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t off = 0xffffffffu;
-        if (q < AU) {
-            if (q < head) off = q;
-        } else if (head + body + (q - AU) < cc) {
-            off = head + body + (q - AU);
-        }
-        if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
-    }
+    if constexpr (!std::is_same<OUT, OutRows>::value) write_runs<V, M, THREADS>(stage, sh, out);
     return true;
 }
 
@@ -467,7 +503,7 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
                                             TileShared<2>& sh, uint32_t par, const OUT& out, bool ok,
                                             AfterCounts after_counts) {
     using G = TileGeom<V, THREADS, 2, ITEMS * static_cast<int>(sizeof(V))>;
-    constexpr uint32_t AU = G::kAU;
+    constexpr uint32_t AU = OUT::kAU;
     constexpr int W = THREADS / 32;
     static_assert(ITEMS <= 16 && W <= 32, "16-bit packed warp counts, one lane per warp");
     uint32_t* wsum = scr;      // [W] packed class totals of each warp
@@ -510,12 +546,12 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
             const uint32_t cc = c ? (tot >> 16) : (tot & 0xffffu);
             const uint32_t cur = sh.cursor[par][c];
             const uint32_t dst = FORWARD ? cur : cur - cc;
-            const uint32_t q0 = c ? (tot & 0xffffu) + AU : 0u;  // class 0's room comes first
+            const uint32_t q0 = c ? (tot & 0xffffu) + AU - 1u : 0u;  // class 0's room comes first
             const uint32_t st = q0 + (((out.phase() + dst) - q0) & (AU - 1u));
             sh.cursor[par ^ 1u][c] = FORWARD ? cur + cc : dst;
             sh.run_start[c] = st;
             sh.run_cnt[c] = cc;
-            sh.run_dst[c] = dst;
+            sh.run_dst[c] = run_position<OUT>(dst, st);
         }
     }
     // the stage is about to be rewritten: the previous tile's bulk stores
@@ -545,35 +581,7 @@ __device__ __forceinline__ bool tile_filter(const D& d, const V (&v)[ITEMS], uin
     fence_proxy_async_smem();
     __syncthreads();  // (C)
 
-    // ---- write-out: as tile_scatter
-    if (tid < 2) {
-        const uint32_t s = sh.run_start[tid], cc = sh.run_cnt[tid];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t a0 = sh.run_dst[tid] + head, sl = s + head;
-        const uint32_t a1 = a0 + body;
-        while (a0 < a1) {  // one piece per destination buffer
-            const uint32_t b = out.piece_end(a0, a1);
-            bulk_store_s2g(out.at(a0), stage + sl, (b - a0) * sizeof(V));
-            sl += b - a0;
-            a0 = b;
-        }
-        bulk_commit();
-    } else if (tid >= 32 && tid < 32 + 2 * 2 * static_cast<int>(AU)) {
-        const uint32_t c = (tid - 32) / (2 * AU), q = (tid - 32) % (2 * AU);
-        const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t off = 0xffffffffu;
-        if (q < AU) {
-            if (q < head) off = q;
-        } else if (head + body + (q - AU) < cc) {
-            off = head + body + (q - AU);
-        }
-        if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
-    }
+    if constexpr (!std::is_same<OUT, OutRows>::value) write_runs<V, 2, THREADS>(stage, sh, out);
     return true;
 }
 
@@ -624,7 +632,7 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
     using CC = CountColumns<THREADS>;
     static_assert(G::kItems == ITEMS, "geometry");
     static_assert(M == 32 || M == 64, "class bound");
-    constexpr uint32_t AU = G::kAU;
+    constexpr uint32_t AU = OUT::kAU;
     constexpr int W = THREADS / 32;
     constexpr int PER = static_cast<int>(CC::kPer);
     constexpr int ROWS = M / 4;
@@ -735,13 +743,13 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
             cc[q] = cls ? sh.rowtot[c] : 0u;
             const uint32_t cur = cls ? sh.cursor[par][c] : 0u;
             dst[q] = FORWARD ? cur : cur - cc[q];
-            room += cc[q] + (cls ? AU : 0u);
+            room += cc[q] + (cls ? AU - 1u : 0u);
         }
         uint32_t q0 = warp_incl_scan(room) - room;
 #pragma unroll
         for (int q = 0; q < CPL; q++) {
             st[q] = q0 + (((out.phase() + dst[q]) - q0) & (AU - 1u));
-            q0 += cc[q] + AU;
+            q0 += cc[q] + AU - 1u;
         }
         if (warp == 0 && cls) {
 #pragma unroll
@@ -750,7 +758,7 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
                 sh.cursor[par ^ 1u][c] = FORWARD ? dst[q] + cc[q] : dst[q];
                 sh.run_start[c] = st[q];
                 sh.run_cnt[c] = cc[q];
-                sh.run_dst[c] = dst[q];
+                sh.run_dst[c] = run_position<OUT>(dst[q], st[q]);
             }
         }
         const uint32_t st2 = CPL == 2 ? st[0] | (st[CPL - 1] << 16) : st[0];  // slots < 2^16
@@ -798,40 +806,7 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
     fence_proxy_async_smem();
     __syncthreads();  // (D)
 
-    // ---- write-out: bulk store of each run's aligned interior; all threads
-    // store the unaligned heads and tails
-    if (tid < M) {
-        const uint32_t s = sh.run_start[tid], cc = sh.run_cnt[tid];
-        uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-        if (head > cc) head = cc;
-        const uint32_t body = ((cc - head) / AU) * AU;
-        uint32_t a0 = sh.run_dst[tid] + head, sl = s + head;
-        const uint32_t a1 = a0 + body;
-        while (a0 < a1) {  // one piece per destination buffer
-            const uint32_t b = out.piece_end(a0, a1);
-            bulk_store_s2g(out.at(a0), stage + sl, (b - a0) * sizeof(V));
-            sl += b - a0;
-            a0 = b;
-        }
-        bulk_commit();
-    }
-    if constexpr (AU > 1) {
-#pragma unroll
-        for (int t = tid; t < M * 2 * static_cast<int>(AU); t += THREADS) {
-            const uint32_t c = static_cast<uint32_t>(t) / (2 * AU), q = static_cast<uint32_t>(t) % (2 * AU);
-            const uint32_t s = sh.run_start[c], cc = sh.run_cnt[c];
-            uint32_t head = (AU - (s & (AU - 1u))) & (AU - 1u);
-            if (head > cc) head = cc;
-            const uint32_t body = ((cc - head) / AU) * AU;
-            uint32_t off = 0xffffffffu;
-            if (q < AU) {
-                if (q < head) off = q;
-            } else if (head + body + (q - AU) < cc) {
-                off = head + body + (q - AU);
-            }
-            if (off != 0xffffffffu) *out.at(sh.run_dst[c] + off) = stage[s + off];
-        }
-    }
+    if constexpr (!std::is_same<OUT, OutRows>::value) write_runs<V, M, THREADS>(stage, sh, out);
     return true;
 }
 

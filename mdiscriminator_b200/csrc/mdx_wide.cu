@@ -4,36 +4,25 @@
 // are permuted together (the _tuples variant's u32 / u8 / bool arrays,
 // cuda_code/MdiscrHost_tuples.cu.h:13-48,262-429).
 //
-// Both go through the 8-byte record path:
-//   1. build:     rec[i] = {key_i, i}        (key: the record's first u32 word,
-//                                            or column 0)
+// Rows of up to kMaxRowBytes are moved whole through shared memory by the row
+// kernels (mdx_rows.cuh).  Longer records go through 8-byte records:
+//   1. build:     rec[i] = {key_i, i}        (key: the record's first u32 word)
 //   2. partition: the REC8 kernels with the caller's discriminator on the key
 //                 give the stable order of (key, row) and the class sizes;
-//   3. gather:    output row p = input row (rec_out[p] >> 32), for the whole
-//                 record or for every column; the key comes from rec_out[p].
-// Traffic per row: 4 + 8 (build) + 24 (partition) + 8 + 2R (gather) bytes for
-// R bytes of row data, against 2R for a kernel specialised to the width; 4-,
-// 8- and (16-byte aligned) 16-byte records take the direct record kernels.
+//   3. gather:    output row p = input row (rec_out[p] >> 32).
+// 4-, 8- and (16-byte aligned) 16-byte records take the element kernels.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
 
 #include "mdx_host.cuh"
+#include "mdx_rows.cuh"
 
 namespace mdx {
 namespace wide {
 
 constexpr int kThreads = 256;
-constexpr int kMaxCols = 8;
-
-struct Cols {
-    const void* in[kMaxCols];
-    void* out[kMaxCols];
-    uint32_t bytes[kMaxCols];
-    uint32_t num;
-};
-
 // rec[i] = key_i | (i << 32), key_i = the u32 at byte offset stride * i of keys
 __global__ void __launch_bounds__(kThreads) build_key_index(const unsigned char* keys, uint64_t stride,
                                                             uint64_t n, uint64_t* rec) {
@@ -56,29 +45,6 @@ __global__ void __launch_bounds__(kThreads) gather_records(const uint32_t* in, u
         const uint32_t w = static_cast<uint32_t>(t - p * words);
         const uint64_t src = perm[p] >> 32;
         out[t] = in[src * words + w];
-    }
-}
-
-template <class T>
-__device__ __forceinline__ void move_one(const void* in, void* out, uint64_t src, uint64_t p) {
-    static_cast<T*>(out)[p] = static_cast<const T*>(in)[src];
-}
-
-// Columns: out_c[p] = in_c[perm[p] >> 32]; column 0 (the u32 key) from perm[p].
-__global__ void __launch_bounds__(kThreads) gather_columns(Cols cols, const uint64_t* perm, uint64_t n) {
-    for (uint64_t p = static_cast<uint64_t>(blockIdx.x) * kThreads + threadIdx.x; p < n;
-         p += static_cast<uint64_t>(gridDim.x) * kThreads) {
-        const uint64_t r = perm[p];
-        const uint64_t src = r >> 32;
-        static_cast<uint32_t*>(cols.out[0])[p] = static_cast<uint32_t>(r);
-        for (uint32_t c = 1; c < cols.num; c++) {
-            switch (cols.bytes[c]) {
-                case 1: move_one<uint8_t>(cols.in[c], cols.out[c], src, p); break;
-                case 2: move_one<uint16_t>(cols.in[c], cols.out[c], src, p); break;
-                case 4: move_one<uint32_t>(cols.in[c], cols.out[c], src, p); break;
-                default: move_one<uint64_t>(cols.in[c], cols.out[c], src, p); break;
-            }
-        }
     }
 }
 
@@ -116,6 +82,127 @@ inline mdx_status key_order(const unsigned char* keys, uint64_t stride, uint64_t
     if (cudaGetLastError() != cudaSuccess) return MDX_ERR_CUDA;
     return mdx_partition(rec_in, rec_out, n, MDX_ELEM_REC8, discr, d_sizes, d_headflags,
                          ws + w.plain, w.L.total, reinterpret_cast<mdx_stream_t>(st));
+}
+
+// The row kernels' tiles: 256 threads and two buffers of 20 KB, four CTAs to an SM;
+// above 16 classes 512 threads and two of 36 KB, two CTAs, so that the byte counters'
+// scan is shared by twice the rows (2 * 10^7 rows of a key and 1, 2 and 8 bytes, a
+// call: m = 6 187 us with 256 threads, 192 with 512; m = 32 260 and 205).
+constexpr int rows_threads(int M) { return M > 16 ? 512 : 256; }
+constexpr uint32_t rows_buffer(int M) { return M > 16 ? 36864 : 20480; }
+
+// The row kernels take every record a tile of 16 of which fits the buffer and whose
+// words do not outnumber the threads; the gathered route is behind at every width
+// measured (6 * 10^8 bytes, m = 8: rows of 20, 64, 256 and 1024 bytes 929, 689, 559
+// and 505 us gathered, 347, 317, 260 and 221 whole).
+constexpr uint32_t kMaxRowBytes = 1024;
+static_assert(16 * kMaxRowBytes <= rows_buffer(2) && kMaxRowBytes / 4 <= rows_threads(2), "tile of 16");
+
+template <class D, int M, int ITEMS, bool RECORD>
+mdx_status launch_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
+    constexpr int TS = rows_threads(M);
+    auto scatter = rows_scatter_kernel<D, M, TS, ITEMS, RECORD>;
+    using SL = RowsSmem<M, TS, ITEMS>;
+    const size_t smem = SL::bytes(a.buf_bytes);
+    // the shared-memory limit is set for the largest buffers, once per kernel
+    int blocks = 0, sms = 0;
+    if (host::occupancy(reinterpret_cast<const void*>(scatter), SL::bytes(rows_buffer(M)), &blocks,
+                        &sms, TS) != cudaSuccess)
+        return MDX_ERR_CUDA;
+    uint32_t G = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
+    G = std::min(std::min(G, a.p.num_tiles), std::min(max_stride, host::kMaxChunks));
+    a.p.num_chunks = G;
+    a.p.chunk_stride = (G + 3u) & ~3u;
+    if (a.p.headflags != nullptr &&
+        cudaMemsetAsync(a.p.headflags, 0, a.p.n * sizeof(uint32_t), st) != cudaSuccess)
+        return MDX_ERR_CUDA;
+    rows_count_kernel<D, M><<<G, kRowsCountThreads, 0, st>>>(a, d);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G);
+    cfg.blockDim = dim3(TS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, scatter, a, d) != cudaSuccess) return MDX_ERR_CUDA;
+    return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
+}
+
+template <class D, int M, bool RECORD>
+mdx_status run_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
+    constexpr uint32_t TS = rows_threads(M);
+    uint32_t row_bytes = 0;
+    for (uint32_t c = 0; c < a.num_cols; c++) row_bytes += a.col[c].bytes;
+    // eight rows a thread where that many (three quarters of them) fit the buffer,
+    // else four; shorter tiles when that gives every SM two of them
+    const uint32_t fit = rows_buffer(M) / row_bytes;
+    const bool eight = fit >= 6 * TS;
+    uint32_t T = std::min(fit & ~15u, TS * (eight ? 8u : 4u));
+    while (T > 256 && a.p.n / T < 296) T = (T / 2) & ~15u;
+    a.tile_rows = T;
+    uint32_t off = 0;
+    a.all_bulk = 1;
+    for (uint32_t c = 0; c < a.num_cols; c++) {
+        a.col[c].offset = off;
+        off += T * a.col[c].bytes;  // T is a multiple of 16: 16-byte aligned
+        a.col[c].bulk = reinterpret_cast<uintptr_t>(a.col[c].in) % 16 == 0;
+        a.all_bulk = a.all_bulk && a.col[c].bulk;
+    }
+    a.key_offset = RECORD ? 0u : a.col[a.end[0]].offset;  // the first of the 4-byte columns
+    a.buf_bytes = (off + 127u) & ~127u;
+    a.p.num_tiles = static_cast<uint32_t>((a.p.n + T - 1) / T);
+    return eight ? launch_rows<D, M, 8, RECORD>(a, d, max_stride, st)
+                 : launch_rows<D, M, 4, RECORD>(a, d, max_stride, st);
+}
+
+template <class D, bool RECORD>
+mdx_status rows_by_bound(const RowsArgs& a, D d, uint32_t max_stride, cudaStream_t st) {
+    switch (host::class_bound(a.p.m)) {
+        case 2: return run_rows<D, 2, RECORD>(a, d, max_stride, st);
+        case 4: return run_rows<D, 4, RECORD>(a, d, max_stride, st);
+        case 8: return run_rows<D, 8, RECORD>(a, d, max_stride, st);
+        case 16: return run_rows<D, 16, RECORD>(a, d, max_stride, st);
+        case 32: return run_rows<D, 32, RECORD>(a, d, max_stride, st);
+        default: return run_rows<D, 64, RECORD>(a, d, max_stride, st);
+    }
+}
+
+// Rows held in a.col[0 .. num_cols); the keys are the first words of column 0.  The
+// workspace is that of `layout`; the chunk counts may take the room of the record
+// arrays, which the row kernels do not use.
+template <bool RECORD>
+mdx_status partition_rows(RowsArgs a, uint64_t n, mdx_discr discr, uint32_t* d_sizes,
+                          uint32_t* d_headflags, unsigned char* ws, const Layout& w,
+                          cudaStream_t st) {
+    a.p = PlainArgs{};
+    a.p.n = n;
+    a.p.m = discr.m;
+    a.p.chunk_cnt = reinterpret_cast<uint32_t*>(ws + w.L.chunk_cnt);
+    a.p.class_base = reinterpret_cast<uint32_t*>(ws + w.L.class_base);
+    a.p.class_tot = reinterpret_cast<uint32_t*>(ws + w.L.class_tot);
+    a.p.sizes = d_sizes;
+    a.p.headflags = d_headflags;
+    a.p.error = &reinterpret_cast<host::WsHeader*>(ws)->error;
+    a.p.prefix_in_scatter = 1;
+    a.keys = a.col[0].in;
+    a.key_stride = a.col[0].bytes;
+    if (!RECORD) {  // the wider first; the key stays the first of its width
+        std::stable_sort(a.col, a.col + a.num_cols,
+                         [](const RowsColumn& x, const RowsColumn& y) { return x.bytes > y.bytes; });
+        for (uint32_t q = 0; q < 4; q++)
+            a.end[q] = static_cast<uint32_t>(
+                std::count_if(a.col, a.col + a.num_cols,
+                              [q](const RowsColumn& x) { return x.bytes >= (8u >> q); }));
+    }
+    const uint32_t M = host::class_bound(discr.m);
+    const uint32_t max_stride = static_cast<uint32_t>(std::min<uint64_t>(
+                                    (w.total - w.L.chunk_cnt) / (4ull * M), host::kMaxChunks)) & ~3u;
+    if (host::use_mask(discr))
+        return rows_by_bound<DiscrMask, RECORD>(a, DiscrMask{discr.m - 1u}, max_stride, st);
+    return rows_by_bound<DiscrMod, RECORD>(a, DiscrMod::make(discr.m), max_stride, st);
 }
 
 }  // namespace wide
@@ -167,6 +254,19 @@ mdx_status mdx_partition_records(const void* d_in, void* d_out, uint64_t n, uint
     if (d_ws == nullptr || ws_bytes < w.total || reinterpret_cast<uintptr_t>(d_ws) % host::kAlign)
         return MDX_ERR_WORKSPACE;
     unsigned char* ws = static_cast<unsigned char*>(d_ws);
+    if (record_bytes <= wide::kMaxRowBytes) {
+        RowsArgs a{};
+        a.num_cols = 1;
+        RowsColumn& c = a.col[0];
+        c.in = static_cast<const unsigned char*>(d_in);
+        c.out = static_cast<unsigned char*>(d_out);
+        c.bytes = record_bytes;
+        c.unit = 16;
+        while (record_bytes % c.unit || reinterpret_cast<uintptr_t>(d_in) % c.unit ||
+               reinterpret_cast<uintptr_t>(d_out) % c.unit)
+            c.unit /= 2;  // 4 divides all three
+        return wide::partition_rows<true>(a, n, discr, d_sizes, d_headflags, ws, w, st);
+    }
     s = wide::key_order(static_cast<const unsigned char*>(d_in), record_bytes, n, discr, d_sizes,
                         d_headflags, ws, w, st);
     if (s != MDX_OK) return s;
@@ -185,7 +285,7 @@ size_t mdx_columns_workspace_size(uint64_t n, uint32_t m) {
 mdx_status mdx_partition_columns(const mdx_column* cols, uint32_t num_cols, uint64_t n,
                                  mdx_discr discr, uint32_t* d_sizes, uint32_t* d_headflags,
                                  void* d_ws, size_t ws_bytes, mdx_stream_t stream) {
-    if (cols == nullptr || num_cols < 1 || num_cols > static_cast<uint32_t>(wide::kMaxCols))
+    if (cols == nullptr || num_cols < 1 || num_cols > static_cast<uint32_t>(kMaxCols))
         return MDX_ERR_INVALID;
     mdx_status s = host::check_discr(discr);
     if (s != MDX_OK) return s;
@@ -196,8 +296,8 @@ mdx_status mdx_partition_columns(const mdx_column* cols, uint32_t num_cols, uint
             return MDX_ERR_CUDA;
         return MDX_OK;
     }
-    wide::Cols c{};
-    c.num = num_cols;
+    RowsArgs a{};
+    a.num_cols = num_cols;
     for (uint32_t i = 0; i < num_cols; i++) {
         const uint32_t b = cols[i].elem_bytes;
         if ((b != 1 && b != 2 && b != 4 && b != 8) || cols[i].in == nullptr || cols[i].out == nullptr ||
@@ -212,20 +312,16 @@ mdx_status mdx_partition_columns(const mdx_column* cols, uint32_t num_cols, uint
                 if (o < y + n * cols[j].elem_bytes && y < o + n * b) return MDX_ERR_INVALID;
             }
         }
-        c.in[i] = cols[i].in;
-        c.out[i] = cols[i].out;
-        c.bytes[i] = b;
+        a.col[i].in = static_cast<const unsigned char*>(cols[i].in);
+        a.col[i].out = static_cast<unsigned char*>(cols[i].out);
+        a.col[i].bytes = b;
+        a.col[i].unit = b;
     }
     const wide::Layout w = wide::layout(n, discr.m);
     if (d_ws == nullptr || ws_bytes < w.total || reinterpret_cast<uintptr_t>(d_ws) % host::kAlign)
         return MDX_ERR_WORKSPACE;
-    unsigned char* ws = static_cast<unsigned char*>(d_ws);
-    s = wide::key_order(static_cast<const unsigned char*>(cols[0].in), 4, n, discr, d_sizes,
-                        d_headflags, ws, w, st);
-    if (s != MDX_OK) return s;
-    wide::gather_columns<<<wide::grid_for(n), wide::kThreads, 0, st>>>(
-        c, reinterpret_cast<const uint64_t*>(ws + w.rec_out), n);
-    return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
+    return wide::partition_rows<false>(a, n, discr, d_sizes, d_headflags,
+                                       static_cast<unsigned char*>(d_ws), w, st);
 }
 
 }  // extern "C"

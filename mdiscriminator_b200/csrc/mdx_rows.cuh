@@ -59,6 +59,9 @@ struct DiscrRow {
     __device__ __forceinline__ uint32_t operator()(uint32_t v) const { return v >> 16; }
 };
 
+template <>
+struct CheapClass<DiscrRow> : std::true_type {};
+
 template <class D, int M>
 __global__ void __launch_bounds__(kRowsCountThreads, 4) rows_count_kernel(const __grid_constant__ RowsArgs a, D d) {
     constexpr int W = kRowsCountThreads / 32;

@@ -14,16 +14,15 @@
 //                   block totals, records the counts and resets the tickets.
 //   seg_plan_emit   writes the run entries {segment, [p0, p1), last run of
 //                   the segment} and the group heads, in element order.
-//   seg_main        persistent; CTAs take tickets for batches of groups.
-//                   Each group's range is read into shared memory by one bulk
-//                   copy and partitioned by the whole CTA (seg_group_cta:
-//                   every thread owns ~L/256 consecutive elements whatever the
-//                   segment lengths; a segmented scan of per-thread class
-//                   counts, the segments' class bases in shared memory) into
-//                   a shared output image written back with 16-byte stores --
-//                   one HBM read and one write per element;
-//   seg_run_count   the class counts of every run of the large segments,
-//                   one CTA per run (16-byte loads, warp reductions).
+//   seg_main        persistent; CTAs take tickets for batches of groups.  Each
+//                   group's range is read into shared memory by one bulk copy and
+//                   partitioned by the whole CTA (seg_group_cta: every thread owns
+//                   consecutive elements whatever the segment lengths; one scan of
+//                   per-thread class counts gives every segment's sizes and every
+//                   element's place) into a shared output image that one bulk store
+//                   writes back -- one HBM read and one write per element;
+//   seg_run_count   the class counts of every run of the large segments, one CTA per
+//                   run (16-byte loads, warp reductions);
 //   seg_run_scan    per large segment (a lane, or a warp for many runs):
 //                   the runs' exclusive class prefixes, the segment's sizes
 //                   and head flags, and every run's output position per class.
@@ -59,7 +58,7 @@ constexpr int kGroupBatch = 8;   // small-segment groups per ticket of seg_main
 constexpr int kMaxGroupBatch = 32;
 
 struct SegHeader {      // lives at the start of the segmented workspace
-    uint32_t ticket;    // seg_main's group-batch tickets (reset by the planner)
+    uint32_t ticket;    // seg_main's tickets (reset by the planner)
     uint32_t error;     // latched error bits
     uint32_t num_mids;  // medium segments this call
     uint32_t num_runs;  // large-segment runs this call
@@ -360,6 +359,11 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
 }
 
 // --------------------------------------------------------------- main kernel --
+template <int M, int THREADS>
+struct GroupScratch;
+template <int M, int THREADS>
+constexpr size_t group_scratch_bytes();
+
 template <class V, int M, int THREADS, int STAGES>
 struct SegSmem {
     using G = TileGeom<V, THREADS, M>;
@@ -372,87 +376,106 @@ struct SegSmem {
     static constexpr int kGroupElems =
         static_cast<int>(group_window<kTile>()) + kTile + 2 * static_cast<int>(kAU);
     static constexpr size_t kGroupBytes = 2ull * kGroupElems * sizeof(V);
-    static constexpr size_t kBytes = 128 + kGroupBytes;  // seg_main
+    static constexpr size_t kBytes = 128 + kGroupBytes + group_scratch_bytes<M, THREADS>();  // seg_main
     // seg_run_scatter: TMA ring + tile stage + count matrix
     static constexpr size_t kRingBytes = static_cast<size_t>(STAGES) * kTile * sizeof(V);
     static constexpr size_t kRunBytes = 1024 + kRingBytes + G::kStageBytes + G::kCntBytes;
 };
 
-// Per-thread class counters in 16-bit fields (M <= 16: (M+1)/2 words), wide
-// enough for any count within one group (< 2P < 2^16 elements).
-template <int M>
-struct HalfCounts {
-    static constexpr int NW = (M + 1) / 2;
-    uint32_t w[NW];
-    __device__ __forceinline__ void zero() {
+// ------------------------------------------------------------ small segments --
+// Shared state of one group (at most kGroupSegs segments).  Positions y count from
+// the 16-byte address at or before the group's first element, in the input buffer
+// and in the output image alike.
+template <int M, int THREADS>
+struct GroupScratch {
+    static constexpr int NB = M > 4 ? M / 4 : 1;  // words of byte counts
+    static constexpr int NH = M / 2;              // words of 16-bit counts
+    uint32_t hcnt[kGroupSegs][NB];     // its owner thread's class counts before the head
+    uint32_t hpre[kGroupSegs][NH];     // the group's class counts before the head
+    uint32_t hcur[kGroupSegs][NH];     // first position of each class of the segment
+    uint32_t col[NH][THREADS];         // class counts before each thread's elements; before
+                                       // that byte counters (M = 16), after it cursors (M > 4)
+    uint32_t wagg[NH][THREADS / 32];
+    uint16_t hpos[kGroupSegs + 2];     // head of each segment; [nseg] = the group's end
+    uint8_t msz[kGroupSegs];           // the segment's class count (per-segment m)
+};
+
+template <int M, int THREADS>
+constexpr size_t group_scratch_bytes() {
+    return sizeof(GroupScratch<M, THREADS>);
+}
+
+// Class counts of one thread's elements, a byte per class (a thread owns at most
+// 36): in registers up to 8 classes, in the thread's column above.
+template <int M, int THREADS>
+struct GroupCounts {
+    using GS = GroupScratch<M, THREADS>;
+    uint64_t w;
+    unsigned char* mine;
+    __device__ __forceinline__ void init(GS& gs) {
+        w = 0;
+        if constexpr (M > 8) {
+            mine = reinterpret_cast<unsigned char*>(&gs.col[0][threadIdx.x]);
 #pragma unroll
-        for (int q = 0; q < NW; q++) w[q] = 0;
-    }
-    __device__ __forceinline__ uint32_t get(uint32_t c) const {
-        if constexpr (NW == 2) {  // four fields: one 64-bit shift
-            const uint64_t x = (static_cast<uint64_t>(w[1]) << 32) | w[0];
-            return static_cast<uint32_t>(x >> (c << 4)) & 0xffffu;
-        } else if constexpr (NW == 4) {  // eight fields: two 64-bit halves
-            const uint64_t lo = (static_cast<uint64_t>(w[1]) << 32) | w[0];
-            const uint64_t hi = (static_cast<uint64_t>(w[3]) << 32) | w[2];
-            return static_cast<uint32_t>(((c & 4u) ? hi : lo) >> ((c & 3u) << 4)) & 0xffffu;
-        } else if constexpr (NW == 8) {  // sixteen fields: four 64-bit quarters
-            uint64_t x = (static_cast<uint64_t>(w[1]) << 32) | w[0];
-#pragma unroll
-            for (int q = 1; q < 4; q++)
-                x = (c >> 2) == static_cast<uint32_t>(q)
-                        ? (static_cast<uint64_t>(w[2 * q + 1]) << 32) | w[2 * q]
-                        : x;
-            return static_cast<uint32_t>(x >> ((c & 3u) << 4)) & 0xffffu;
-        } else {
-            uint32_t x = w[0];
-#pragma unroll
-            for (int q = 1; q < NW; q++) x = (c >> 1) == static_cast<uint32_t>(q) ? w[q] : x;
-            return (x >> ((c & 1u) << 4)) & 0xffffu;
+            for (int q = 0; q < GS::NB; q++) gs.col[q][threadIdx.x] = 0u;
         }
     }
     __device__ __forceinline__ void inc(uint32_t c) {
-        if constexpr (NW == 2) {
-            uint64_t x = (static_cast<uint64_t>(w[1]) << 32) | w[0];
-            x += 1ull << (c << 4);
-            w[0] = static_cast<uint32_t>(x);
-            w[1] = static_cast<uint32_t>(x >> 32);
-        } else if constexpr (NW == 4) {
-            uint64_t lo = (static_cast<uint64_t>(w[1]) << 32) | w[0];
-            uint64_t hi = (static_cast<uint64_t>(w[3]) << 32) | w[2];
-            const uint64_t one = 1ull << ((c & 3u) << 4);
-            if (c & 4u) hi += one; else lo += one;
-            w[0] = static_cast<uint32_t>(lo);
-            w[1] = static_cast<uint32_t>(lo >> 32);
-            w[2] = static_cast<uint32_t>(hi);
-            w[3] = static_cast<uint32_t>(hi >> 32);
-        } else if constexpr (NW == 8) {
-            const uint64_t one = 1ull << ((c & 3u) << 4);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                uint64_t x = (static_cast<uint64_t>(w[2 * q + 1]) << 32) | w[2 * q];
-                if ((c >> 2) == static_cast<uint32_t>(q)) x += one;
-                w[2 * q] = static_cast<uint32_t>(x);
-                w[2 * q + 1] = static_cast<uint32_t>(x >> 32);
-            }
+        if constexpr (M <= 4) {
+            w = static_cast<uint32_t>(w) + (1u << (c << 3));
+        } else if constexpr (M <= 8) {
+            w += 1ull << (c << 3);
         } else {
-            const uint32_t one = 1u << ((c & 1u) << 4);
-#pragma unroll
-            for (int q = 0; q < NW; q++) w[q] += (c >> 1) == static_cast<uint32_t>(q) ? one : 0u;
+            unsigned char& x = mine[(c >> 2) * (4u * THREADS) + (c & 3u)];
+            x = static_cast<unsigned char>(x + 1u);
         }
+    }
+    __device__ __forceinline__ uint32_t word(const GS& gs, int q) const {
+        if constexpr (M > 8) return gs.col[q][threadIdx.x];
+        else return static_cast<uint32_t>(w >> (32 * q));
     }
 };
 
-// Shared state of one group partition (at most kGroupSegs non-empty
-// segments).
+// 16-bit pairs (classes 2 i, 2 i + 1) of a word of byte counts.
+__device__ __forceinline__ uint32_t widen_lo(uint32_t x) { return __byte_perm(x, 0u, 0x4140); }
+__device__ __forceinline__ uint32_t widen_hi(uint32_t x) { return __byte_perm(x, 0u, 0x4342); }
+template <int M>
+__device__ __forceinline__ uint32_t widen_pair(uint32_t x, int h) {  // pair h of word h / 2
+    return (h & 1) ? widen_hi(x) : widen_lo(x);
+}
+
+// Where a thread's next element of each class goes: 16-bit fields, in registers up
+// to 4 classes, in the thread's column above.
 template <int M, int THREADS>
-struct GroupScratch {
-    static constexpr int NW = HalfCounts<M>::NW;
-    uint32_t base[kGroupSegs][NW];  // class bases of each non-empty segment (u16 pairs)
-    uint32_t wagg[THREADS / 32][NW + 1];
-    uint16_t hpos[kGroupSegs + 1];  // head of each non-empty segment in the group; [nseg] = L
-    uint16_t sidx[kGroupSegs];      // its index - h
-    uint8_t msz[kGroupSegs];        // its class count (per-segment m)
+struct GroupCursors {
+    using GS = GroupScratch<M, THREADS>;
+    uint64_t w;
+    unsigned char* mine;
+    __device__ __forceinline__ void init(GS& gs) {
+        mine = reinterpret_cast<unsigned char*>(&gs.col[0][threadIdx.x]);
+        w = 0;
+    }
+    __device__ __forceinline__ void set(GS& gs, int h, uint32_t x) {
+        if constexpr (M == 2) w = x;
+        else if constexpr (M == 4) w = h == 0 ? ((w >> 32) << 32 | x) : ((w & 0xffffffffull) | static_cast<uint64_t>(x) << 32);
+        else gs.col[h][threadIdx.x] = x;
+    }
+    __device__ __forceinline__ uint32_t next(uint32_t c) {
+        if constexpr (M == 2) {
+            const uint32_t x = static_cast<uint32_t>(w);
+            w = x + (1u << (c << 4));
+            return (x >> (c << 4)) & 0xffffu;
+        } else if constexpr (M == 4) {
+            const uint32_t p = static_cast<uint32_t>(w >> (c << 4)) & 0xffffu;
+            w += 1ull << (c << 4);
+            return p;
+        } else {
+            uint16_t& x = *reinterpret_cast<uint16_t*>(mine + (c >> 1) * (4u * THREADS) + (c & 1u) * 2u);
+            const uint32_t p = x;
+            x = static_cast<uint16_t>(p + 1u);
+            return p;
+        }
+    }
 };
 
 // Offsets (and class count) of segment h + threadIdx.x of the next group,
@@ -479,248 +502,287 @@ __device__ __forceinline__ D group_discr(const SegArgs& a, const D& d, const uin
     return d;
 }
 
-// One CTA partitions one group of small segments held in shared memory
-// (element x of the group at src[x], 0 <= x < L) into the output image
-// dst[0 .. L) and writes the segments' sizes.  Every thread owns k = ~L/256
-// consecutive elements whatever the segment lengths (k odd: the threads'
-// strided shared-memory reads fall in different banks):
-//   P0  one thread per segment: ordinals of the non-empty segments and their
-//       heads; each thread finds the segment holding its first element by a
-//       binary search over the heads;
-//   P1  the class counts of the fragment after the thread's last segment
-//       head; a segment that begins and ends inside the thread's range is
-//       closed here (its class bases to shared memory, its sizes and head
-//       flags to global memory);
-//   P2  a segmented exclusive scan of those counts over the threads gives the
-//       counts of the thread's first segment before its first element;
-//   P3  the thread's first segment, if it ends in the thread's range, is
-//       closed with the scanned counts plus its part in the range;
-//   P4  every element goes to head + base[class] + its rank in the segment.
+// One CTA partitions one group of small segments held in shared memory (its element
+// y at src[y], phase <= y < end) into the output image dst and writes the segments'
+// sizes.  Every thread owns k consecutive positions whatever the segment lengths, k
+// an odd number of 16-byte words (a warp's loads then fall in different banks):
+//   heads   one thread per segment publishes its head; each thread finds the first
+//           head at or after its own range (binary search);
+//   counts  class counts of the thread's elements; where a head lies inside, the
+//           counts so far are noted for it.  A 16-byte word without a head in it
+//           (all but one in a thousand for segments of a thousand) takes no test;
+//   scan    exclusive 16-bit class counts over the threads, segments disregarded;
+//   sizes   one thread per segment: the group's class counts before its head and
+//           before the next give its sizes, and with them where each class begins;
+//   place   every element to the next position of its class: at a head those of the
+//           segment, before it those of the segment the thread's range begins in
+//           (its first positions plus what lies between its head and the range).
+// The counts are kept per class and never per segment, so no scan carries segment
+// flags and no thread closes a segment for the others.  6 * 10^7 u32 in segments
+// of up to 4096 (mean 1600), m = 4: 46 instructions an element and 167 us, where a
+// segmented scan with the segments closed by the threads that hold their ends took
+// 78 and 212; 10^5 LogNormal(ln 1024, 1.5) segments, m = 2, 4, 8, 16: 363, 368,
+// 457, 745 -> 294, 306, 361, 689 us.  What bounds it now is latency: four barriers
+// a group and 24 warps to an SM (shared memory).  Windows of P / 2 and 3 P / 4, the
+// former with four CTAs: 309 and 336 against 306 us at m = 4, 448 and 398 against
+// 361 at m = 8.  The run counts as items of this kernel, to fill the idle memory
+// pipe: 545 us for both against 306 + 157.
 template <class V, class D, int M, int THREADS>
-__device__ void seg_group_cta(const SegArgs& a, const D& d, const uint32_t* cmod, uint32_t h,
-                              uint32_t he, uint64_t r0, uint32_t L, const V* src, V* dst,
-                              GroupScratch<M, THREADS>& gs, GroupPrefetch& pf,
-                              const uint32_t* next_h, const uint32_t* next_he) {
-    using HC = HalfCounts<M>;
-    constexpr int NW = HC::NW;
+__device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, const uint32_t* cmod,
+                                              uint32_t h, uint32_t nseg, uint64_t as, uint32_t phase,
+                                              uint32_t end, const V* src, V* dst,
+                                              GroupScratch<M, THREADS>& gs, uint32_t qn0, uint32_t nq) {
+    using GS = GroupScratch<M, THREADS>;
+    constexpr int NB = GS::NB, NH = GS::NH;
     constexpr int W = THREADS / 32;
-    static_assert(static_cast<int>(kGroupSegs) <= THREADS, "one thread per segment");
+    constexpr uint32_t VE = 16 / sizeof(V);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t k = ((L + THREADS - 1) / THREADS) | 1u;
-    const uint32_t lo = min(tid * k, L), hi = min(lo + k, L);
+    const uint32_t k = nq * VE, lo = static_cast<uint32_t>(tid) * k;
 
-    // ---- P0
-    const uint64_t sg = static_cast<uint64_t>(h) + tid;
-    uint32_t ne = 0, x0 = 0, x1 = 0, ms = a.m;
-    if (sg < he && tid < static_cast<int>(kGroupSegs)) {
-        uint64_t o0, o1;
-        if (pf.valid) {
-            o0 = pf.o0;
-            o1 = pf.o1;
-            ms = pf.m;
-        } else {
-            o0 = a.offsets[sg];
-            o1 = a.offsets[sg + 1];
-            if (a.seg_m != nullptr) ms = min(max(a.seg_m[sg], 1u), a.m_bound);
-        }
-        x0 = static_cast<uint32_t>(o0 - r0);
-        x1 = static_cast<uint32_t>(o1 - r0);
-        ne = (o1 > o0 && o0 >= r0 && x1 <= L) ? 1u : 0u;
-        if (o1 == o0 && a.seg_sizes != nullptr)
-            for (uint32_t c = 0; c < a.m; c++) a.seg_sizes[sg * a.m + c] = 0u;
-    }
-    const uint32_t incl = warp_incl_scan(ne);
-    if (lane == 31) gs.wagg[warp][0] = incl;
-    __syncthreads();
-    // the next group's head and end are visible now: start its loads
-    pf.valid = next_h != nullptr;
-    if (pf.valid) {
-        const uint64_t ns = static_cast<uint64_t>(*next_h) + tid;
-        pf.m = a.m;
-        if (ns < *next_he && tid < static_cast<int>(kGroupSegs)) {
-            pf.o0 = a.offsets[ns];
-            pf.o1 = a.offsets[ns + 1];
-            if (a.seg_m != nullptr) pf.m = min(max(a.seg_m[ns], 1u), a.m_bound);
-        }
-    }
-    uint32_t before = 0, nseg = 0;
+    // ---- counts
+    GroupCounts<M, THREADS> cnt;
+    cnt.init(gs);
+    {
+        uint32_t qn = qn0, nxt = gs.hpos[qn0];
+        D dc = group_discr(a, d, cmod, qn > 0u ? gs.msz[qn - 1u] : a.m);
+        for (uint32_t j = 0; j < nq; j++) {
+            const uint32_t y0 = lo + j * VE;
+            if (y0 >= end) break;
+            V v[VE];
+            unpack16_to<V>(*reinterpret_cast<const uint4*>(src + y0), v);
+            if (nxt >= y0 + VE) {
 #pragma unroll
-    for (int w = 0; w < W; w++) {
-        const uint32_t x = gs.wagg[w][0];
-        before += w < warp ? x : 0u;
-        nseg += x;
-    }
-    if (ne) {
-        const uint32_t q = before + incl - 1u;
-        gs.hpos[q] = static_cast<uint16_t>(x0);
-        gs.sidx[q] = static_cast<uint16_t>(tid);
-        gs.msz[q] = static_cast<uint8_t>(ms);
-    }
-    if (tid == 0) gs.hpos[nseg] = static_cast<uint16_t>(L);
-    __syncthreads();
-
-    // ---- P1
-    const bool active = lo < hi && nseg > 0;
-    uint32_t q0 = 0;  // the last non-empty segment with head <= lo (hpos[nseg] = L > lo)
-    if (active) {
-        uint32_t qb = nseg;
-        while (qb - q0 > 1u) {
-            const uint32_t mid = (q0 + qb) >> 1;
-            if (gs.hpos[mid] <= lo) q0 = mid; else qb = mid;
+                for (uint32_t e = 0; e < VE; e++) cnt.inc(dc(v[e]));
+            } else {
+#pragma unroll
+                for (uint32_t e = 0; e < VE; e++) {
+                    const uint32_t y = y0 + e;
+                    while (nxt == y && qn < nseg) {
+#pragma unroll
+                        for (int q = 0; q < NB; q++) gs.hcnt[qn][q] = cnt.word(gs, q);
+                        dc = group_discr(a, d, cmod, gs.msz[qn]);
+                        nxt = gs.hpos[++qn];
+                    }
+                    if (qn > 0u && y < end) cnt.inc(dc(v[e]));
+                }
+            }
         }
     }
-    const bool head_at_lo = active && gs.hpos[q0] == lo;
-    const D d0 = active ? group_discr(a, d, cmod, gs.msz[q0]) : d;
-    // segment qq ends here with class totals `tot`: its class bases (shared),
-    // sizes and head flags (global)
-    auto close = [&](uint32_t qq, const HC& tot) {
-        const uint64_t s = static_cast<uint64_t>(h) + gs.sidx[qq];
-        const uint64_t xh = r0 + gs.hpos[qq];
+
+    // ---- scan over the threads: exclusive counts within the warp, warp totals
+    uint32_t inc[NH];
+    {
+        uint32_t own[NH];
+#pragma unroll
+        for (int i = 0; i < NH; i++) own[i] = widen_pair<M>(cnt.word(gs, i / 2), i);
+#pragma unroll
+        for (int i = 0; i < NH; i++) {
+            inc[i] = warp_incl_scan(own[i]);
+            if (lane == 31) gs.wagg[i][warp] = inc[i];
+            inc[i] -= own[i];
+            gs.col[i][tid] = inc[i];
+        }
+    }
+    __syncthreads();
+    // the warps before this one, by the first lanes of every warp (lane w: warp w)
+    uint32_t wpre[NH], tot[NH];  // lane w: counts before warp w; the group's
+#pragma unroll
+    for (int i = 0; i < NH; i++) {
+        const uint32_t x = lane < W ? gs.wagg[i][lane] : 0u;
+        uint32_t in = x;
+#pragma unroll
+        for (int dd = 1; dd < W; dd <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, in, dd);
+            if (lane >= dd) in += up;
+        }
+        wpre[i] = in - x;
+        tot[i] = __shfl_sync(0xffffffffu, in, W - 1);
+        inc[i] += __shfl_sync(0xffffffffu, wpre[i], warp);
+    }
+
+    // ---- sizes (whole warps, so that the warp totals can be looked up by shuffles)
+    if (static_cast<uint32_t>(warp) * 32u < nseg) {
+        const bool mine = static_cast<uint32_t>(tid) < nseg;
+        const uint32_t hq = gs.hpos[mine ? tid : 0], hn = gs.hpos[mine ? tid + 1 : 0];
+        uint32_t p0[NH], p1[NH];
+        auto before = [&](uint32_t q, uint32_t y, uint32_t (&p)[NH]) {  // counts before head q at y
+            const bool inside = y < end && q < nseg;
+            const uint32_t t = inside ? y / k : 0u;
+#pragma unroll
+            for (int i = 0; i < NH; i++) {
+                const uint32_t w = __shfl_sync(0xffffffffu, wpre[i], t >> 5);
+                p[i] = inside ? w + gs.col[i][t] + widen_pair<M>(gs.hcnt[q][i / 2], i) : tot[i];
+            }
+        };
+        before(tid, hq, p0);
+        before(tid + 1, hn, p1);
+        const uint64_t s = static_cast<uint64_t>(h) + tid;
         uint32_t off = 0;
-        uint32_t bw[NW];
+        if (mine) {
 #pragma unroll
-        for (int w = 0; w < NW; w++) bw[w] = 0;
-#pragma unroll
-        for (int c = 0; c < M; c++) {
-            const uint32_t t = tot.get(c);
-            bw[c >> 1] |= off << (16 * (c & 1));
-            if (a.seg_sizes != nullptr && static_cast<uint32_t>(c) < a.m) a.seg_sizes[s * a.m + c] = t;
-            if (a.headflags != nullptr && t > 0) a.headflags[xh + off] = t;
-            off += t;
-        }
-#pragma unroll
-        for (int w = 0; w < NW; w++) gs.base[qq][w] = bw[w];
-    };
-    // the counts of the fragment after the last head in (lo, hi) (all of the
-    // range without one); segments that begin and end inside the range are
-    // closed on the way, the first segment's part is kept for after the scan
-    HC tail, pre;
-    tail.zero();
-    pre.zero();
-    bool inner = false;  // a segment head in (lo, hi)
-    if (active) {
-        uint32_t q = q0, nxt = gs.hpos[q0 + 1];
-        D dc = d0;
-        for (uint32_t x = lo; x < hi; x++) {
-            if (x == nxt) {
-                if (inner) close(q, tail);
-                else pre = tail;
-                inner = true;
-                tail.zero();
-                q++;
-                nxt = gs.hpos[q + 1];
-                dc = group_discr(a, d, cmod, gs.msz[q]);
+            for (int i = 0; i < NH; i++) {
+                const uint32_t n = p1[i] - p0[i];  // each 16-bit field is no smaller
+                const uint32_t n0 = n & 0xffffu, n1 = n >> 16;
+                const uint32_t o0 = off, o1 = off + n0;
+                off = o1 + n1;
+                gs.hpre[tid][i] = p0[i];
+                gs.hcur[tid][i] = (hq + o0) | ((hq + o1) << 16);
+                if (a.seg_sizes != nullptr) {
+                    if (2u * i < a.m) a.seg_sizes[s * a.m + 2 * i] = n0;
+                    if (2u * i + 1u < a.m) a.seg_sizes[s * a.m + 2 * i + 1] = n1;
+                }
+                if (a.headflags != nullptr) {
+                    if (n0 > 0u) a.headflags[as + hq + o0] = n0;
+                    if (n1 > 0u) a.headflags[as + hq + o1] = n1;
+                }
             }
-            tail.inc(dc(src[x]));
-        }
-        if (inner && hi == nxt) close(q, tail);
-        if (!inner) pre = tail;
-    }
-
-    // ---- P2: segmented exclusive scan of (reset, counts) over the threads
-    uint32_t f = (head_at_lo || inner) ? 1u : 0u;
-    HC v = tail;
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-        const uint32_t fu = __shfl_up_sync(0xffffffffu, f, dd);
-        HC vu;
-#pragma unroll
-        for (int w = 0; w < NW; w++) vu.w[w] = __shfl_up_sync(0xffffffffu, v.w[w], dd);
-        if (lane >= dd) {
-            if (!f) {
-#pragma unroll
-                for (int w = 0; w < NW; w++) v.w[w] += vu.w[w];
-            }
-            f |= fu;
         }
     }
-    if (lane == 31) {
-        gs.wagg[warp][0] = f;
-#pragma unroll
-        for (int w = 0; w < NW; w++) gs.wagg[warp][1 + w] = v.w[w];
-    }
-    const uint32_t fe = __shfl_up_sync(0xffffffffu, f, 1);
-    HC ve;
-#pragma unroll
-    for (int w = 0; w < NW; w++) ve.w[w] = __shfl_up_sync(0xffffffffu, v.w[w], 1);
-    __syncthreads();
-    HC carry;
-    carry.zero();
-    for (int w = 0; w < warp; w++) {
-        const bool fw = gs.wagg[w][0] != 0u;
-#pragma unroll
-        for (int q = 0; q < NW; q++) carry.w[q] = (fw ? 0u : carry.w[q]) + gs.wagg[w][1 + q];
-    }
-    if (lane > 0) {
-#pragma unroll
-        for (int q = 0; q < NW; q++) carry.w[q] = (fe ? 0u : carry.w[q]) + ve.w[q];
-    }
-    if (head_at_lo) carry.zero();
-
-    // ---- P3: the first segment ends at the first head inside, or exactly at hi
-    if (active) {
-        const bool ends = inner || hi == gs.hpos[q0 + 1];
-        if (ends) {
-            HC t;
-#pragma unroll
-            for (int w = 0; w < NW; w++) t.w[w] = carry.w[w] + pre.w[w];
-            close(q0, t);
-        }
-    }
+    // the output image is about to be rewritten: the previous group's bulk store
+    // must have finished reading it
+    if (tid == 0) bulk_wait_read<0>();
     __syncthreads();
 
-    // ---- P4: positions = head + class base + rank in the segment (packed per class)
-    if (active) {
-        uint32_t q = q0, nxt = gs.hpos[q0 + 1], xh = gs.hpos[q0];
-        HC cur;
+    // ---- place
+    {
+        uint32_t qn = qn0, nxt = gs.hpos[qn0];
+        D dc = group_discr(a, d, cmod, qn > 0u ? gs.msz[qn - 1u] : a.m);
+        GroupCursors<M, THREADS> cur;
+        cur.init(gs);
+        if (qn > 0u) {
 #pragma unroll
-        for (int w = 0; w < NW; w++) cur.w[w] = gs.base[q0][w] + carry.w[w];
-        D dc = d0;
-        for (uint32_t x = lo; x < hi; x++) {
-            if (x == nxt) {
-                q++;
-                xh = x;
-                nxt = gs.hpos[q + 1];
+            for (int i = 0; i < NH; i++)
+                cur.set(gs, i, gs.hcur[qn - 1u][i] + (inc[i] - gs.hpre[qn - 1u][i]));
+        }
+        for (uint32_t j = 0; j < nq; j++) {
+            const uint32_t y0 = lo + j * VE;
+            if (y0 >= end) break;
+            V v[VE];
+            unpack16_to<V>(*reinterpret_cast<const uint4*>(src + y0), v);
+            if (nxt >= y0 + VE) {
 #pragma unroll
-                for (int w = 0; w < NW; w++) cur.w[w] = gs.base[q][w];
-                dc = group_discr(a, d, cmod, gs.msz[q]);
+                for (uint32_t e = 0; e < VE; e++) dst[cur.next(dc(v[e]))] = v[e];
+            } else {
+#pragma unroll
+                for (uint32_t e = 0; e < VE; e++) {
+                    const uint32_t y = y0 + e;
+                    while (nxt == y && qn < nseg) {
+#pragma unroll
+                        for (int i = 0; i < NH; i++) cur.set(gs, i, gs.hcur[qn][i]);
+                        dc = group_discr(a, d, cmod, gs.msz[qn]);
+                        nxt = gs.hpos[++qn];
+                    }
+                    if (qn > 0u && y < end) dst[cur.next(dc(v[e]))] = v[e];
+                }
             }
-            const V v = src[x];
-            const uint32_t c = dc(v);
-            const uint32_t pos = xh + cur.get(c);
-            cur.inc(c);
-            if (pos < L) dst[pos] = v;
         }
     }
 }
 
+// The class counts of run j of a large segment by one CTA: 16-byte loads eight deep
+// per thread, per-thread packed counters, warp reductions and one barrier (`red` is
+// used in turns by the caller's parity).
+template <class V, class D, int M, int THREADS>
+__device__ __forceinline__ void count_run(const SegArgs& a, const D& d, uint32_t j,
+                                          uint32_t (*red)[M]) {
+    constexpr uint32_t AU = 16 / sizeof(V);
+    constexpr int W = THREADS / 32;
+    constexpr int UNROLL = M <= 8 ? 8 : 4;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const V* in = static_cast<const V*>(a.in);
+    const bool in_vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+    const RunEntry ent = a.runs[j];
+    const D dj = seg_discr(a, d, ent.seg);
+    PackedCounts<M> pc;
+    pc.init();
+    const uint64_t p0 = ent.p0, p1 = ent.p1;
+    const uint64_t vs = in_vec ? min((p0 + AU - 1u) & ~static_cast<uint64_t>(AU - 1u), p1) : p1;
+    const uint64_t ve = in_vec ? max(vs, p1 & ~static_cast<uint64_t>(AU - 1u)) : p1;
+    uint32_t k = 0;
+    auto edge = [&](uint64_t e) {
+        pc.add(dj(in[e]));
+        if (++k == 8u) {
+            pc.fold();
+            k = 0;
+        }
+    };
+    for (uint64_t e = p0 + tid; e < vs; e += THREADS) edge(e);
+    for (uint64_t e = ve + tid; e < p1; e += THREADS) edge(e);
+    pc.fold();
+    const uint4* vp = reinterpret_cast<const uint4*>(in + vs);
+    const uint32_t nv = static_cast<uint32_t>((ve - vs) / AU);
+    for (uint32_t q = tid; q < nv; q += THREADS * UNROLL) {
+        uint4 r[UNROLL];
+#pragma unroll
+        for (int uu = 0; uu < UNROLL; uu++)
+            if (q + uu * THREADS < nv) r[uu] = __ldg(vp + q + uu * THREADS);
+#pragma unroll
+        for (int uu = 0; uu < UNROLL; uu++) {
+            if (q + uu * THREADS < nv) {
+                V e[AU];
+                unpack16_to<V>(r[uu], e);
+#pragma unroll
+                for (uint32_t z = 0; z < AU; z++) pc.add(dj(e[z]));
+            }
+            if (uu & 1) pc.fold();  // every two vectors: <= 8 increments
+        }
+    }
+    pc.finish();
+#pragma unroll
+    for (int c = 0; c < M; c++) {
+        const uint32_t x = warp_sum(pc.acc[c]);
+        if (lane == 0) red[warp][c] = x;
+    }
+    __syncthreads();
+    if (tid < static_cast<uint32_t>(M)) {
+        uint32_t agg = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) agg += red[w][tid];
+        a.run_cnt[static_cast<uint64_t>(j) * M + tid] = agg;
+    }
+}
+
+// The class counts of every run of the large segments, one CTA per run.
+template <class V, class D, int M, int THREADS>
+__global__ void __launch_bounds__(THREADS, 4) seg_run_count(SegArgs a, D d) {
+    __shared__ uint32_t red[2][THREADS / 32][M];
+    __shared__ uint32_t ticket_sh[2];
+    const uint32_t num_runs = a.hdr->num_runs;
+    for (uint32_t it = 0;; it++) {
+        if (threadIdx.x == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket3, 1u);
+        __syncthreads();
+        const uint32_t j = ticket_sh[it & 1u];
+        if (j >= num_runs) break;
+        count_run<V, D, M, THREADS>(a, d, j, red[it & 1u]);
+    }
+}
+
+// Persistent; CTAs take tickets for batches of small-segment groups.
 template <class V, class D, int M, int THREADS, int STAGES>
 __global__ void __launch_bounds__(THREADS, 3)
     seg_main(SegArgs a, D d) {
     using L = SegSmem<V, M, THREADS, STAGES>;
     constexpr uint32_t AU = L::kAU;
+    constexpr uint32_t P = L::kTile;
     static_assert(M <= 16 && M >= 2, "class bound");
+    static_assert(static_cast<int>(kGroupSegs) <= THREADS, "one thread per segment");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     unsigned char* base = smem_raw + (((raw + 127u) & ~127u) - raw);
-    V* g_in0 = reinterpret_cast<V*>(base);
-    V* g_out = g_in0 + L::kGroupElems;
+    V* g_in = reinterpret_cast<V*>(base);
+    V* g_out = g_in + L::kGroupElems;
+    GroupScratch<M, THREADS>& gs = *reinterpret_cast<GroupScratch<M, THREADS>*>(g_out + L::kGroupElems);
 
-    __shared__ __align__(8) uint64_t gbars[2];
+    __shared__ __align__(8) uint64_t gbar;
     __shared__ uint32_t ticket_sh[2];
-    __shared__ uint32_t gi_h[2], gi_he[2];  // group pipeline slots
-    __shared__ uint64_t gi_r0[2], gi_r1[2], gi_as[2], gi_tail[2];
-    __shared__ GroupScratch<M, THREADS> gs;
     __shared__ uint32_t gb_h[kMaxGroupBatch], gb_he[kMaxGroupBatch];  // the batch's groups
-    __shared__ uint64_t gb_r0[kMaxGroupBatch], gb_r1[kMaxGroupBatch];
+    __shared__ uint32_t gb_r0[kMaxGroupBatch], gb_r1[kMaxGroupBatch];
     __shared__ uint32_t cmod[17];  // DiscrMod constants for m = 1 .. 16
 
     const int tid = threadIdx.x;
     const V* in = static_cast<const V*>(a.in);
     V* out = static_cast<V*>(a.out);
-    const uint32_t out_phase =
-        static_cast<uint32_t>(reinterpret_cast<uintptr_t>(out) / sizeof(V)) & (AU - 1u);
     const bool in_vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     const bool out_vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
     const uint64_t S = seg_count(a);
@@ -730,12 +792,10 @@ __global__ void __launch_bounds__(THREADS, 3)
     const uint32_t batch =
         max(1u, min(a.group_batch, (num_groups + gridDim.x - 1) / gridDim.x));
     const uint32_t num_batches = (num_groups + batch - 1) / batch;
-    const uint32_t total = num_batches;
-    uint32_t group_uses = 0;
+    uint32_t uses = 0;  // of the input buffer
 
     if (tid == 0) {
-        mbar_init(&gbars[0], 1);
-        mbar_init(&gbars[1], 1);
+        mbar_init(&gbar, 1);
         mbar_fence_init();
     }
     if (tid >= 1 && tid <= 16) cmod[tid] = DiscrMod::make(static_cast<uint32_t>(tid)).c;
@@ -746,185 +806,117 @@ __global__ void __launch_bounds__(THREADS, 3)
         if (tid == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket, 1u);
         __syncthreads();
         const uint32_t t = ticket_sh[it & 1u];
-        if (t >= total) break;
-
-        if (t < num_batches) {
-            // ---------------- a batch of small-segment groups ----------------
-            // group i of the batch: segments [h, he), elements [r0, r1); its
-            // range is fetched by one bulk copy while the previous group is
-            // partitioned
-            const uint32_t g0 = t * batch;
-            const uint32_t gcnt = min(batch, num_groups - g0);
-            // the batch's group heads, ends and element ranges, loaded once
-            if (tid < static_cast<int>(gcnt)) {
-                const uint32_t h = a.groups[g0 + tid];
-                const uint32_t he =
-                    static_cast<uint32_t>(min(static_cast<uint64_t>(a.groups_end[g0 + tid]), S));
-                gb_h[tid] = h;
-                gb_he[tid] = he;
-                gb_r0[tid] = a.offsets[h];
-                gb_r1[tid] = a.offsets[he];
+        if (t >= num_batches) break;
+        // group i of the batch: segments [h, he), elements [r0, r1); its range is
+        // fetched by one bulk copy while the previous group is written
+        const uint32_t g0 = t * batch;
+        const uint32_t gcnt = min(batch, num_groups - g0);
+        if (tid < static_cast<int>(gcnt)) {
+            const uint32_t h = a.groups[g0 + tid];
+            uint32_t he = static_cast<uint32_t>(min(static_cast<uint64_t>(a.groups_end[g0 + tid]), S));
+            he = min(max(he, h), h + kGroupSegs);
+            uint64_t r0 = a.offsets[h], r1 = a.offsets[he];
+            if (r1 < r0 || r1 - r0 >= 2u * P || r1 > a.n) {  // malformed: nothing to do
+                he = h;
+                r0 = r1 = 0u;
             }
+            gb_h[tid] = h;
+            gb_he[tid] = he;
+            gb_r0[tid] = static_cast<uint32_t>(r0);  // n < 2^32
+            gb_r1[tid] = static_cast<uint32_t>(r1);
+        }
+        __syncthreads();
+        // the 16-byte words of group i that one bulk copy brings
+        auto vec_end = [&](uint32_t i, uint64_t as) {
+            const uint64_t ve =
+                min((static_cast<uint64_t>(gb_r1[i]) + AU - 1u) & ~static_cast<uint64_t>(AU - 1u),
+                    a.n & ~static_cast<uint64_t>(AU - 1u));
+            return in_vec && ve > as ? ve : as;
+        };
+        auto issue_group = [&](uint32_t i) {  // thread 0 only
+            const uint64_t as = gb_r0[i] & ~(AU - 1u);
+            const uint32_t bytes = static_cast<uint32_t>((vec_end(i, as) - as) * sizeof(V));
+            if (bytes > 0) {
+                mbar_arrive_expect_tx(&gbar, bytes);
+                bulk_load_g2s(g_in, in + as, bytes, &gbar);
+            } else {
+                mbar_arrive(&gbar);
+            }
+        };
+        if (tid == 0) issue_group(0);
+        bool failed = false;
+        GroupPrefetch pf;
+        pf.valid = false;
+        for (uint32_t i = 0; i < gcnt; i++) {
+            const uint32_t h = gb_h[i], nseg = gb_he[i] - h;
+            const uint32_t r0 = gb_r0[i], r1 = gb_r1[i];
+            const uint64_t as = r0 & ~static_cast<uint64_t>(AU - 1u);
+            const uint32_t phase = static_cast<uint32_t>(r0 - as);
+            const uint32_t end = static_cast<uint32_t>(r1 - as);
+            // ---- heads, while the group's elements are on their way
+            bool bad = false;
+            if (static_cast<uint32_t>(tid) < nseg) {
+                if (!pf.valid) {
+                    pf.o0 = a.offsets[h + tid];
+                    pf.o1 = a.offsets[h + tid + 1];
+                    pf.m = a.seg_m != nullptr ? min(max(a.seg_m[h + tid], 1u), a.m_bound) : a.m;
+                }
+                bad = pf.o0 < r0 || pf.o1 < pf.o0 || pf.o1 > r1;
+                gs.hpos[tid] = static_cast<uint16_t>(pf.o0 - as);
+                gs.msz[tid] = static_cast<uint8_t>(pf.m);
+            }
+            if (tid == 0) gs.hpos[nseg] = static_cast<uint16_t>(end);
+            const bool ok = mbar_wait_bounded(&gbar, uses & 1u);
+            const uint64_t ve = vec_end(i, as);
+            if (ve < r1) {  // what the bulk copy did not bring (CTA-uniform)
+                for (uint64_t e = max(ve, static_cast<uint64_t>(r0)) + tid; e < r1; e += THREADS)
+                    g_in[e - as] = in[e];
+            }
+            if (__syncthreads_or(bad || !ok)) {  // a malformed group is left alone
+                if (tid == 0) {  // only this group's copy can be in flight
+                    const bool late = mbar_wait_bounded(&gbar, uses & 1u);
+                    if (!late) atomicOr(&a.hdr->error, kErrTimeout);
+                }
+                failed = true;
+                break;
+            }
+            uses++;
+            pf.valid = i + 1 < gcnt;
+            if (pf.valid && static_cast<uint32_t>(tid) < gb_he[i + 1] - gb_h[i + 1]) {
+                const uint64_t ns = static_cast<uint64_t>(gb_h[i + 1]) + tid;
+                pf.o0 = a.offsets[ns];
+                pf.o1 = a.offsets[ns + 1];
+                pf.m = a.seg_m != nullptr ? min(max(a.seg_m[ns], 1u), a.m_bound) : a.m;
+            }
+            const uint32_t nq = ((end + THREADS * AU - 1u) / (THREADS * AU)) | 1u;
+            uint32_t qn = 0;  // heads before the thread's first position
+            if (nseg > 0u) {
+                const uint32_t lo = static_cast<uint32_t>(tid) * nq * AU;
+                for (uint32_t step = 1u << (31 - __clz(nseg)); step > 0u; step >>= 1)
+                    if (qn + step <= nseg && gs.hpos[qn + step - 1u] < lo) qn += step;
+            }
+            seg_group_cta<V, D, M, THREADS>(a, d, cmod, h, nseg, as, phase, end, g_in, g_out, gs, qn, nq);
+            // every access of the buffers precedes the copies of them
+            fence_proxy_async_smem();
             __syncthreads();
-            auto issue_group = [&](uint32_t i) {  // thread 0 only
-                const uint32_t slot = (group_uses + i) & 1u;
-                const uint32_t h = gb_h[i], he = gb_he[i];
-                const uint64_t r0 = gb_r0[i], r1 = gb_r1[i];
-                const uint64_t as = r0 & ~static_cast<uint64_t>(AU - 1u);
-                uint64_t ve = min((r1 + AU - 1u) & ~static_cast<uint64_t>(AU - 1u),
-                                  a.n & ~static_cast<uint64_t>(AU - 1u));
-                if (!in_vec || ve < as) ve = as;
-                gi_h[slot] = h;
-                gi_he[slot] = he;
-                gi_r0[slot] = r0;
-                gi_r1[slot] = r1;
-                gi_as[slot] = as;
-                gi_tail[slot] = max(ve, r0);
-                V* dst = g_in0;
-                const uint32_t bytes = static_cast<uint32_t>((ve - as) * sizeof(V));
-                if (bytes > 0) {
-                    mbar_arrive_expect_tx(&gbars[slot], bytes);
-                    bulk_load_g2s(dst, in + as, bytes, &gbars[slot]);
-                } else {
-                    mbar_arrive(&gbars[slot]);
+            if (tid == 0 && i + 1 < gcnt) issue_group(i + 1);
+            // write the range back from the output image
+            const uint32_t vs = min((phase + AU - 1u) & ~(AU - 1u), end), vt = max(vs, end & ~(AU - 1u));
+            if (out_vec) {
+                if (tid == 0 && vt > vs) {
+                    bulk_store_s2g(out + as + vs, g_out + vs, (vt - vs) * sizeof(V));
+                    bulk_commit();
                 }
-            };
-            if (tid == 0) issue_group(0);
-            bool failed = false;
-            GroupPrefetch pf;
-            pf.valid = false;
-            for (uint32_t i = 0; i < gcnt; i++) {
-                const uint32_t use = group_uses + i;
-                const uint32_t slot = use & 1u;
-                const bool ok = mbar_wait_bounded(&gbars[slot], (use >> 1) & 1u);
-                __syncthreads();  // slot info visible
-                V* gin = g_in0;
-                const uint64_t as = gi_as[slot], r0 = gi_r0[slot], r1 = gi_r1[slot];
-                for (uint64_t e = gi_tail[slot] + tid; e < r1; e += THREADS) gin[e - as] = in[e];
-                if (__syncthreads_or(!ok)) {
-                    failed = true;
-                    if (tid == 0) {  // only this group's copy can be in flight
-                        atomicOr(&a.hdr->error, kErrTimeout);
-                        (void)mbar_wait_bounded(&gbars[slot], (use >> 1) & 1u);
-                    }
-                    break;
-                }
-                const bool more = i + 1 < gcnt;
-                seg_group_cta<V, D, M, THREADS>(
-                    a, d, cmod, gi_h[slot], gi_he[slot], r0, static_cast<uint32_t>(r1 - r0),
-                    gin + (r0 - as), g_out + (r0 - as), gs, pf, more ? &gb_h[i + 1] : nullptr,
-                    more ? &gb_he[i + 1] : nullptr);
-                // every read of the input buffer precedes the next group's copy
-                fence_proxy_async_smem();
+                if (static_cast<uint32_t>(tid) < vs - phase) out[r0 + tid] = g_out[phase + tid];
+                if (static_cast<uint32_t>(tid) < end - vt) out[as + vt + tid] = g_out[vt + tid];
+            } else {
+                for (uint32_t y = phase + tid; y < end; y += THREADS) out[as + y] = g_out[y];
                 __syncthreads();
-                if (tid == 0 && more) issue_group(i + 1);
-                // write the range back from the output image
-                if (out_vec && out_phase == 0u) {
-                    const uint64_t vs = (r0 + AU - 1u) & ~static_cast<uint64_t>(AU - 1u);
-                    const uint64_t ve = r1 & ~static_cast<uint64_t>(AU - 1u);
-                    if (vs < ve) {
-                        const uint4* srcv = reinterpret_cast<const uint4*>(g_out + (vs - as));
-                        uint4* dstv = reinterpret_cast<uint4*>(out + vs);
-                        const uint32_t nv = static_cast<uint32_t>((ve - vs) / AU);
-                        for (uint32_t q = tid; q < nv; q += THREADS) dstv[q] = srcv[q];
-                        for (uint64_t e = r0 + tid; e < vs; e += THREADS) out[e] = g_out[e - as];
-                        for (uint64_t e = ve + tid; e < r1; e += THREADS) out[e] = g_out[e - as];
-                    } else {
-                        for (uint64_t e = r0 + tid; e < r1; e += THREADS) out[e] = g_out[e - as];
-                    }
-                } else {
-                    for (uint64_t e = r0 + tid; e < r1; e += THREADS) out[e] = g_out[e - as];
-                }
-                // generic-proxy accesses of these buffers precede the next TMA writes
-                fence_proxy_async_smem();
             }
-            group_uses += gcnt;
-            __syncthreads();
-            if (failed) break;
-            continue;
         }
+        if (failed) break;
     }
-}
-
-// Class counts of every run of the large segments: one CTA per run (run
-// tickets), 16-byte loads four deep per thread, per-thread packed counters,
-// warp reductions and one barrier per run.  A few hundred bytes of shared
-// memory, so more CTAs per SM than the group kernel keep loads in flight.
-template <class V, class D, int M, int THREADS>
-__global__ void __launch_bounds__(THREADS, 4) seg_run_count(SegArgs a, D d) {
-    constexpr uint32_t AU = 16 / sizeof(V);
-    constexpr int W = THREADS / 32;
-    __shared__ uint32_t red[W][M];
-    __shared__ uint32_t ticket_sh[2];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const V* in = static_cast<const V*>(a.in);
-    const bool in_vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
-    const uint32_t num_runs = a.hdr->num_runs;
-    for (uint32_t it = 0;; it++) {
-        if (tid == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket3, 1u);
-        __syncthreads();
-        const uint32_t j = ticket_sh[it & 1u];
-        if (j >= num_runs) break;
-        const RunEntry ent = a.runs[j];
-        const D dj = seg_discr(a, d, ent.seg);
-        PackedCounts<M> pc;
-        pc.init();
-        const uint64_t p0 = ent.p0, p1 = ent.p1;
-        const uint64_t vs = in_vec ? ((p0 + AU - 1u) & ~static_cast<uint64_t>(AU - 1u)) : p1;
-        const uint64_t ve = in_vec ? max(vs, p1 & ~static_cast<uint64_t>(AU - 1u)) : p1;
-        {
-            uint32_t k = 0;
-            for (uint64_t e = p0 + tid; e < min(vs, p1); e += THREADS) {
-                pc.add(dj(in[e]));
-                if (++k == 8u) {
-                    pc.fold();
-                    k = 0;
-                }
-            }
-            for (uint64_t e = ve + tid; e < p1 && vs < p1; e += THREADS) {
-                pc.add(dj(in[e]));
-                if (++k == 8u) {
-                    pc.fold();
-                    k = 0;
-                }
-            }
-            pc.fold();
-        }
-        {
-            const uint4* vp = reinterpret_cast<const uint4*>(in + vs);
-            const uint32_t nv = static_cast<uint32_t>((ve - vs) / AU);
-            constexpr int UNROLL = 4;
-            for (uint32_t q = tid; q < nv; q += THREADS * UNROLL) {
-                uint4 r[UNROLL];
-#pragma unroll
-                for (int uu = 0; uu < UNROLL; uu++)
-                    if (q + uu * THREADS < nv) r[uu] = __ldg(vp + q + uu * THREADS);
-#pragma unroll
-                for (int uu = 0; uu < UNROLL; uu++) {
-                    if (q + uu * THREADS < nv) {
-                        V e[AU];
-                        unpack16_to<V>(r[uu], e);
-#pragma unroll
-                        for (uint32_t z = 0; z < AU; z++) pc.add(dj(e[z]));
-                    }
-                    if (uu & 1) pc.fold();  // every two vectors: <= 8 increments
-                }
-            }
-        }
-        pc.finish();
-#pragma unroll
-        for (int c = 0; c < M; c++) {
-            const uint32_t x = warp_sum(pc.acc[c]);
-            if (lane == 0) red[warp][c] = x;
-        }
-        __syncthreads();
-        if (tid < static_cast<uint32_t>(M)) {
-            uint32_t agg = 0;
-#pragma unroll
-            for (int w = 0; w < W; w++) agg += red[w][tid];
-            a.run_cnt[static_cast<uint64_t>(j) * M + tid] = agg;
-        }
-    }
+    if (tid == 0) bulk_wait_all();
 }
 
 // One large segment's runs [j, jl]: lane l takes a contiguous share of the

@@ -227,6 +227,10 @@ struct CountColumns {
     }
 };
 
+// Discriminators that are as cheap to evaluate twice as to remember.
+template <class D>
+struct CheapClass : std::is_same<D, DiscrMask> {};
+
 // Per-thread class counts of the nibble step and where class c's 16-bit count
 // lies: classes k and k + M / 2 share word k.
 template <int M>
@@ -363,8 +367,21 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
 #pragma unroll
         for (int q = 0; q < (ITEMS + 7) / 8; q++) lr[q] = 0;
     }
+    // classes kept for pass 2 where working them out again costs more (a byte each;
+    // m <= 8 has no registers to spare for them)
+    constexpr bool kKeep = M == 16 && !CheapClass<D>::value;
+    uint32_t kept[kKeep ? (ITEMS + 3) / 4 : 1];
+    if constexpr (kKeep) {
+#pragma unroll
+        for (int q = 0; q < (ITEMS + 3) / 4; q++) kept[q] = 0;
+    }
+    auto class_of = [&](int j) -> uint32_t {
+        if constexpr (kKeep) return __byte_perm(kept[j >> 2], 0u, 0x4440 + (j & 3));
+        else return d(v[j]);
+    };
     auto count = [&](int j) {
         const uint32_t c = d(v[j]);
+        if constexpr (kKeep) kept[j >> 2] += c << (8 * (j & 3));
         if constexpr (kRanks) lr[j >> 3] += tc.get(c) << (4 * (j & 7));
         if (j < kIn) tc.inc(c); else last_c = c;
     };
@@ -376,7 +393,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
         for (int j = 0; j < ITEMS; j++)
             if (e0 + j >= lo && e0 + j < hi) count(j);
     }
-    const uint32_t c_last = d(v[ITEMS - 1]);
+    const uint32_t c_last = class_of(ITEMS - 1);
     bool one_class = false;  // the warp's elements
     if constexpr (CLUSTERED) one_class = full && warp_of_one_class(tc.get(c_last) == kIn, c_last);
 #pragma unroll
@@ -453,7 +470,7 @@ __device__ __forceinline__ bool tile_scatter(const D& d, const V (&v)[ITEMS], ui
 
     // ---- pass 2: scatter into the class-sorted stage
     auto place = [&](int j) {
-        uint16_t& next = count_at(d(v[j]));
+        uint16_t& next = count_at(class_of(j));
         if constexpr (kRanks) {
             stage[next + ((lr[j >> 3] >> (4 * (j & 7))) & 15u)] = v[j];
         } else {  // the thread's slot of a class moves on with every element of it
@@ -655,8 +672,20 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
     uint32_t lr[(ITEMS + 3) / 4];
 #pragma unroll
     for (int q = 0; q < (ITEMS + 3) / 4; q++) lr[q] = 0;
+    constexpr bool kKeep = !CheapClass<D>::value;  // as in tile_scatter
+    uint32_t kept[kKeep ? (ITEMS + 3) / 4 : 1];
+    if constexpr (kKeep) {
+#pragma unroll
+        for (int q = 0; q < (ITEMS + 3) / 4; q++) kept[q] = 0;
+    }
+    auto class_of = [&](int j) -> uint32_t {
+        if constexpr (kKeep) return __byte_perm(kept[j >> 2], 0u, 0x4440 + (j & 3));
+        else return d(v[j]);
+    };
     auto count = [&](int j) {
-        unsigned char& x = at(d(v[j]));
+        const uint32_t c = d(v[j]);
+        if constexpr (kKeep) kept[j >> 2] += c << (8 * (j & 3));
+        unsigned char& x = at(c);
         const uint32_t r = x;
         x = static_cast<unsigned char>(r + 1u);
         lr[j >> 2] += r << (8 * (j & 3));
@@ -669,7 +698,7 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
         for (int j = 0; j < ITEMS; j++)
             if (e0 + j >= lo && e0 + j < hi) count(j);
     }
-    const uint32_t c_last = d(v[ITEMS - 1]);
+    const uint32_t c_last = class_of(ITEMS - 1);
     bool one_class = false;  // the warp's elements
     if constexpr (CLUSTERED)
         one_class = full && warp_of_one_class(
@@ -790,7 +819,7 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
     // ---- pass 2: scatter into the class-sorted stage
     const uint16_t* gb = grp + tid / (PER * LPG) * kGroupRow<M>;
     auto place = [&](int j) {
-        const uint32_t c = d(v[j]);
+        const uint32_t c = class_of(j);
         stage[gb[c] + at(c) + __byte_perm(lr[j >> 2], 0u, 0x4440 + (j & 3))] = v[j];
     };
     if (CLUSTERED && one_class) {

@@ -1,0 +1,74 @@
+"""The small-segment groups of the segmented path at their edges, bit-exact against
+the oracle: segments that begin and end inside a thread's 16-byte words, several in
+one word, empty ones at a group's ends, groups of one segment and of 128, lengths at
+the window, buffers off their alignment, every class bound, and a class count per
+segment."""
+import numpy as np
+import pytest
+
+import mdiscriminator_b200 as mdx
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def lengths_of(form, P, rng):
+    if form == "tiny":  # many heads in every word
+        return rng.integers(0, 5, 9000)
+    if form == "empty":  # runs of empty segments before, between and after full ones
+        x = np.zeros(3000, dtype=np.int64)
+        x[rng.choice(3000, 120, replace=False)] = rng.integers(1, P + 1, 120)
+        return x
+    if form == "window":  # at the small-segment bound and the window
+        return rng.choice([1, 2, 3, P - 5, P - 4, P - 3, P - 1, P], 60)
+    if form == "words":  # around a thread's words at every number of them
+        return rng.choice([3, 4, 5, 12, 19, 20, 21, 28, 36, 37, 1019, 1020, 1025], 900)
+    return np.concatenate([[P, 0, 1], rng.integers(1, 400, 200), [P - 1], np.zeros(130, np.int64), [7]])
+
+
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("form", ["tiny", "empty", "window", "words", "mixed"])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 7, 8, 13, 16])
+def test_groups(cuda_ready, m, form, rec):
+    torch = cuda_ready
+    rng = np.random.default_rng(m * 7 + len(form))
+    P = 2048 if rec else 4096
+    offs = np.concatenate([[0], np.cumsum(lengths_of(form, P, rng))]).astype(np.uint64)
+    n = int(offs[-1])
+    x = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    if rec:
+        x = x.astype(np.uint64) | (np.arange(n, dtype=np.uint64) << np.uint64(32))
+    eo, es, ef = oracle.partition_segmented(x, offs, m, headflags=True)
+    kind = np.int64 if rec else np.int32
+    do = torch.from_numpy(offs.view(np.int64)).cuda()
+    for off_in, off_out in ((0, 0), (1, 0), (0, 1)):
+        base = torch.zeros(n + 4, dtype=torch.int64 if rec else torch.int32, device="cuda")
+        base[off_in:off_in + n] = torch.from_numpy(x.view(kind)).cuda()
+        out = torch.zeros_like(base)
+        o, sizes, hf = mdx.partition_segmented(base[off_in:off_in + n], do, ("mod", m),
+                                               out=out[off_out:off_out + n], headflags=True)
+        torch.cuda.synchronize()
+        assert mdx.workspace(0).error() == mdx.MDX_OK
+        assert np.array_equal(sizes.cpu().numpy(), es)
+        assert np.array_equal(o.cpu().numpy().view(x.dtype), eo), (off_in, off_out)
+        assert np.array_equal(hf.cpu().numpy(), ef)
+
+
+def test_class_count_per_segment(cuda_ready):
+    torch = cuda_ready
+    rng = np.random.default_rng(2)
+    lengths = np.concatenate([rng.integers(0, 40, 2000), rng.integers(1, 4097, 60), [9000, 5, 70_000]])
+    seg_m = rng.integers(1, 17, lengths.size).astype(np.int32)
+    offs = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint64)
+    x = rng.integers(0, 1 << 32, int(offs[-1]), dtype=np.uint64).astype(np.uint32)
+    out, sizes = mdx.partition_segmented_multi(
+        torch.from_numpy(x.view(np.int32)).cuda(), torch.from_numpy(offs.view(np.int64)).cuda(),
+        torch.from_numpy(seg_m).cuda(), 16)
+    torch.cuda.synchronize()
+    assert mdx.workspace(0).error() == mdx.MDX_OK
+    got, gs = out.cpu().numpy().view(np.uint32), sizes.cpu().numpy()
+    for s in range(lengths.size):
+        a, b = int(offs[s]), int(offs[s + 1])
+        cls = x[a:b] % seg_m[s]
+        assert np.array_equal(got[a:b], x[a:b][np.argsort(cls, kind="stable")]), s
+        assert np.array_equal(gs[s], np.bincount(cls, minlength=16)), s

@@ -524,9 +524,6 @@ mdx_status dispatch_plain(const void* in, void* out, uint64_t n, mdx_discr dc, u
 
 // ------------------------------------------------------------- segmented --
 constexpr int kPlanThreads = 256;
-constexpr uint32_t kMaxPlanBlocks = 1024;
-constexpr int kFlagsTile = 4096;
-constexpr uint32_t kMaxFlagChunks = 4096;
 
 inline uint32_t window_elems(mdx_elem e) { return tile_elems(e); }
 
@@ -571,8 +568,26 @@ inline SegLayout seg_layout(uint64_t n, uint64_t S, mdx_elem e, uint32_t m, bool
     return L;
 }
 
+// Launch with programmatic stream serialization: the kernel may be scheduled before
+// the one before it has finished and waits for that where it says so (pdl_wait).
+template <class... KArgs, class... Args>
+bool launch_dependent(void (*fn)(KArgs...), uint32_t grid, int threads, size_t smem, cudaStream_t st,
+                      const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, args...) == cudaSuccess;
+}
+
 inline uint32_t plan_blocks_for(uint64_t S_bound) {
-    uint64_t g = (S_bound + 511) / 512;
+    uint64_t g = (S_bound + 255) / 256;
     if (g < 1) g = 1;
     if (g > kMaxPlanBlocks) g = kMaxPlanBlocks;
     return static_cast<uint32_t>(g);
@@ -583,16 +598,18 @@ mdx_status run_segm(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
                     const uint64_t* d_offsets, uint64_t S, uint64_t S_bound, const int32_t* in_flags,
                     uint32_t* d_seg_sizes, uint32_t* d_headflags, unsigned char* ws,
                     const SegLayout& L, cudaStream_t st, const uint32_t* d_seg_m = nullptr) {
-    using SL = SegSmem<V, M, kThreads, kStages>;
+    using SL = SegSmem<V, M, kThreads>;
+    using RL = RunSmem<V, M, kThreads>;
     constexpr int P = SL::kTile;
     using ML = MidSmem<V, M, kThreads, kMidTiles>;
-    auto main_fn = seg_main<V, D, M, kThreads, kStages>;
-    auto scatter_fn = seg_run_scatter<V, D, M, kThreads, kStages>;
+    auto main_fn = seg_main<V, D, M, kThreads>;
+    auto scatter_fn = seg_run_scatter<V, D, M, kThreads>;
+    auto count_fn = seg_run_count<V, D, M, kThreads>;
     auto mid_fn = seg_mid<V, D, M, kThreads, kMidTiles>;
-    int blocks = 0, sms = 0, sblocks = 0, mblocks = 0;
+    int blocks = 0, sms = 0, sblocks = 0, mblocks = 0, cblocks = 0;
     if (occupancy(reinterpret_cast<const void*>(main_fn), SL::kBytes, &blocks, &sms) != cudaSuccess ||
-        occupancy(reinterpret_cast<const void*>(scatter_fn), SL::kRunBytes, &sblocks, &sms) !=
-            cudaSuccess ||
+        occupancy(reinterpret_cast<const void*>(scatter_fn), RL::kBytes, &sblocks, &sms) != cudaSuccess ||
+        occupancy(reinterpret_cast<const void*>(count_fn), 0, &cblocks, &sms) != cudaSuccess ||
         occupancy(reinterpret_cast<const void*>(mid_fn), ML::kBytes, &mblocks, &sms) != cudaSuccess)
         return MDX_ERR_CUDA;
     SegArgs a;
@@ -638,24 +655,23 @@ mdx_status run_segm(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
     if (d_headflags != nullptr &&
         cudaMemsetAsync(d_headflags, 0, n * sizeof(uint32_t), st) != cudaSuccess)
         return MDX_ERR_CUDA;
-    if (cudaMemsetAsync(a.groups_end, 0xff, L.max_groups * sizeof(uint32_t), st) != cudaSuccess)
-        return MDX_ERR_CUDA;
+    // Small kernels, and those after them, are scheduled while the one before drains
+    // and wait for its results (programmatic dependent launch: 2^24 elements in 84
+    // segments, per-segment m, 118 -> 87 us a call).  Not seg_mid and seg_run_count:
+    // scheduled early they share the SMs with seg_main's last CTAs and wait there
+    // (10^5 segments, m = 4: 896 us a call with seg_run_count early, 851 without).
+    const uint32_t scan_blocks = static_cast<uint32_t>(std::min<uint64_t>((L.max_runs + 255) / 256, 4096));
     seg_plan_spans<P, kPlanThreads><<<a.plan_blocks, kPlanThreads, 0, st>>>(a);
-    seg_plan_emit<P, kPlanThreads><<<a.plan_blocks, kPlanThreads, 0, st>>>(a);
-    main_fn<<<static_cast<uint32_t>(blocks) * sms, kThreads, SL::kBytes, st>>>(a, d);
+    bool launched =
+        launch_dependent(seg_plan_emit<P, kPlanThreads>, a.plan_blocks, kPlanThreads, 0, st, a) &&
+        launch_dependent(main_fn, blocks * sms, kThreads, SL::kBytes, st, a, d);
     if (a.mid_tiles > 0)
         mid_fn<<<static_cast<uint32_t>(mblocks) * sms, kThreads, ML::kBytes, st>>>(a, d, map);
-    {
-        auto count_fn = seg_run_count<V, D, M, kThreads>;
-        int cblocks = 0;
-        if (occupancy(reinterpret_cast<const void*>(count_fn), 0, &cblocks, &sms) != cudaSuccess)
-            return MDX_ERR_CUDA;
-        count_fn<<<static_cast<uint32_t>(cblocks) * sms, kThreads, 0, st>>>(a, d);
-    }
+    count_fn<<<static_cast<uint32_t>(cblocks) * sms, kThreads, 0, st>>>(a, d);
     // a warp per 32 runs (the run count is on the device: enough for the capacity)
-    const uint64_t scan_blocks = std::min<uint64_t>((L.max_runs + 255) / 256, 4096);
-    seg_run_scan<M><<<static_cast<uint32_t>(scan_blocks), 256, 0, st>>>(a);
-    scatter_fn<<<static_cast<uint32_t>(sblocks) * sms, kThreads, SL::kRunBytes, st>>>(a, d, map);
+    launched = launched && launch_dependent(seg_run_scan<M>, scan_blocks, 256, 0, st, a) &&
+               launch_dependent(scatter_fn, sblocks * sms, kThreads, RL::kBytes, st, a, d, map);
+    if (!launched) return MDX_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
 }
 
@@ -688,26 +704,27 @@ mdx_status dispatch_segm(const void* in, void* out, uint64_t n, mdx_discr dc, co
 // area) and S into the header, ahead of run_segm with kSegsOnDevice.
 inline mdx_status launch_flags_to_offsets(const int32_t* d_flags, uint64_t n, unsigned char* ws,
                                           const SegLayout& L, cudaStream_t st) {
-    auto stage_fn = seg_flags_stage<kThreads, kFlagsTile>;
+    // a warp per chunk, chunks of whole 512-byte rows
+    constexpr uint32_t W = kThreads / 32;
+    const uint64_t rows = (n + 127) / 128;
     int blocks = 0, sms = 0;
-    if (occupancy(reinterpret_cast<const void*>(stage_fn), 0, &blocks, &sms) != cudaSuccess)
+    if (occupancy(reinterpret_cast<const void*>(seg_flags_stage<kThreads>), 0, &blocks, &sms) != cudaSuccess)
         return MDX_ERR_CUDA;
-    const uint64_t tiles = (n + kFlagsTile - 1) / kFlagsTile;
-    uint64_t G = static_cast<uint64_t>(blocks) * sms;
-    if (G > tiles) G = tiles;
-    if (G > kMaxFlagChunks) G = kMaxFlagChunks;
-    if (G < 1) G = 1;
+    // as many CTAs on every SM, within the chunk tables
+    const uint64_t most = kMaxFlagChunks / W, even = most / sms * sms;
+    const uint64_t G = std::min<uint64_t>((rows + W - 1) / W, even > 0 ? even : most);
     FlagsArgs fa;
     fa.flags = d_flags;
     fa.n = n;
-    fa.chunk = ((n + G - 1) / G + 3u) & ~uint64_t{3};
+    fa.chunk = (rows + G * W - 1) / (G * W) * 128;
     fa.stage = reinterpret_cast<uint32_t*>(ws + L.flag_stage);
     fa.cnt = reinterpret_cast<uint32_t*>(ws + L.flag_cnt);
     fa.pre = reinterpret_cast<uint32_t*>(ws + L.flag_pre);
     fa.offsets = reinterpret_cast<uint64_t*>(ws + L.offsets);
     fa.hdr = reinterpret_cast<SegHeader*>(ws);
-    stage_fn<<<static_cast<uint32_t>(G), kThreads, 0, st>>>(fa);
-    seg_flags_compact<kThreads><<<static_cast<uint32_t>(G), kThreads, 0, st>>>(fa);
+    seg_flags_stage<kThreads><<<static_cast<uint32_t>(G), kThreads, 0, st>>>(fa);
+    if (!launch_dependent(seg_flags_compact<kThreads>, static_cast<uint32_t>(G), kThreads, 0, st, fa))
+        return MDX_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
 }
 

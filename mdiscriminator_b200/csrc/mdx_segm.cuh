@@ -56,6 +56,7 @@ constexpr int kRunTiles = 8;     // tiles per run of a large segment
 constexpr int kMidTiles = 2;     // most tiles a medium segment may span (seg_mid's slab)
 constexpr int kGroupBatch = 8;   // small-segment groups per ticket of seg_main
 constexpr int kMaxGroupBatch = 32;
+constexpr uint32_t kMaxPlanBlocks = 1024;
 
 struct SegHeader {      // lives at the start of the segmented workspace
     uint32_t ticket;    // seg_main's tickets (reset by the planner)
@@ -75,10 +76,13 @@ struct SegHeader {      // lives at the start of the segmented workspace
     uint32_t pad[1];
 };
 
-struct RunEntry {       // a run of up to run_tiles tiles of one large segment
-    uint32_t seg;       // segment index
-    uint32_t p0, p1;    // element range of the run
-    uint32_t jlast;     // entry index of the segment's last run
+struct alignas(16) RunEntry {  // a run of up to run_tiles tiles of one large segment
+    uint32_t seg;              // segment index
+    uint32_t p0;               // its first element
+    uint32_t len_m;            // its length (low 24 bits: at most 64 tiles) and, when the call
+                               // carries class counts per segment, the segment's (high 8)
+    uint32_t jlast;            // entry index of the segment's last run
+    __device__ __forceinline__ uint32_t p1() const { return p0 + (len_m & 0xffffffu); }
 };
 
 struct SegArgs {
@@ -119,15 +123,16 @@ struct SegArgs {
     uint32_t max_mids;
 };
 
-// The discriminator of segment s: the launch's, or -- when the call carries
-// per-segment class counts -- key % m_s (m_s clamped to [1, m_bound]).
+// Class count of segment s, clamped to [1, m_bound], when the call carries them.
+__device__ __forceinline__ uint32_t seg_classes(const SegArgs& a, uint64_t s) {
+    return a.seg_m != nullptr ? min(max(a.seg_m[s], 1u), a.m_bound) : 0u;
+}
+// The discriminator of a segment with class count m: the launch's, or -- when the
+// call carries class counts per segment -- key % m.
 template <class D>
-__device__ __forceinline__ D seg_discr(const SegArgs& a, const D& d, uint64_t s) {
+__device__ __forceinline__ D seg_discr(const SegArgs& a, const D& d, uint32_t m) {
     if constexpr (std::is_same<D, DiscrMod>::value) {
-        if (a.seg_m != nullptr) {
-            const uint32_t m = min(max(a.seg_m[s], 1u), a.m_bound);
-            return DiscrMod::make(m);
-        }
+        if (a.seg_m != nullptr) return DiscrMod::make(m);
     }
     return d;
 }
@@ -181,7 +186,11 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
     __shared__ uint32_t warp_runs[W], warp_grps[W], warp_mids[W];
     __shared__ int am_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
     const uint64_t S = seg_count(a);
+    // no group has an end yet
+    for (uint32_t g = blockIdx.x * THREADS + tid; g < a.max_groups; g += gridDim.x * THREADS)
+        a.groups_end[g] = 0xffffffffu;
     const uint64_t G = gridDim.x;
     const uint64_t R = (S + G - 1) / G;
     const uint64_t s0 = blockIdx.x * R, s1 = min(s0 + R, S);
@@ -248,26 +257,43 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
     __syncthreads();
     if (!am_last) return;
     __threadfence();
-    // last CTA: exclusive scans of the block totals (in place)
-    if (warp < 3) {
-        uint32_t* arr = warp == 0 ? a.blk_runs : warp == 1 ? a.blk_grps : a.blk_mids;
-        uint32_t run = 0;
-        for (uint32_t b0 = 0; b0 < gridDim.x; b0 += 32) {
-            const uint32_t b = b0 + lane;
-            const uint32_t x = b < gridDim.x ? __ldcg(&arr[b]) : 0u;
-            const uint32_t incl = warp_incl_scan(x);
-            if (b < gridDim.x) arr[b] = run + incl - x;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+    // last CTA: exclusive scans of the block totals (in place), four a thread so that
+    // all are in flight at once
+    static_assert(4 * THREADS >= kMaxPlanBlocks, "four block totals a thread");
+    uint32_t* const arrs[3] = {a.blk_runs, a.blk_grps, a.blk_mids};
+    const uint32_t bounds[3] = {a.max_runs, a.max_groups, a.max_mids};
+    uint32_t* const counts[3] = {&a.hdr->num_runs, &a.hdr->num_groups, &a.hdr->num_mids};
+    uint32_t* const wsum[3] = {warp_runs, warp_grps, warp_mids};
+    uint32_t x[3][4], incl[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t b = 4u * tid + u;
+            x[q][u] = b < gridDim.x ? __ldcg(&arrs[q][b]) : 0u;
         }
-        if (lane == 0) {
-            if (warp == 0) {
-                a.hdr->num_runs = run <= a.max_runs ? run : 0u;  // over capacity: malformed
-            } else if (warp == 1) {
-                a.hdr->num_groups = run <= a.max_groups ? run : 0u;
-            } else {
-                a.hdr->num_mids = run <= a.max_mids ? run : 0u;
-            }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        incl[q] = warp_incl_scan(x[q][0] + x[q][1] + x[q][2] + x[q][3]);
+        if (lane == 31) wsum[q][warp] = incl[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            before += w < warp ? wsum[q][w] : 0u;
+            all += wsum[q][w];
         }
+        uint32_t run = before + incl[q] - (x[q][0] + x[q][1] + x[q][2] + x[q][3]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (4u * tid + u < gridDim.x) arrs[q][4u * tid + u] = run;
+            run += x[q][u];
+        }
+        if (tid == 0) *counts[q] = all <= bounds[q] ? all : 0u;  // over capacity: malformed
     }
     __syncthreads();
     if (tid == 0) {
@@ -281,9 +307,12 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
 
 template <int P, int THREADS>
 __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
-    __shared__ uint32_t list_seg[THREADS], list_pos[THREADS], list_runs[THREADS];
+    __shared__ uint32_t list_seg[THREADS], list_pos[THREADS], list_a0[THREADS], list_a1[THREADS];
+    __shared__ uint32_t list_m[THREADS];
     __shared__ uint32_t list_n;
     const int tid = threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     const uint64_t S = seg_count(a);
     const uint64_t G = gridDim.x;
     const uint64_t R = (S + G - 1) / G;
@@ -292,6 +321,19 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
     const uint32_t moff = a.blk_mids[blockIdx.x];
     const uint32_t num_runs = a.hdr->num_runs, num_groups = a.hdr->num_groups;
     const uint32_t num_mids = a.hdr->num_mids;
+    // run r of the nr runs of segment s ([a0, a1), class count m), entries from pos on
+    auto emit = [&](uint32_t s, uint32_t a0, uint32_t a1, uint32_t m, uint32_t pos, uint32_t nr,
+                    uint32_t r) {
+        const uint64_t rb = seg_row_start<P>(a0);
+        const uint64_t len = static_cast<uint64_t>(a.run_tiles) * P;
+        RunEntry e;
+        e.seg = s;
+        e.p0 = static_cast<uint32_t>(max(static_cast<uint64_t>(a0), rb + r * len));
+        e.len_m = (static_cast<uint32_t>(min(static_cast<uint64_t>(a1), rb + (r + 1) * len)) - e.p0) |
+                  (m << 24);
+        e.jlast = pos + nr - 1u;
+        a.runs[pos + r] = e;
+    };
     for (uint64_t base = s0; base < s1; base += THREADS) {
         if (tid == 0) list_n = 0;
         __syncthreads();
@@ -305,24 +347,20 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
                 } else if (a1 - a0 > static_cast<uint64_t>(P)) {
                     const uint32_t nr = (seg_tiles<P>(a0, a1) + a.run_tiles - 1) / a.run_tiles;
                     const uint32_t pos = roff + a.run_loc[s];
-                    if (nr <= 16) {  // this thread emits the runs itself
-                        if (static_cast<uint64_t>(pos) + nr <= num_runs) {
-                            const uint64_t rb = seg_row_start<P>(a0);
-                            const uint64_t len = static_cast<uint64_t>(a.run_tiles) * P;
-                            for (uint32_t r = 0; r < nr; r++) {
-                                RunEntry e;
-                                e.seg = static_cast<uint32_t>(s);
-                                e.p0 = static_cast<uint32_t>(max(a0, rb + r * len));
-                                e.p1 = static_cast<uint32_t>(min(a1, rb + (r + 1) * len));
-                                e.jlast = pos + nr - 1u;
-                                a.runs[pos + r] = e;
-                            }
+                    if (static_cast<uint64_t>(pos) + nr <= num_runs) {  // else malformed offsets
+                        const uint32_t m = seg_classes(a, s);
+                        if (nr <= 4) {  // this thread emits the runs itself
+                            for (uint32_t r = 0; r < nr; r++)
+                                emit(static_cast<uint32_t>(s), static_cast<uint32_t>(a0),
+                                     static_cast<uint32_t>(a1), m, pos, nr, r);
+                        } else {  // longer segments: a warp each, below
+                            const uint32_t q = atomicAdd(&list_n, 1u);
+                            list_seg[q] = static_cast<uint32_t>(s);
+                            list_pos[q] = pos;
+                            list_a0[q] = static_cast<uint32_t>(a0);
+                            list_a1[q] = static_cast<uint32_t>(a1);
+                            list_m[q] = m;
                         }
-                    } else {  // long segments: the whole block emits them below
-                        const uint32_t q = atomicAdd(&list_n, 1u);
-                        list_seg[q] = static_cast<uint32_t>(s);
-                        list_pos[q] = pos;
-                        list_runs[q] = nr;
                     }
                 } else if (group_head<P>(a, s, a0)) {
                     const uint32_t g = goff + a.grp_loc[s];
@@ -339,20 +377,11 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
         }
         __syncthreads();
         const uint32_t cnt = list_n;
-        for (uint32_t q = 0; q < cnt; q++) {  // the block emits each large segment's runs
-            const uint32_t seg = list_seg[q], pos = list_pos[q], nr = list_runs[q];
-            if (static_cast<uint64_t>(pos) + nr > num_runs) continue;  // malformed offsets
-            const uint64_t a0 = a.offsets[seg], a1 = a.offsets[seg + 1];
-            const uint64_t rb = seg_row_start<P>(a0);
-            const uint64_t len = static_cast<uint64_t>(a.run_tiles) * P;
-            for (uint32_t r = tid; r < nr; r += THREADS) {
-                RunEntry e;
-                e.seg = seg;
-                e.p0 = static_cast<uint32_t>(max(a0, rb + r * len));
-                e.p1 = static_cast<uint32_t>(min(a1, rb + (r + 1) * len));
-                e.jlast = pos + nr - 1u;
-                a.runs[pos + r] = e;
-            }
+        for (uint32_t q = tid >> 5; q < cnt; q += THREADS / 32) {
+            const uint32_t a0 = list_a0[q], a1 = list_a1[q];
+            const uint32_t nr = (seg_tiles<P>(a0, a1) + a.run_tiles - 1) / a.run_tiles;
+            for (uint32_t r = tid & 31; r < nr; r += 32)
+                emit(list_seg[q], a0, a1, list_m[q], list_pos[q], nr, r);
         }
         __syncthreads();
     }
@@ -364,7 +393,7 @@ struct GroupScratch;
 template <int M, int THREADS>
 constexpr size_t group_scratch_bytes();
 
-template <class V, int M, int THREADS, int STAGES>
+template <class V, int M, int THREADS>
 struct SegSmem {
     using G = TileGeom<V, THREADS, M>;
     static constexpr int kTile = G::kTile;  // == P
@@ -377,9 +406,14 @@ struct SegSmem {
         static_cast<int>(group_window<kTile>()) + kTile + 2 * static_cast<int>(kAU);
     static constexpr size_t kGroupBytes = 2ull * kGroupElems * sizeof(V);
     static constexpr size_t kBytes = 128 + kGroupBytes + group_scratch_bytes<M, THREADS>();  // seg_main
-    // seg_run_scatter: TMA ring + tile stage + count matrix
-    static constexpr size_t kRingBytes = static_cast<size_t>(STAGES) * kTile * sizeof(V);
-    static constexpr size_t kRunBytes = 1024 + kRingBytes + G::kStageBytes + G::kCntBytes;
+};
+
+// seg_run_scatter: TMA slot + tile stage + count matrix
+template <class V, int M, int THREADS>
+struct RunSmem {
+    using G = TileGeom<V, THREADS, M>;
+    static constexpr size_t kSlotBytes = static_cast<size_t>(G::kTile) * sizeof(V);
+    static constexpr size_t kBytes = 1024 + kSlotBytes + G::kStageBytes + G::kCntBytes;
 };
 
 // ------------------------------------------------------------ small segments --
@@ -692,10 +726,10 @@ __device__ __forceinline__ void count_run(const SegArgs& a, const D& d, uint32_t
     const V* in = static_cast<const V*>(a.in);
     const bool in_vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     const RunEntry ent = a.runs[j];
-    const D dj = seg_discr(a, d, ent.seg);
+    const D dj = seg_discr(a, d, ent.len_m >> 24);
     PackedCounts<M> pc;
     pc.init();
-    const uint64_t p0 = ent.p0, p1 = ent.p1;
+    const uint64_t p0 = ent.p0, p1 = ent.p1();
     const uint64_t vs = in_vec ? min((p0 + AU - 1u) & ~static_cast<uint64_t>(AU - 1u), p1) : p1;
     const uint64_t ve = in_vec ? max(vs, p1 & ~static_cast<uint64_t>(AU - 1u)) : p1;
     uint32_t k = 0;
@@ -747,6 +781,8 @@ template <class V, class D, int M, int THREADS>
 __global__ void __launch_bounds__(THREADS, 4) seg_run_count(SegArgs a, D d) {
     __shared__ uint32_t red[2][THREADS / 32][M];
     __shared__ uint32_t ticket_sh[2];
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t num_runs = a.hdr->num_runs;
     for (uint32_t it = 0;; it++) {
         if (threadIdx.x == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket3, 1u);
@@ -758,10 +794,10 @@ __global__ void __launch_bounds__(THREADS, 4) seg_run_count(SegArgs a, D d) {
 }
 
 // Persistent; CTAs take tickets for batches of small-segment groups.
-template <class V, class D, int M, int THREADS, int STAGES>
+template <class V, class D, int M, int THREADS>
 __global__ void __launch_bounds__(THREADS, 3)
     seg_main(SegArgs a, D d) {
-    using L = SegSmem<V, M, THREADS, STAGES>;
+    using L = SegSmem<V, M, THREADS>;
     constexpr uint32_t AU = L::kAU;
     constexpr uint32_t P = L::kTile;
     static_assert(M <= 16 && M >= 2, "class bound");
@@ -785,6 +821,8 @@ __global__ void __launch_bounds__(THREADS, 3)
     V* out = static_cast<V*>(a.out);
     const bool in_vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     const bool out_vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    pdl_launch_dependents();
+    pdl_wait();
     const uint64_t S = seg_count(a);
     const uint32_t num_groups = a.hdr->num_groups;
     // groups per ticket: the tuned batch, but no more than spreads the groups
@@ -919,6 +957,35 @@ __global__ void __launch_bounds__(THREADS, 3)
     if (tid == 0) bulk_wait_all();
 }
 
+// A row of M u32 words in 16-byte (8-byte) accesses.
+template <int M>
+__device__ __forceinline__ void load_row(const uint32_t* p, uint32_t (&x)[M]) {
+    if constexpr (M == 2) {
+        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
+        x[0] = v.x;
+        x[1] = v.y;
+    } else {
+#pragma unroll
+        for (int q = 0; q < M / 4; q++) {
+            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p) + q);
+            x[4 * q] = v.x;
+            x[4 * q + 1] = v.y;
+            x[4 * q + 2] = v.z;
+            x[4 * q + 3] = v.w;
+        }
+    }
+}
+template <int M>
+__device__ __forceinline__ void store_row(uint32_t* p, const uint32_t (&x)[M]) {
+    if constexpr (M == 2) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(x[0], x[1]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < M / 4; q++)
+            reinterpret_cast<uint4*>(p)[q] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    }
+}
+
 // One large segment's runs [j, jl]: lane l takes a contiguous share of the
 // runs, class counts in registers; warp scans per class give each run's
 // output position per class, the segment's sizes and head flags.
@@ -929,13 +996,13 @@ __device__ __forceinline__ void scan_segment_runs(const SegArgs& a, uint32_t j, 
     const uint32_t R = jl - j + 1u;
     const uint32_t per = (R + 31u) >> 5;
     const uint32_t rb = j + min(lane * per, R), re = j + min(lane * per + per, R);
-    uint32_t acc[M];
+    uint32_t acc[M], x[M];
 #pragma unroll
     for (int c = 0; c < M; c++) acc[c] = 0;
     for (uint32_t r = rb; r < re; r++) {
-        const uint32_t* row = a.run_cnt + static_cast<uint64_t>(r) * M;
+        load_row<M>(a.run_cnt + static_cast<uint64_t>(r) * M, x);
 #pragma unroll
-        for (int c = 0; c < M; c++) acc[c] += __ldcg(row + c);
+        for (int c = 0; c < M; c++) acc[c] += x[c];
     }
     uint32_t cur[M];
     uint32_t off = seg_start;
@@ -952,70 +1019,72 @@ __device__ __forceinline__ void scan_segment_runs(const SegArgs& a, uint32_t j, 
         off += tot;
     }
     for (uint32_t r = rb; r < re; r++) {
-        const uint32_t* row = a.run_cnt + static_cast<uint64_t>(r) * M;
-        uint32_t* dst = a.run_base + static_cast<uint64_t>(r) * M;
+        if (per > 1u) load_row<M>(a.run_cnt + static_cast<uint64_t>(r) * M, x);
+        store_row<M>(a.run_base + static_cast<uint64_t>(r) * M, cur);
 #pragma unroll
-        for (int c = 0; c < M; c++) {
-            const uint32_t x = __ldcg(row + c);
-            dst[c] = cur[c];
-            cur[c] += x;
-        }
+        for (int c = 0; c < M; c++) cur[c] += x[c];
     }
 }
 
-// One large segment with few runs [j, jl], by one lane alone.
+// One large segment with at most kLaneRuns runs [j, jl], by one lane alone, the
+// counts of all of them in flight at once.
+constexpr uint32_t kLaneRuns = 4;
 template <int M>
 __device__ __forceinline__ void scan_segment_runs_lane(const SegArgs& a, uint32_t j, uint32_t jl,
                                                        uint32_t seg, uint32_t seg_start) {
-    uint32_t tot[M];
+    uint32_t x[kLaneRuns][M], cur[M];
 #pragma unroll
-    for (int c = 0; c < M; c++) tot[c] = 0;
-    for (uint32_t r = j; r <= jl; r++) {
-        const uint32_t* row = a.run_cnt + static_cast<uint64_t>(r) * M;
+    for (uint32_t r = 0; r < kLaneRuns; r++) {
+        if (j + r <= jl) {
+            load_row<M>(a.run_cnt + static_cast<uint64_t>(j + r) * M, x[r]);
+        } else {
 #pragma unroll
-        for (int c = 0; c < M; c++) tot[c] += __ldcg(row + c);
+            for (int c = 0; c < M; c++) x[r][c] = 0u;
+        }
     }
-    uint32_t cur[M];
     uint32_t off = seg_start;
 #pragma unroll
     for (int c = 0; c < M; c++) {
+        uint32_t tot = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < kLaneRuns; r++) tot += x[r][c];
         cur[c] = off;
         if (a.seg_sizes != nullptr && static_cast<uint32_t>(c) < a.m)
-            a.seg_sizes[static_cast<uint64_t>(seg) * a.m + c] = tot[c];
-        if (a.headflags != nullptr && tot[c] > 0) a.headflags[off] = tot[c];
-        off += tot[c];
+            a.seg_sizes[static_cast<uint64_t>(seg) * a.m + c] = tot;
+        if (a.headflags != nullptr && tot > 0) a.headflags[off] = tot;
+        off += tot;
     }
-    for (uint32_t r = j; r <= jl; r++) {
-        const uint32_t* row = a.run_cnt + static_cast<uint64_t>(r) * M;
-        uint32_t* dst = a.run_base + static_cast<uint64_t>(r) * M;
 #pragma unroll
-        for (int c = 0; c < M; c++) {
-            const uint32_t x = __ldcg(row + c);
-            dst[c] = cur[c];
-            cur[c] += x;
-        }
+    for (uint32_t r = 0; r < kLaneRuns; r++) {
+        if (j + r <= jl) store_row<M>(a.run_base + static_cast<uint64_t>(j + r) * M, cur);
+#pragma unroll
+        for (int c = 0; c < M; c++) cur[c] += x[r][c];
     }
 }
 
-// Every warp looks at 32 consecutive runs at a time: the lane holding a
-// segment's first run scans a segment of at most 4 runs by itself, the whole
-// warp takes the longer ones in turn.
+// Every warp looks at up to 32 consecutive runs at a time (fewer when there are few:
+// the long segments in a warp's part are scanned one after the other): the lane
+// holding a segment's first run scans a segment of at most kLaneRuns runs by itself,
+// the whole warp takes the longer ones in turn.
 template <int M>
 __global__ void __launch_bounds__(256) seg_run_scan(SegArgs a) {
     const uint32_t lane = threadIdx.x & 31u;
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t num_runs = a.hdr->num_runs;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t j0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u; j0 < num_runs;
-         j0 += warps * 32u) {
+    const uint32_t per = min(32u, (num_runs + warps - 1u) / warps);
+    for (uint32_t j0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; j0 < num_runs;
+         j0 += warps * per) {
         const uint32_t j = j0 + lane;
         RunEntry e{};
         bool first = false;
-        if (j < num_runs) {
+        if (lane < per && j < num_runs) {
             e = a.runs[j];
-            first = e.p0 == static_cast<uint32_t>(a.offsets[e.seg]);
+            first = j == 0u || a.runs[j - 1u].seg != e.seg;
         }
         const uint32_t jl = min(e.jlast, num_runs - 1u);
-        const bool shortseg = first && jl >= j && jl - j < 4u;
+        const bool shortseg = first && jl >= j && jl - j < kLaneRuns;
         if (shortseg) scan_segment_runs_lane<M>(a, j, jl, e.seg, e.p0);
         uint32_t longs = __ballot_sync(0xffffffffu, first && !shortseg);
         while (longs != 0u) {
@@ -1029,32 +1098,41 @@ __global__ void __launch_bounds__(256) seg_run_scan(SegArgs a) {
     }
 }
 
-// Every run of a large segment through the TMA ring and tile_scatter, from
-// the run_base positions.  Runs are taken in reverse order of the counts, so
+// Every run of a large segment through a TMA slot and the tile step, from the
+// run_base positions.  Runs are taken in reverse order of the counts, so
 // the first re-reads find the runs counted last still in L2.
-template <class V, class D, int M, int THREADS, int STAGES>
+//
+// A run is 2.5 tiles on average, so what it needs before its first tile is fetched
+// during the run before: its ticket is drawn at the last tile of the run before
+// that, its entry is loaded (by one thread of the last warp, which waits for nothing
+// it has not had a tile's time for) while that run is placed, and at that run's last
+// tile its first tile and its class positions are requested.
+template <class V, class D, int M, int THREADS>
 __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 64 registers
     seg_run_scatter(SegArgs a, D d, const __grid_constant__ CUtensorMap tmap) {
-    using L = SegSmem<V, M, THREADS, STAGES>;
+    using L = RunSmem<V, M, THREADS>;
     using TG = typename L::G;
     constexpr int ITEMS = TG::kItems;
-    constexpr int P = L::kTile;
+    constexpr int P = TG::kTile;
     constexpr int ROWS = TG::kRows;
-    constexpr uint32_t AU = L::kAU;
+    constexpr uint32_t AU = TG::kAU;
     static_assert(M <= 16 && M >= 2, "class bound");
     static_assert(ROWS <= 256, "TMA box height");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-    V* ring = reinterpret_cast<V*>(base);
-    V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + TG::kStageBytes);
+    V* slot = reinterpret_cast<V*>(base);
+    V* stage = reinterpret_cast<V*>(base + L::kSlotBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kSlotBytes + TG::kStageBytes);
 
-    __shared__ __align__(8) uint64_t bars[STAGES];
+    __shared__ __align__(8) uint64_t bar;
     __shared__ TileShared<M> sh;
-    __shared__ uint32_t ticket_sh[2];
+    __shared__ RunEntry ent_sh[2];  // by parity of the run
+    __shared__ uint32_t run_sh[2];  // its index, or kNoRun
 
+    constexpr uint32_t kNoRun = 0xffffffffu;
+    constexpr int kFetcher = THREADS - 32;
     const int tid = threadIdx.x;
     const V* in = static_cast<const V*>(a.in);
     V* out = static_cast<V*>(a.out);
@@ -1063,67 +1141,96 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
     const bool tma_ok = a.use_tma != 0;
     constexpr uint32_t kPerRow = 128u / sizeof(V);  // elements per 128-byte row
     const uint64_t map_elems = (a.n * sizeof(V) / 128u) * kPerRow;
-    const uint32_t num_runs = a.hdr->num_runs;
-    uint32_t ring_uses = 0;  // mbarrier phase bookkeeping across runs
-
     if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < STAGES; s++) mbar_init(&bars[s], 1);
+        mbar_init(&bar, 1);
         mbar_fence_init();
     }
-    __syncthreads();
+    pdl_wait();
+    const uint32_t num_runs = a.hdr->num_runs;
 
-    for (uint32_t it = 0;; it++) {
-        if (tid == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket2, 1u);
-        __syncthreads();
-        const uint32_t t = ticket_sh[it & 1u];
-        if (t >= num_runs) break;
-        const uint32_t j = num_runs - 1u - t;
-        const RunEntry ent = a.runs[j];
-        const D dj = seg_discr(a, d, ent.seg);
-        if (tid < M) sh.cursor[0][tid] = __ldcg(a.run_base + static_cast<uint64_t>(j) * M + tid);
-        __syncthreads();
-        // the run's tiles start at the 128-byte row holding its first element
-        // (not at multiples of P), so only its last tile is short
-        const uint64_t rb = ent.p0 & ~static_cast<uint64_t>(kPerRow - 1u);
-        const uint32_t ntiles = static_cast<uint32_t>((ent.p1 - rb + P - 1u) / P);
-        // a tile comes by TMA when the run's part of it lies inside the tensor
-        // map (the input's whole 128-byte rows; rows past the map read as zeros
-        // and lie outside the run)
-        auto via_tma = [&](uint32_t i) {
-            return tma_ok && min(static_cast<uint64_t>(ent.p1), rb + static_cast<uint64_t>(i + 1) * P) <= map_elems;
-        };
-        auto issue = [&](uint32_t i) {  // tile i of the run into ring slot (ring_uses+i) % STAGES
-            const uint32_t slot = (ring_uses + i) % STAGES;
-            if (via_tma(i)) {
-                mbar_arrive_expect_tx(&bars[slot], P * sizeof(V));
-                tma_load_2d(ring + slot * P, &tmap, 0,
-                            static_cast<int32_t>(rb / kPerRow + static_cast<uint64_t>(i) * ROWS), &bars[slot]);
-            } else {
-                mbar_arrive(&bars[slot]);
-            }
-        };
-        if (tid == 0)
-            for (uint32_t i = 0; i < STAGES && i < ntiles; i++) issue(i);
-        const uint32_t e0 = tid * ITEMS;
-        bool failed = false;
+    // the run's tiles start at the 128-byte row holding its first element
+    // (not at multiples of P), so only its last tile is short
+    auto row_start = [&](const RunEntry& e) {
+        return static_cast<uint64_t>(e.p0 & ~(kPerRow - 1u));
+    };
+    // a tile comes by TMA when the run's part of it lies inside the tensor
+    // map (the input's whole 128-byte rows; rows past the map read as zeros
+    // and lie outside the run)
+    auto via_tma = [&](const RunEntry& e, uint32_t i) {
+        return tma_ok && min(static_cast<uint64_t>(e.p1()),
+                             row_start(e) + static_cast<uint64_t>(i + 1) * P) <= map_elems;
+    };
+    auto issue = [&](const RunEntry& e, uint32_t i) {  // thread 0: tile i of a run
+        if (via_tma(e, i)) {
+            mbar_arrive_expect_tx(&bar, P * sizeof(V));
+            tma_load_2d(slot, &tmap, 0,
+                        static_cast<int32_t>(row_start(e) / kPerRow + static_cast<uint64_t>(i) * ROWS),
+                        &bar);
+        } else {
+            mbar_arrive(&bar);
+        }
+    };
+    // kFetcher's state: the ticket of the run after the next known one, and its entry
+    uint32_t ticket = 0;
+    RunEntry next_ent{};
+    bool have_next = false;
+    auto fetch_entry = [&] {  // the entry of `ticket`'s run, used only later
+        have_next = ticket < num_runs;
+        if (have_next) next_ent = a.runs[num_runs - 1u - ticket];
+    };
+    auto publish = [&](uint32_t q) {
+        ent_sh[q] = next_ent;
+        run_sh[q] = have_next ? num_runs - 1u - ticket : kNoRun;
+    };
+    if (tid == kFetcher) {
+        ticket = atomicAdd(&a.hdr->ticket2, 1u);
+        fetch_entry();
+        publish(0);
+        ticket = have_next ? atomicAdd(&a.hdr->ticket2, 1u) : num_runs;
+    }
+    __syncthreads();
+    if (run_sh[0] != kNoRun) {
+        if (tid == 0) issue(ent_sh[0], 0);
+        if (tid < M) sh.cursor[0][tid] = __ldcg(a.run_base + static_cast<uint64_t>(run_sh[0]) * M + tid);
+    }
+
+    const uint32_t e0 = tid * ITEMS;
+    uint32_t uses = 0;  // of the slot
+    bool failed = false;
+    for (uint32_t q = 0; !failed && run_sh[q] != kNoRun; q ^= 1u) {
+        const RunEntry ent = ent_sh[q];
+        const D dj = seg_discr(a, d, ent.len_m >> 24);
+        if (tid == kFetcher) fetch_entry();
+        const uint64_t rb = row_start(ent);
+        const uint32_t ntiles = static_cast<uint32_t>((ent.p1() - rb + P - 1u) / P);
+        uint32_t next_cur = 0;
         for (uint32_t i = 0; i < ntiles; i++) {
             const uint64_t ts = rb + static_cast<uint64_t>(i) * P;
             const uint32_t lo = static_cast<uint32_t>(max(static_cast<uint64_t>(ent.p0), ts) - ts);
-            const uint32_t hi = static_cast<uint32_t>(min(static_cast<uint64_t>(ent.p1), ts + P) - ts);
+            const uint32_t hi = static_cast<uint32_t>(min(static_cast<uint64_t>(ent.p1()), ts + P) - ts);
             const bool full = lo == 0u && hi == static_cast<uint32_t>(P);
-            const uint32_t use = ring_uses + i;
-            const bool ok = mbar_wait_bounded(&bars[use % STAGES], (use / STAGES) & 1u);
+            const bool last = i + 1u == ntiles;
+            const bool ok = mbar_wait_bounded(&bar, uses & 1u);
             V v[ITEMS];
-            if (via_tma(i)) {
-                take_swizzled<V, ITEMS>(ring + (use % STAGES) * P, v);
+            if (via_tma(ent, i)) {
+                take_swizzled<V, ITEMS>(slot, v);
             } else {
 #pragma unroll
-                for (int q = 0; q < ITEMS; q++)
-                    v[q] = (e0 + q >= lo && e0 + q < hi) ? in[ts + e0 + q] : V();
+                for (int z = 0; z < ITEMS; z++)
+                    v[z] = (e0 + z >= lo && e0 + z < hi) ? in[ts + e0 + z] : V();
             }
-            auto refill = [&] {
-                if (tid == 0 && i + STAGES < ntiles) issue(i + STAGES);
+            if (last && tid == kFetcher) {
+                publish(q ^ 1u);
+                ticket = have_next ? atomicAdd(&a.hdr->ticket2, 1u) : num_runs;
+            }
+            auto refill = [&] {  // the slot is free: the next tile of this run or of the next
+                if (!last) {
+                    if (tid == 0) issue(ent, i + 1u);
+                } else if (run_sh[q ^ 1u] != kNoRun) {
+                    if (tid == 0) issue(ent_sh[q ^ 1u], 0);
+                    if (tid < M)
+                        next_cur = __ldcg(a.run_base + static_cast<uint64_t>(run_sh[q ^ 1u]) * M + tid);
+                }
             };
             bool done;
             if constexpr (M == 2)
@@ -1131,21 +1238,21 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
                                                         OutFlat<V>{out, out_phase}, ok, refill);
             else
                 done = tile_scatter<V, D, M, THREADS, true, false>(dj, v, lo, hi, full, stage, cnt_sm, sh,
-                                                            i & 1u, OutFlat<V>{out, out_phase}, ok,
-                                                            refill);
+                                                                   i & 1u, OutFlat<V>{out, out_phase},
+                                                                   ok, refill);
             if (!done) {
                 failed = true;
-                if (tid == 0) {
+                if (tid == 0) {  // only this tile's copy can be in flight
                     atomicOr(&a.hdr->error, kErrTimeout);
-                    for (uint32_t q = i; q < ntiles && q < i + STAGES; q++)
-                        (void)mbar_wait_bounded(&bars[(ring_uses + q) % STAGES],
-                                                ((ring_uses + q) / STAGES) & 1u);
+                    (void)mbar_wait_bounded(&bar, uses & 1u);
                 }
                 break;
             }
+            uses++;
         }
-        ring_uses += ntiles;
-        if (failed) break;
+        // read after the next tile's first barrier; this run's last reads of the
+        // cursors lie before its last tile's third
+        if (tid < M) sh.cursor[0][tid] = next_cur;
     }
     if (tid < M) bulk_wait_all();
 }
@@ -1213,6 +1320,8 @@ __global__ void __launch_bounds__(THREADS, 4)
         static_cast<uint32_t>(reinterpret_cast<uintptr_t>(out) / sizeof(V)) & (AU - 1u);
     const bool tma_ok = a.use_tma != 0;
     const uint64_t map_elems = (a.n * sizeof(V) / 128u) * kPerRow;
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t num_mids = a.hdr->num_mids;
     const uint32_t G = gridDim.x;
     const uint32_t e0 = tid * ITEMS;
@@ -1293,7 +1402,7 @@ __global__ void __launch_bounds__(THREADS, 4)
             n1 = a.offsets[s_next + 1];
         }
         const uint32_t s_after = t + 2u * G < num_mids ? a.mids[t + 2u * G] : 0u;
-        const D dj = seg_discr(a, d, cur.s);
+        const D dj = seg_discr(a, d, seg_classes(a, cur.s));
 
         // ---- count pass: lane c of every warp keeps the warp's count of class c
         uint32_t wt = 0;
@@ -1387,110 +1496,130 @@ __global__ void __launch_bounds__(THREADS, 4)
 // into offsets[0..S] and S (in the header); the planner then checks that every
 // flag equals the distance to the next start.
 //
-//   seg_flags_stage    CTA k reads chunk k of the flags once (tiles of FT
-//                      flags, 16 per thread), writes the positions of its
-//                      non-zero flags in order into its own part of a staging
-//                      array (stage[chunk start + j]) and its count; the last
-//                      CTA to finish (ticket, no waiting) scans the chunk
-//                      counts into chunk prefixes, S and offsets[S] = n.
-//   seg_flags_compact  CTA k moves its staged positions to offsets[prefix + j].
+//   seg_flags_stage    a warp per chunk reads its flags once, eight 16-byte words a
+//                      lane in flight, and writes the positions of its non-zero
+//                      flags in order into the chunk's part of a staging array
+//                      (stage[chunk start + j]) and their number; the last CTA to
+//                      finish (ticket, no waiting) scans the chunk counts into
+//                      chunk prefixes, S and offsets[S] = n.
+//   seg_flags_compact  a warp per chunk moves its staged positions to
+//                      offsets[prefix + j].
 //
-// No CTA waits on another: the single pass with a decoupled look-back that
-// this replaces spent most of its time walking predecessors, because ~10^3
-// tiles of a few microseconds each were in flight at once.
+// Flags are sparse (a segment has one): a word of all lanes without one costs a
+// vote.  No CTA waits on another, and no warp on its CTA before the end: 10^8 flags
+// in 87 us when CTAs read tiles of 4096 flags with two barriers each, FLAGFIG now
+// (61 at the copy rate).
+constexpr uint32_t kMaxFlagChunks = 4096;
+
 struct FlagsArgs {
     const int32_t* flags;
     uint64_t n;
-    uint64_t chunk;      // flags per chunk (a multiple of 4)
+    uint64_t chunk;      // flags per chunk (a multiple of 128)
     uint32_t* stage;     // [n] staged start positions, chunk k's from k * chunk
-    uint32_t* cnt;       // [G] start positions per chunk
-    uint32_t* pre;       // [G] exclusive prefix of cnt
+    uint32_t* cnt;       // [chunks] start positions per chunk
+    uint32_t* pre;       // [chunks] exclusive prefix of cnt
     uint64_t* offsets;   // [S + 1]
     SegHeader* hdr;
 };
 
-template <int THREADS, int FT>
+template <int THREADS>
 __global__ void __launch_bounds__(THREADS) seg_flags_stage(FlagsArgs fa) {
-    constexpr int ITEMS = FT / THREADS;
     constexpr int W = THREADS / 32;
-    static_assert(ITEMS * THREADS == FT && ITEMS % 4 == 0, "tile");
+    constexpr int U = 8;
+    constexpr int PER = static_cast<int>(kMaxFlagChunks) / THREADS;
     __shared__ uint32_t warp_tot[W];
     __shared__ int last_sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t c0 = min(static_cast<uint64_t>(blockIdx.x) * fa.chunk, fa.n);
+    pdl_launch_dependents();
+    const uint32_t k = blockIdx.x * W + warp;
+    const uint64_t c0 = min(static_cast<uint64_t>(k) * fa.chunk, fa.n);
     const uint64_t c1 = min(c0 + fa.chunk, fa.n);
-    const bool vec = (reinterpret_cast<uintptr_t>(fa.flags) & 15u) == 0;
-    uint32_t running = 0;  // start positions of this chunk so far
+    uint32_t* out = fa.stage + c0;
     bool bad = false;
-    for (uint64_t ts = c0; ts < c1; ts += FT) {
-        const uint64_t e0 = ts + static_cast<uint64_t>(tid) * ITEMS;
-        int32_t f[ITEMS];
-        if (vec && e0 + ITEMS <= c1) {
+    // four flags a lane, in order over the lanes: positions of the non-zero ones
+    auto take = [&](const int4& f, uint64_t e) {
+        const uint32_t nz = (f.x != 0 ? 1u : 0u) | (f.y != 0 ? 2u : 0u) | (f.z != 0 ? 4u : 0u) |
+                            (f.w != 0 ? 8u : 0u);
+        if (__ballot_sync(0xffffffffu, nz != 0u) == 0u) return;
+        bad |= (f.x | f.y | f.z | f.w) < 0;
+        const uint32_t c = static_cast<uint32_t>(__popc(nz));
+        const uint32_t incl = warp_incl_scan(c);
+        uint32_t* p = out + (incl - c);
 #pragma unroll
-            for (int q = 0; q < ITEMS / 4; q++) {
-                const int4 r = __ldg(reinterpret_cast<const int4*>(fa.flags + e0) + q);
-                f[4 * q] = r.x; f[4 * q + 1] = r.y; f[4 * q + 2] = r.z; f[4 * q + 3] = r.w;
-            }
-        } else {
+        for (uint32_t q = 0; q < 4; q++)
+            if (nz >> q & 1u) *p++ = static_cast<uint32_t>(e + q);
+        out += __shfl_sync(0xffffffffu, incl, 31);
+    };
+    uint64_t e = c0 + 4u * lane;
+    if ((reinterpret_cast<uintptr_t>(fa.flags) & 15u) == 0) {
+        for (; e - 4u * lane + 128u * U <= c1; e += 128u * U) {
+            int4 f[U];
 #pragma unroll
-            for (int q = 0; q < ITEMS; q++) f[q] = e0 + q < c1 ? __ldg(fa.flags + e0 + q) : 0;
+            for (int u = 0; u < U; u++) f[u] = __ldg(reinterpret_cast<const int4*>(fa.flags + e + 128u * u));
+            int any = 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) any |= f[u].x | f[u].y | f[u].z | f[u].w;
+            if (__ballot_sync(0xffffffffu, any != 0) == 0u) continue;
+#pragma unroll
+            for (int u = 0; u < U; u++) take(f[u], e + 128u * u);
         }
-        uint32_t nz = 0;
-#pragma unroll
-        for (int q = 0; q < ITEMS; q++) {
-            nz += f[q] != 0 ? 1u : 0u;
-            bad |= f[q] < 0;
-        }
-        const uint32_t incl = warp_incl_scan(nz);
-        if (lane == 31) warp_tot[warp] = incl;
-        __syncthreads();
-        uint32_t wpre = 0, agg = 0;
-#pragma unroll
-        for (int w = 0; w < W; w++) {
-            const uint32_t x = warp_tot[w];
-            wpre += w < warp ? x : 0u;
-            agg += x;
-        }
-        uint32_t pos = running + wpre + incl - nz;
-#pragma unroll
-        for (int q = 0; q < ITEMS; q++)
-            if (f[q] != 0) fa.stage[c0 + pos++] = static_cast<uint32_t>(e0 + q);
-        running += agg;
-        __syncthreads();  // warp_tot is rewritten by the next tile
+    }
+    for (; e - 4u * lane < c1; e += 128u) {  // the rest, and all of unaligned flags
+        int4 f;
+        f.x = e < c1 ? __ldg(fa.flags + e) : 0;
+        f.y = e + 1u < c1 ? __ldg(fa.flags + e + 1u) : 0;
+        f.z = e + 2u < c1 ? __ldg(fa.flags + e + 2u) : 0;
+        f.w = e + 3u < c1 ? __ldg(fa.flags + e + 3u) : 0;
+        take(f, e);
     }
     if (bad) atomicOr(&fa.hdr->error, kErrSegments);
-    if (tid == 0) {
-        fa.cnt[blockIdx.x] = running;
-        __threadfence();
-        last_sh = (atomicAdd(&fa.hdr->flags_done, 1u) == gridDim.x - 1u);
-    }
+    if (lane == 0) fa.cnt[k] = static_cast<uint32_t>(out - (fa.stage + c0));
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last_sh = (atomicAdd(&fa.hdr->flags_done, 1u) == gridDim.x - 1u);
     __syncthreads();
     if (!last_sh) return;
     __threadfence();
-    // last CTA: exclusive scan of the chunk counts (one warp), S, offsets[S]
-    if (warp == 0) {
-        uint64_t run = 0;
-        for (uint32_t b0 = 0; b0 < gridDim.x; b0 += 32) {
-            const uint32_t b = b0 + lane;
-            const uint32_t x = b < gridDim.x ? __ldcg(&fa.cnt[b]) : 0u;
-            const uint32_t inc = warp_incl_scan(x);
-            if (b < gridDim.x) fa.pre[b] = static_cast<uint32_t>(run) + inc - x;
-            run += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) {
-            fa.hdr->num_segs = run;
-            fa.offsets[run] = fa.n;
-            if (fa.n > 0 && __ldg(fa.flags) == 0) atomicOr(&fa.hdr->error, kErrSegments);
-            fa.hdr->flags_done = 0u;  // for the next call
-        }
+    // last CTA: exclusive scan of the chunk counts, S, offsets[S]
+    const uint32_t chunks = gridDim.x * W;
+    uint32_t x[PER], sum = 0;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const uint32_t b = static_cast<uint32_t>(tid) * PER + q;
+        x[q] = b < chunks ? __ldcg(&fa.cnt[b]) : 0u;
+        sum += x[q];
+    }
+    const uint32_t incl = warp_incl_scan(sum);
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+        before += w < warp ? warp_tot[w] : 0u;
+        all += warp_tot[w];
+    }
+    uint32_t run = before + incl - sum;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const uint32_t b = static_cast<uint32_t>(tid) * PER + q;
+        if (b < chunks) fa.pre[b] = run;
+        run += x[q];
+    }
+    if (tid == 0) {
+        fa.hdr->num_segs = all;
+        fa.offsets[all] = fa.n;
+        if (fa.n > 0 && __ldg(fa.flags) == 0) atomicOr(&fa.hdr->error, kErrSegments);
+        fa.hdr->flags_done = 0u;  // for the next call
     }
 }
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) seg_flags_compact(FlagsArgs fa) {
-    const uint64_t c0 = min(static_cast<uint64_t>(blockIdx.x) * fa.chunk, fa.n);
-    const uint32_t k = fa.cnt[blockIdx.x], p = fa.pre[blockIdx.x];
-    for (uint32_t j = threadIdx.x; j < k; j += THREADS) fa.offsets[p + j] = fa.stage[c0 + j];
+    pdl_wait();
+    const uint32_t w = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
+    const uint64_t c0 = min(static_cast<uint64_t>(w) * fa.chunk, fa.n);
+    const uint32_t k = fa.cnt[w], p = fa.pre[w];
+    for (uint32_t j = threadIdx.x & 31u; j < k; j += 32u) fa.offsets[p + j] = fa.stage[c0 + j];
 }
 
 }  // namespace mdx

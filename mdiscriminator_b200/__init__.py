@@ -323,10 +323,11 @@ def partition(d_in, discr, out=None, sizes=None, headflags=False, ws: Optional[W
     elif headflags is not False and headflags is not None:
         hf = headflags
     _require_cuda(out, sizes, hf)
-    need = workspace_size(n, elem, dc.m)
-    if need == 0:
-        raise MdxError(MDX_ERR_INVALID, "mdx_workspace_size")
-    ws = ws or workspace(need, d_in.device, stream)
+    if ws is None:
+        need = workspace_size(n, elem, dc.m)
+        if need == 0:
+            raise MdxError(MDX_ERR_INVALID, "mdx_workspace_size")
+        ws = workspace(need, d_in.device, stream)
     ev = ctypes.c_void_p(count_done_event.cuda_event if count_done_event is not None else 0)
     st = lib().mdx_partition_timed(ctypes.c_void_p(d_in.data_ptr()),
                                    ctypes.c_void_p(out.data_ptr()), n, elem, dc,
@@ -508,10 +509,11 @@ def partition_segmented(d_in, d_offsets, discr, out=None, seg_sizes=None, headfl
     elif headflags is not False and headflags is not None:
         hf = headflags
     _require_cuda(out, seg_sizes, hf)
-    need = segmented_workspace_size(n, S, elem, dc.m)
-    if need == 0:
-        raise MdxError(MDX_ERR_INVALID, "mdx_segmented_workspace_size")
-    ws = ws or workspace(need, d_in.device, stream)
+    if ws is None:
+        need = segmented_workspace_size(n, S, elem, dc.m)
+        if need == 0:
+            raise MdxError(MDX_ERR_INVALID, "mdx_segmented_workspace_size")
+        ws = workspace(need, d_in.device, stream)
     st = lib().mdx_partition_segmented(
         ctypes.c_void_p(d_in.data_ptr()), ctypes.c_void_p(out.data_ptr()), n, elem, dc,
         ctypes.c_void_p(d_offsets.data_ptr()), S, ctypes.c_void_p(seg_sizes.data_ptr()),

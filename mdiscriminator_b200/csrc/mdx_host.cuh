@@ -15,6 +15,7 @@
 #include "mdx_fused.cuh"
 #include "mdx_plain.cuh"
 #include "mdx_segm.cuh"
+#include "mdx_small.cuh"
 #include "mdx_tile.cuh"
 
 namespace mdx {
@@ -344,6 +345,33 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
         if (ev_mid != nullptr && cudaEventRecord(ev_mid, stream) != cudaSuccess) return MDX_ERR_CUDA;
         return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
     }
+    if constexpr (kBase) {
+        // a cluster's worth of tiles: one launch, whatever form the knobs pick for
+        // larger inputs (the two kernels apart stay apart)
+        if (step == PlainStep::kBoth && dist == nullptr && ev_mid == nullptr && nt <= kSmallTiles) {
+            using SL = SmallSmem<V, M, kThreads>;
+            auto small = plain_small_kernel<V, D, M, kThreads>;
+            int sb = 0, ss = 0;  // sets the shared-memory limit once
+            if (occupancy(reinterpret_cast<const void*>(small), SL::kBytes, &sb, &ss) != cudaSuccess)
+                return MDX_ERR_CUDA;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(nt);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = SL::kBytes;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = nt;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            const OutFlat<V> o{static_cast<V*>(d_out),
+                               static_cast<uint32_t>((reinterpret_cast<uintptr_t>(d_out) / sizeof(V)) &
+                                                     (16u / sizeof(V) - 1u))};
+            return cudaLaunchKernelEx(&cfg, small, a, d, o) == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
+        }
+    }
     if constexpr (kBase) {  // the one-kernel path has the base geometry only
         if (step == PlainStep::kBoth && dist == nullptr && ev_mid == nullptr && allow_fused &&
             tun.plain_two_kernel == 0) {
@@ -476,7 +504,8 @@ mdx_status run_plain(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
                      const DistOut* dist = nullptr, bool allow_fused = true) {
     if constexpr (sizeof(V) <= 8) {
         const Tuning tun = tuning_for(sizeof(V) == 8 ? MDX_ELEM_REC8 : MDX_ELEM_U32, M, n);
-        if (dist == nullptr && step == PlainStep::kBoth) {
+        constexpr uint64_t kBaseTile = kThreads * 64 / sizeof(V);
+        if (dist == nullptr && step == PlainStep::kBoth && n > kSmallTiles * kBaseTile) {
             if (tun.tile_threads == 512)
                 return run_plain_g<V, D, M, 64, 512>(d_in, d_out, n, d, m, d_sizes, d_headflags, ws,
                                                      L, stream, ev_mid, step, dist, allow_fused);

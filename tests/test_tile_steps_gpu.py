@@ -90,3 +90,32 @@ def test_records_of_16_bytes(cuda_ready, m):
             torch.cuda.synchronize()
             assert np.array_equal(out.cpu().numpy().view(np.uint32), rows[order])
             assert np.array_equal(sizes.cpu().numpy(), np.bincount(keys % m, minlength=m))
+
+
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 13, 32, 64])
+def test_a_few_tiles_in_one_launch(cuda_ready, m, rec):
+    """Up to eight tiles of 16 KB go through one cluster launch: its tile edges, the
+    largest size it takes and the first it does not, buffers off their alignment."""
+    torch = cuda_ready
+    tile = 2048 if rec else 4096
+    kind = np.int64 if rec else np.int32
+    for n in (1, 15, tile - 1, tile, tile + 1, 5 * tile + 77, 8 * tile - 1, 8 * tile, 8 * tile + 1):
+        for form in ("runs", "sorted"):
+            x = clustered(n, m, form, m + n)
+            if rec:
+                x = x.astype(np.uint64) | (np.arange(n, dtype=np.uint64) << np.uint64(32))
+            eo, es, ef = oracle.partition(x, m, headflags=True)
+            for off_in, off_out in ((0, 0), (1, 0), (0, 1)):
+                base = torch.zeros(n + 2, dtype=torch.int64 if rec else torch.int32, device="cuda")
+                base[off_in:off_in + n] = torch.from_numpy(x.view(kind)).cuda()
+                out = torch.zeros_like(base)
+                o, sizes, hf = mdx.partition(base[off_in:off_in + n], ("mod", m),
+                                             out=out[off_out:off_out + n], headflags=True)
+                torch.cuda.synchronize()
+                assert np.array_equal(sizes.cpu().numpy(), es), (n, form)
+                assert np.array_equal(o.cpu().numpy().view(x.dtype), eo), (n, form, off_in, off_out)
+                assert np.array_equal(hf.cpu().numpy().view(np.uint32), ef), (n, form)
+                assert not out[:off_out].any() and not out[off_out + n:].any()
+        host, host_sizes = mdx.mdiscr(base[:n].clone(), ("mod", m))
+        assert sum(host_sizes) == n

@@ -55,7 +55,8 @@ PLAIN_CANDIDATES = [(1, 0, 0, 64, 256), (1, 3, 0, 64, 256), (1, 2, 0, 64, 256),
 
 def timeit(graph, torch, reps=9):
     """Median time of one of ten replays of a captured call (no host time between
-    its launches)."""
+    its launches).  Replays of a few microseconds come in steps of two, so a
+    candidate has to be clearly faster to replace the one before it."""
     for _ in range(10):
         graph.launch()
     torch.cuda.synchronize()
@@ -116,7 +117,7 @@ def main(argv=None):
                     ms = timeit(mdx.capture_partition(d, ("mask", M), out, sizes, ws=ws), torch)
                     if ws.error() != mdx.MDX_OK:
                         raise SystemExit(f"device error while tuning {ename} m={M}")
-                    if best is None or ms < 0.99 * best[0]:  # ties stay with the first
+                    if best is None or ms < 0.96 * best[0]:  # ties stay with the first
                         best = (ms, k, two, pool, tb, tt)
                 entries.append({"elem": ename, "m": M, "log2_n": [lo, hi], "path": "plain",
                                 "plain_ctas_per_sm": best[1], "plain_two_kernel": best[2],
@@ -156,7 +157,7 @@ def main(argv=None):
                                    tile_threads=tt, run_tiles=rt, group_batch=gb, mid_tiles=mid)
                     ms = timeit(mdx.capture_partition_segmented(d, do, ("mask", M), out, ss, ws=ws),
                                 torch)
-                    if best is None or ms < 0.99 * best[0]:
+                    if best is None or ms < 0.98 * best[0]:
                         best = (ms, rt, gb, mid)
                 entries.append({"elem": ename, "m": M, "log2_n": [lo, hi], "path": "segmented",
                                 "plain_ctas_per_sm": plain_k, "plain_two_kernel": plain_two,

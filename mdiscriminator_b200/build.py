@@ -1,6 +1,6 @@
 """Build recipe for libmdx.so (sm_100a) -- run by ``__graft_entry__.build()``.
 
-Compiles ``csrc/mdx_capi.cu`` (which includes every kernel header) with nvcc
+Compiles the sources under ``csrc/`` (which include the kernel headers) with nvcc
 directly into ``mdiscriminator_b200/libmdx.so``, in-tree, so the library
 travels with the repository snapshot.
 """
@@ -13,8 +13,8 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libmdx.so")
-SOURCES = [os.path.join(HERE, "csrc", "mdx_capi.cu"), os.path.join(HERE, "csrc", "mdx_noalloc.cu"),
-           os.path.join(HERE, "csrc", "mdx_server.cu"), os.path.join(HERE, "csrc", "mdx_wide.cu")]
+SOURCES = [os.path.join(HERE, "csrc", f) for f in
+           ("mdx_capi.cu", "mdx_capi_segm.cu", "mdx_noalloc.cu", "mdx_server.cu", "mdx_wide.cu")]
 HEADERS_DIRS = [os.path.join(HERE, "csrc"), os.path.join(os.path.dirname(HERE), "include")]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -47,6 +47,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
         return LIB
     cmd = [nvcc(), *ARCH, "-lineinfo", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
+           "-t", str(len(SOURCES)),  # the sources at the same time
            "-Xptxas", "-v" if verbose else "-O3", "-o", LIB + ".tmp", *SOURCES]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

@@ -87,7 +87,8 @@ template <class V, class D, int M, int THREADS, int STAGES>
 __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 64 registers
     plain_fused_kernel(FusedArgs fa, D d, const __grid_constant__ CUtensorMap tmap,
                        const __grid_constant__ OutFlat<V> out) {
-    using L = ScatterTmaSmem<V, THREADS, STAGES, M>;
+    static_assert(STAGES == 2, "ring slots");
+    using L = ScatterTmaSmem<V, THREADS, M>;
     constexpr int ITEMS = L::kItems;
     constexpr int TILE = L::kTile;
     constexpr int ROWS = L::kRows;
@@ -100,8 +101,8 @@ __global__ void __launch_bounds__(THREADS, 4)  // 4 CTAs (32 warps) per SM: <= 6
     const uint32_t raw = smem_addr(smem_raw);
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* ring = reinterpret_cast<V*>(base);
-    V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + L::G::kStageBytes);
+    V* stage = reinterpret_cast<V*>(base + STAGES * L::kSlotBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + STAGES * L::kSlotBytes + L::G::kStageBytes);
     // count-phase tables in the (still unused) stage: chunk reduction [W][M];
     // pool-tile counts by tile parity, M <= 16: [2][W][HW] pairs, else [2][W][M]
     uint32_t* red = reinterpret_cast<uint32_t*>(stage);

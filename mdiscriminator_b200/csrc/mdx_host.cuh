@@ -6,6 +6,7 @@
 #include <cuda.h>  // CUtensorMap and its enums (the encoder is fetched from the runtime)
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -23,13 +24,16 @@ namespace host {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kMaxChunks = 4096;
-constexpr int kStages = 2;  // TMA ring of the one-kernel path and of the segmented run scatter
+constexpr int kStages = 2;  // TMA ring of the one-kernel path
 // The plain scatter's ring has one slot: a tile is taken into registers at
 // once, so the next copy overlaps all but the take.  A second slot per CTA was
 // slower at every class count (N = 2^28 u32, 256 threads: scatter at m = 2, 8,
 // 16: 383, 370, 465 us with two slots, 346, 358, 440 with one): the reads in
-// flight beyond what covers the latency only compete with the writes.
-constexpr int kScatterStages = 1;
+// flight beyond what covers the latency only compete with the writes.  A CTA with
+// two tiles has no earlier step to overlap the second one's copy with: two slots
+// (n = 1.5 * 10^6 records of 8 bytes, m = 16, 1.2 tiles a CTA: scatter 11.2 us with
+// one, 10.7 with two; twice as many records: the call 20.7 with one, 22.5 with two).
+constexpr uint32_t kTwoSlotTiles = 2;  // tiles a CTA up to which the ring has two slots
 constexpr size_t kHeaderBytes = 256;  // done, error, ... (see WsHeader)
 constexpr size_t kAlign = 256;
 
@@ -120,16 +124,17 @@ inline mdx_status check_elem(mdx_elem e) {
                                                                                : MDX_ERR_INVALID;
 }
 
-// Resident CTAs per SM of a kernel, cached per (device, kernel).
+// Resident CTAs per SM of a kernel, cached per (device, kernel, shared memory).
 struct OccEntry {
     int device;
     const void* fn;
+    size_t smem;
     int blocks;
     int sms;
 };
 struct OccCache {
     std::mutex mu;
-    OccEntry e[256];
+    OccEntry e[512];
     int n = 0;
 };
 inline OccCache& occ_cache() {
@@ -149,17 +154,14 @@ inline cudaError_t occupancy(const void* fn, size_t dyn_smem, int* blocks, int* 
     {
         std::lock_guard<std::mutex> lk(g_occ_mu);
         for (int i = 0; i < g_occ_n; i++)
-            if (g_occ[i].device == dev && g_occ[i].fn == fn) {
+            if (g_occ[i].device == dev && g_occ[i].fn == fn && g_occ[i].smem == dyn_smem) {
                 *blocks = g_occ[i].blocks;
                 *sms = g_occ[i].sms;
                 return cudaSuccess;
             }
     }
-    if (dyn_smem > 0) {  // the 48 KB a kernel has without asking hold its static part too
-        err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(dyn_smem));
-        if (err != cudaSuccess) return err;
-    }
+    // (the 48 KB a kernel has without asking hold its static part too)
+    if ((err = raise_smem_limit(fn, dyn_smem)) != cudaSuccess) return err;
     int b = 0, s = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, dyn_smem);
     if (err != cudaSuccess) return err;
@@ -167,7 +169,7 @@ inline cudaError_t occupancy(const void* fn, size_t dyn_smem, int* blocks, int* 
     if (err != cudaSuccess) return err;
     if (b < 1) b = 1;
     std::lock_guard<std::mutex> lk(g_occ_mu);
-    if (g_occ_n < 256) g_occ[g_occ_n++] = OccEntry{dev, fn, b, s};
+    if (g_occ_n < 512) g_occ[g_occ_n++] = OccEntry{dev, fn, dyn_smem, b, s};
     *blocks = b;
     *sms = s;
     return cudaSuccess;
@@ -293,19 +295,24 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     constexpr bool kBase = BPT == 64 && TS == kThreads;  // the geometry of every path
     static_assert(BPT != 64 || ITEMS == ElemCfg<V>::kItems, "64-byte tiles");
     auto count = plain_count_kernel<V, D, M, TS, TILE>;
-    const void* scatter_fn;
-    size_t smem;
-    {
-        using SL = ScatterTmaSmem<V, TS, kScatterStages, M, BPT>;
-        static_assert(SL::kTile == TILE, "both kernels use the same tiles");
-        scatter_fn = reinterpret_cast<const void*>(
-            plain_scatter_tma_kernel<V, D, M, TS, kScatterStages, OutFlat<V>, BPT>);
-        smem = SL::kBytes;
-    }
-    int blocks = 0, sms = 0;
-    if (occupancy(scatter_fn, smem, &blocks, &sms, TS) != cudaSuccess) return MDX_ERR_CUDA;
+    using SL = ScatterTmaSmem<V, TS, M, BPT>;
+    static_assert(SL::kTile == TILE, "both kernels use the same tiles");
     const uint32_t nt = static_cast<uint32_t>((n + TILE - 1) / TILE);
     const Tuning tun = tuning_for(sizeof(V) == 8 ? MDX_ELEM_REC8 : MDX_ELEM_U32, M, n);
+    auto scatter = plain_scatter_tma_kernel<V, D, M, TS, 1, OutFlat<V>, BPT>;
+    int blocks = 0, sms = 0;
+    if (occupancy(reinterpret_cast<const void*>(scatter), SL::bytes(1), &blocks, &sms, TS) != cudaSuccess)
+        return MDX_ERR_CUDA;
+    size_t smem = SL::bytes(1);
+    if constexpr (kBase) {
+        if (step == PlainStep::kBoth &&
+            nt <= kTwoSlotTiles * static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms)) {
+            scatter = plain_scatter_tma_kernel<V, D, M, TS, 2, OutFlat<V>, BPT>;
+            smem = SL::bytes(2);
+            if (occupancy(reinterpret_cast<const void*>(scatter), smem, &blocks, &sms, TS) != cudaSuccess)
+                return MDX_ERR_CUDA;
+        }
+    }
     if (tun.plain_ctas_per_sm > 0 && static_cast<int>(tun.plain_ctas_per_sm) < blocks)
         blocks = static_cast<int>(tun.plain_ctas_per_sm);
     uint32_t G = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
@@ -376,12 +383,12 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
         if (step == PlainStep::kBoth && dist == nullptr && ev_mid == nullptr && allow_fused &&
             tun.plain_two_kernel == 0) {
             // one cooperative kernel: count, grid barrier, scatter (mdx_fused.cuh)
-            using SL = ScatterTmaSmem<V, kThreads, kStages, M>;
+            using FL = ScatterTmaSmem<V, kThreads, M>;
             CUtensorMap map;
-            if (make_row_map(&map, d_in, n, sizeof(V), SL::kRows)) {
+            if (make_row_map(&map, d_in, n, sizeof(V), FL::kRows)) {
                 auto fused = plain_fused_kernel<V, D, M, kThreads, kStages>;
                 int fb = 0, fs = 0;
-                if (occupancy(reinterpret_cast<const void*>(fused), SL::kBytes, &fb, &fs) != cudaSuccess)
+                if (occupancy(reinterpret_cast<const void*>(fused), FL::bytes(kStages), &fb, &fs) != cudaSuccess)
                     return MDX_ERR_CUDA;
                 if (tun.plain_ctas_per_sm > 0 && static_cast<int>(tun.plain_ctas_per_sm) < fb)
                     fb = static_cast<int>(tun.plain_ctas_per_sm);
@@ -421,7 +428,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(FG);
                 cfg.blockDim = dim3(kThreads);
-                cfg.dynamicSmemBytes = SL::kBytes;
+                cfg.dynamicSmemBytes = FL::bytes(kStages);
                 cfg.stream = stream;
                 cudaLaunchAttribute attr[1];
                 attr[0].id = cudaLaunchAttributeCooperative;
@@ -444,14 +451,12 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     }
     if (step == PlainStep::kCount) return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
     {
-        using SL = ScatterTmaSmem<V, TS, kScatterStages, M, BPT>;
         CUtensorMap map;
         a.use_tma = make_row_map(&map, d_in, n, sizeof(V), SL::kRows) ? 1 : 0;
         if (dist == nullptr) {
             const OutFlat<V> o{static_cast<V*>(d_out),
                                static_cast<uint32_t>((reinterpret_cast<uintptr_t>(d_out) / sizeof(V)) &
                                                      (16u / sizeof(V) - 1u))};
-            auto scatter = plain_scatter_tma_kernel<V, D, M, TS, kScatterStages, OutFlat<V>, BPT>;
             if (step == PlainStep::kBoth && ev_mid == nullptr) {
                 // programmatic dependent launch: scheduled while the count grid
                 // drains, it starts its first tile copies before waiting for it
@@ -477,7 +482,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             // chunks of both steps must match)
             int b2 = 0, s2 = 0;
             if (occupancy(reinterpret_cast<const void*>(
-                              plain_scatter_tma_kernel<V, D, M, kThreads, kScatterStages, OutSharded<V>>),
+                              plain_scatter_tma_kernel<V, D, M, kThreads, 1, OutSharded<V>>),
                           smem, &b2, &s2) != cudaSuccess)
                 return MDX_ERR_CUDA;
             uint32_t* skip = reinterpret_cast<uint32_t*>(ws + kDistSkipOffset);
@@ -490,7 +495,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             for (uint32_t q = dist->R; q < static_cast<uint32_t>(kMaxRanks); q++) o.chunks[q] = nullptr;
             o.chunk = static_cast<uint32_t>(dist->chunk);
             o.R = dist->R;
-            plain_scatter_tma_kernel<V, D, M, kThreads, kScatterStages, OutSharded<V>>
+            plain_scatter_tma_kernel<V, D, M, kThreads, 1, OutSharded<V>>
                 <<<G, kThreads, smem, stream>>>(a, d, map, o);
         }
     }

@@ -46,7 +46,7 @@ namespace noalloc {
 
 constexpr size_t kNoAllocScratchBytes = 525312;  // 2052 * 256
 constexpr int kThreadsN = 256;
-constexpr int kStagesN = 1;
+constexpr int kSlotsN = 1;
 constexpr uint32_t kMaxChunksN = 4096;
 constexpr size_t kHeaderN = 256;
 constexpr int kMaxDevices = 64;
@@ -85,11 +85,7 @@ cudaError_t occupancy_n(const void* fn, size_t smem, int* blocks, int* sms) {
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(g_mu);
     if (s_blocks[dev] == 0) {
-        if (smem > 0) {
-            err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-            if (err != cudaSuccess) return err;
-        }
+        if ((err = raise_smem_limit(fn, smem)) != cudaSuccess) return err;
         int b = 0, s = 0;
         if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kThreadsN, smem)) !=
             cudaSuccess)
@@ -163,14 +159,14 @@ inline Layout layout_for(uint32_t M, uint32_t G) {
 template <class V, class D, int M>
 mdx_status run(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m, uint32_t* d_sizes,
                uint32_t* d_headflags, cudaStream_t st) {
-    using SL = ScatterTmaSmem<V, kThreadsN, kStagesN, M>;
+    using SL = ScatterTmaSmem<V, kThreadsN, M>;
     constexpr int TILE = SL::kTile;
-    auto scatter = plain_scatter_tma_kernel<V, D, M, kThreadsN, kStagesN>;
+    auto scatter = plain_scatter_tma_kernel<V, D, M, kThreadsN, kSlotsN>;
     auto count = plain_count_kernel<V, D, M, kThreadsN, TILE>;
     void* scratch = nullptr;
     if (scratch_address(&scratch) != cudaSuccess) return MDX_ERR_CUDA;
     int blocks = 0, sms = 0;
-    if (occupancy_n<KernelTag<V, D, M>>(reinterpret_cast<const void*>(scatter), SL::kBytes,
+    if (occupancy_n<KernelTag<V, D, M>>(reinterpret_cast<const void*>(scatter), SL::bytes(kSlotsN),
                                         &blocks, &sms) != cudaSuccess)
         return MDX_ERR_CUDA;
     const uint32_t nt = static_cast<uint32_t>((n + TILE - 1) / TILE);
@@ -210,7 +206,7 @@ mdx_status run(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m, uint3
                        static_cast<uint32_t>((reinterpret_cast<uintptr_t>(d_out) / sizeof(V)) &
                                              (16u / sizeof(V) - 1u))};
     count<<<G, kThreadsN, 0, st>>>(a, d);
-    scatter<<<G, kThreadsN, SL::kBytes, st>>>(a, d, map, o);
+    scatter<<<G, kThreadsN, SL::bytes(kSlotsN), st>>>(a, d, map, o);
     return cudaGetLastError() == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
 }
 

@@ -35,6 +35,7 @@
 
 #include <cuda.h>  // CUtensorMap (type only; maps are encoded by the host)
 
+#include <mutex>
 #include <type_traits>
 
 #include "mdx_device.cuh"
@@ -329,15 +330,29 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(Pl
     plain_finish_scan<M, THREADS>(a, tot_sh);
 }
 
-template <class V, int THREADS, int STAGES, int M, int BPT = 64>
+// Raise a kernel's dynamic shared-memory limit to `bytes` (host).  Never lowered: one
+// kernel is launched with one and with two slots, and by several entry points, so a
+// call that needs less must not take the limit from one that needs more.
+inline cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes at;
+    const cudaError_t err = cudaFuncGetAttributes(&at, fn);
+    if (err != cudaSuccess || at.maxDynamicSharedSizeBytes >= static_cast<int>(bytes)) return err;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
+template <class V, int THREADS, int M, int BPT = 64>
 struct ScatterTmaSmem {
     using G = TileGeom<V, THREADS, M, BPT>;
     static constexpr int kItems = G::kItems;
     static constexpr int kTile = G::kTile;
     static constexpr int kRows = G::kRows;
-    static constexpr size_t kRingBytes = static_cast<size_t>(STAGES) * kTile * sizeof(V);
+    static constexpr size_t kSlotBytes = static_cast<size_t>(kTile) * sizeof(V);
     // +1024: the ring is re-aligned to 1024 bytes (128-byte swizzle atoms)
-    static constexpr size_t kBytes = 1024 + kRingBytes + G::kStageBytes + G::kCntBytes;
+    static constexpr size_t bytes(uint32_t slots) {
+        return 1024 + slots * kSlotBytes + G::kStageBytes + G::kCntBytes;
+    }
 };
 
 // Where chunk k's class runs end in the output, from the [class][chunk] counts
@@ -402,7 +417,8 @@ __device__ __forceinline__ void scatter_cursors(const PlainArgs& a, uint32_t k, 
             }
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if constexpr (M > 2) {
+        // (a chunk of a few tiles up to 16 classes has nothing to gain from the look)
+        if (M > 16 || (M > 2 && a.num_tiles >= 4u * G)) {
             const uint32_t all = __reduce_add_sync(0xffffffffu, sum);
             const uint32_t top = __reduce_max_sync(0xffffffffu, max1);
             const uint32_t at = __ballot_sync(0xffffffffu, max1 == top);
@@ -416,7 +432,7 @@ __device__ __forceinline__ void scatter_cursors(const PlainArgs& a, uint32_t k, 
 // Scatter kernel: CTA k re-reads chunk k (tiles in reverse order) and writes
 // every element at class_base[c] + chunk_pre[c][k] + its rank in the chunk.
 // Tiles arrive by tensor TMA (one 2-D box of 128-byte rows per tile, 128-byte
-// swizzle, STAGES-deep mbarrier ring) and go through tile_filter (m = 2),
+// swizzle, an mbarrier ring of one or two slots) and go through tile_filter (m = 2),
 // tile_scatter (m <= 16) or tile_scatter_bytes (17..64 classes),
 // then a shared-memory stage at the destination's 16-byte phase and bulk
 // stores of every class run (mdx_tile.cuh).  OUT: one output array, or the
@@ -427,11 +443,12 @@ __device__ __forceinline__ void scatter_cursors(const PlainArgs& a, uint32_t k, 
 // is shared by twice the elements (N = 2^28 u32, m = 2, 4, 8, 16, 64: scatter
 // 346, 359, 367, 404, 707 us with 256 threads, 335, 343, 353, 391, 597 with 512;
 // a device copy of the same bytes takes 337).
-template <class V, class D, int M, int THREADS, int STAGES, class OUT = OutFlat<V>, int BPT = 64>
+// SLOTS: tiles in flight per CTA (1 or 2).
+template <class V, class D, int M, int THREADS, int SLOTS, class OUT = OutFlat<V>, int BPT = 64>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: <= 64 registers
     plain_scatter_tma_kernel(PlainArgs a, D d, const __grid_constant__ CUtensorMap tmap,
                              const __grid_constant__ OUT out) {
-    using L = ScatterTmaSmem<V, THREADS, STAGES, M, BPT>;
+    using L = ScatterTmaSmem<V, THREADS, M, BPT>;
     constexpr int ITEMS = L::kItems;
     constexpr int TILE = L::kTile;
     constexpr int ROWS = L::kRows;
@@ -441,10 +458,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     const uint32_t raw = smem_addr(smem_raw);
     unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     V* ring = reinterpret_cast<V*>(base);
-    V* stage = reinterpret_cast<V*>(base + L::kRingBytes);
-    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + L::kRingBytes + L::G::kStageBytes);
+    constexpr uint32_t wrap = SLOTS - 1;  // masks and shifts
+    static_assert(SLOTS == 1 || SLOTS == 2, "ring slots");
+    V* stage = reinterpret_cast<V*>(base + SLOTS * L::kSlotBytes);
+    uint32_t* cnt_sm = reinterpret_cast<uint32_t*>(base + SLOTS * L::kSlotBytes + L::G::kStageBytes);
 
-    __shared__ __align__(8) uint64_t bars[STAGES];
+    __shared__ __align__(8) uint64_t bars[SLOTS];
     __shared__ TileShared<M> sh;
     __shared__ uint32_t tot_sh[M], pre_sh[M];
     __shared__ int clustered_sh;  // two classes hold nearly all of this chunk
@@ -463,7 +482,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
 
     if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < STAGES; s++) mbar_init(&bars[s], 1);
+        for (int s = 0; s < SLOTS; s++) mbar_init(&bars[s], 1);
         mbar_fence_init();
         clustered_sh = 0;
     }
@@ -477,10 +496,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     // backwards, so the tiles the counting kernel read last are still in L2).
     auto issue = [&](uint32_t i) {
         const uint32_t tile = t1 - 1u - i;
-        uint64_t* bar = &bars[i % STAGES];
+        uint64_t* bar = &bars[i & wrap];
         if (tma_ok && static_cast<uint64_t>(tile + 1) * TILE <= a.n) {
             mbar_arrive_expect_tx(bar, TILE * sizeof(V));
-            tma_load_2d(ring + (i % STAGES) * TILE, &tmap, 0, static_cast<int32_t>(tile * ROWS), bar);
+            tma_load_2d(ring + (i & wrap) * TILE, &tmap, 0, static_cast<int32_t>(tile * ROWS), bar);
         } else {
             mbar_arrive(bar);
         }
@@ -488,7 +507,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
     // the first tiles only read the input: their copies start before the
     // count grid's results are needed
     if (tid == 0)
-        for (uint32_t i = 0; i < STAGES && i < cnt; i++) issue(i);
+        for (uint32_t i = 0; i < SLOTS && i < cnt; i++) issue(i);
     pdl_wait();
     const uint32_t stride = a.chunk_stride;
     if (a.prefix_in_scatter) {
@@ -507,15 +526,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
             const uint64_t ts = static_cast<uint64_t>(tile) * TILE;
             const uint32_t valid = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - ts));
             const bool full = valid == TILE;
-            const bool ok = mbar_wait_bounded(&bars[i % STAGES], (i / STAGES) & 1u);
+            const bool ok = mbar_wait_bounded(&bars[i & wrap], (i >> wrap) & 1u);
             V v[ITEMS];
             // the ring slot is consumed (values are in registers): refill it
             auto refill = [&] {
-                if (tid == 0 && i + STAGES < cnt) issue(i + STAGES);
+                if (tid == 0 && i + SLOTS < cnt) issue(i + SLOTS);
             };
             bool done;
             if (tma_ok && full) {
-                take_swizzled<V, ITEMS>(ring + (i % STAGES) * TILE, v);
+                take_swizzled<V, ITEMS>(ring + (i & wrap) * TILE, v);
             } else if (full) {
 #pragma unroll
                 for (int j = 0; j < ITEMS; j++) v[j] = in[ts + e0 + j];
@@ -536,8 +555,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
             if (!done) {
                 if (tid == 0) {
                     atomicOr(a.error, kErrTimeout);
-                    for (uint32_t q = i; q < cnt && q < i + STAGES; q++)
-                        (void)mbar_wait_bounded(&bars[q % STAGES], (q / STAGES) & 1u);
+                    for (uint32_t q = i; q < cnt && q < i + SLOTS; q++)
+                        (void)mbar_wait_bounded(&bars[q & wrap], (q >> wrap) & 1u);
                 }
                 break;
             }

@@ -186,6 +186,7 @@ mdx_status run(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m, uint3
     a.in = d_in;
     a.out = d_out;
     a.n = n;
+    a.shift = 0;
     a.num_tiles = nt;
     a.num_chunks = G;
     a.chunk_cnt = reinterpret_cast<uint32_t*>(ws + L.chunk_cnt);

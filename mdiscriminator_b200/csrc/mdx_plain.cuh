@@ -44,9 +44,11 @@
 namespace mdx {
 
 struct PlainArgs {
-    const void* in;
+    const void* in;       // at a 16-byte address when `shift` says how far the elements are off it
     void* out;
-    uint64_t n;
+    uint64_t n;           // elements from `in` on: the input's and the `shift` before them
+    uint32_t shift;       // positions before the first element (they lie in its 16-byte word and
+                          // are skipped); tiles are counted from `in`
     uint32_t num_tiles;   // ceil(n / TILE)
     uint32_t num_chunks;  // G: one chunk of consecutive tiles per CTA
     uint32_t* chunk_cnt;  // [M][G] class counts per chunk
@@ -233,13 +235,17 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(Pl
     const uint64_t e1 = min(static_cast<uint64_t>(t1) * TILE, a.n);
     const V* in = static_cast<const V*>(a.in);
     const bool vec_ok = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+    // the first chunk's first word when it holds positions before the input: its
+    // elements go with the tail's
+    const uint64_t skip = k == 0u && a.shift > 0u ? VEC : 0u;
 
     if constexpr (M <= 16) {
         PackedCounts<M> pc;
         pc.init();
         if (vec_ok) {
-            const uint4* vp = reinterpret_cast<const uint4*>(in + e0);
-            const uint64_t nv = (e1 - e0) / VEC;
+            const uint64_t s0 = min(e0 + skip, e1);
+            const uint4* vp = reinterpret_cast<const uint4*>(in + s0);
+            const uint64_t nv = (e1 - s0) / VEC;
             for (uint64_t i = tid; i < nv; i += static_cast<uint64_t>(THREADS) * UNROLL) {
                 uint4 r[UNROLL];
 #pragma unroll
@@ -260,13 +266,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(Pl
                 }
             }
             uint32_t k = 0;
-            for (uint64_t e = e0 + nv * VEC + tid; e < e1; e += THREADS) {
+            for (uint64_t e = s0 + nv * VEC + tid; e < e1; e += THREADS) {
                 pc.add(d(in[e]));
                 if (++k == 8u) {
                     pc.fold();
                     k = 0;
                 }
             }
+            pc.fold();
+            if (skip > 0u && tid >= a.shift && e0 + tid < s0) pc.add(d(in[e0 + tid]));
         } else {
             uint32_t k = 0;
             for (uint64_t e = e0 + tid; e < e1; e += THREADS) {
@@ -287,8 +295,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(Pl
         for (int c = lane; c < M; c += 32) red[warp][c] = 0;
         __syncwarp();
         if (vec_ok) {
-            const uint4* vp = reinterpret_cast<const uint4*>(in + e0);
-            const uint64_t nv = (e1 - e0) / VEC;
+            const uint64_t s0 = min(e0 + skip, e1);
+            const uint4* vp = reinterpret_cast<const uint4*>(in + s0);
+            const uint64_t nv = (e1 - s0) / VEC;
             for (uint64_t i = tid; i < nv; i += static_cast<uint64_t>(THREADS) * UNROLL) {
                 uint4 r[UNROLL];
 #pragma unroll
@@ -307,8 +316,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) plain_count_kernel(Pl
                     }
                 }
             }
-            for (uint64_t e = e0 + nv * VEC + tid; e < e1; e += THREADS)
+            for (uint64_t e = s0 + nv * VEC + tid; e < e1; e += THREADS)
                 atomicAdd(&red[warp][d(in[e])], 1u);
+            if (skip > 0u && tid >= a.shift && e0 + tid < s0) atomicAdd(&red[warp][d(in[e0 + tid])], 1u);
         } else {
             for (uint64_t e = e0 + tid; e < e1; e += THREADS) atomicAdd(&red[warp][d(in[e])], 1u);
         }
@@ -525,7 +535,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
             const uint32_t tile = t1 - 1u - i;
             const uint64_t ts = static_cast<uint64_t>(tile) * TILE;
             const uint32_t valid = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - ts));
-            const bool full = valid == TILE;
+            const uint32_t lo = tile == 0u ? a.shift : 0u;
+            const bool whole = valid == TILE, full = whole && lo == 0u;
             const bool ok = mbar_wait_bounded(&bars[i & wrap], (i >> wrap) & 1u);
             V v[ITEMS];
             // the ring slot is consumed (values are in registers): refill it
@@ -533,24 +544,24 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: 
                 if (tid == 0 && i + SLOTS < cnt) issue(i + SLOTS);
             };
             bool done;
-            if (tma_ok && full) {
+            if (tma_ok && whole) {
                 take_swizzled<V, ITEMS>(ring + (i & wrap) * TILE, v);
             } else if (full) {
 #pragma unroll
                 for (int j = 0; j < ITEMS; j++) v[j] = in[ts + e0 + j];
             } else {
 #pragma unroll
-                for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j < valid) ? in[ts + e0 + j] : V();
+                for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j >= lo && e0 + j < valid) ? in[ts + e0 + j] : V();
             }
             if constexpr (M == 2)
-                done = tile_filter<V, D, THREADS, false>(d, v, 0u, valid, full, stage, cnt_sm, sh, i & 1u,
+                done = tile_filter<V, D, THREADS, false>(d, v, lo, valid, full, stage, cnt_sm, sh, i & 1u,
                                                          out, ok, refill);
             else if constexpr (M > 16)
                 done = tile_scatter_bytes<V, D, M, THREADS, false, CLUSTERED>(
-                    d, v, 0u, valid, full, stage, reinterpret_cast<unsigned char*>(cnt_sm), sh, i & 1u,
+                    d, v, lo, valid, full, stage, reinterpret_cast<unsigned char*>(cnt_sm), sh, i & 1u,
                     out, ok, refill);
             else
-                done = tile_scatter<V, D, M, THREADS, false, CLUSTERED>(d, v, 0u, valid, full, stage, cnt_sm, sh,
+                done = tile_scatter<V, D, M, THREADS, false, CLUSTERED>(d, v, lo, valid, full, stage, cnt_sm, sh,
                                                              i & 1u, out, ok, refill);
             if (!done) {
                 if (tid == 0) {

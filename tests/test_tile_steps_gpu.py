@@ -119,3 +119,27 @@ def test_a_few_tiles_in_one_launch(cuda_ready, m, rec):
                 assert not out[:off_out].any() and not out[off_out + n:].any()
         host, host_sizes = mdx.mdiscr(base[:n].clone(), ("mod", m))
         assert sum(host_sizes) == n
+
+
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("m", [2, 7, 16, 40])
+def test_inputs_off_a_16_byte_address(cuda_ready, m, rec):
+    """An input that begins inside a 16-byte word is read from that word's address:
+    every position in it, at and around whole tiles counted from there."""
+    torch = cuda_ready
+    tile = 2048 if rec else 4096
+    kind = np.int64 if rec else np.int32
+    for off in (1,) if rec else (1, 2, 3):
+        for n in (8 * tile + 1, 9 * tile - off, 9 * tile - off + 1, 9 * tile, 20 * tile - 1, 700_001):
+            x = clustered(n, m, "two" if off == 2 else "runs", m + n)
+            if rec:
+                x = x.astype(np.uint64) | (np.arange(n, dtype=np.uint64) << np.uint64(32))
+            eo, es, ef = oracle.partition(x, m, headflags=True)
+            base = torch.full((n + 8,), -1, dtype=torch.int64 if rec else torch.int32, device="cuda")
+            base[off:off + n] = torch.from_numpy(x.view(kind)).cuda()
+            out, sizes, hf = mdx.partition(base[off:off + n], ("mod", m), headflags=True)
+            torch.cuda.synchronize()
+            assert mdx.workspace(0).error() == mdx.MDX_OK
+            assert np.array_equal(sizes.cpu().numpy(), es), (n, off)
+            assert np.array_equal(out.cpu().numpy().view(x.dtype), eo), (n, off)
+            assert np.array_equal(hf.cpu().numpy().view(np.uint32), ef), (n, off)

@@ -14,7 +14,7 @@
 //                   block totals, records the counts and resets the tickets.
 //   seg_plan_emit   writes the run entries {segment, [p0, p1), last run of
 //                   the segment} and the group heads, in element order.
-//   seg_main        persistent; CTAs take tickets for batches of groups.  Each
+//   seg_main        persistent; CTAs take tickets for batches of groups.  A
 //                   group's range is read into shared memory by one bulk copy and
 //                   partitioned by the whole CTA (seg_group_cta: every thread owns
 //                   consecutive elements whatever the segment lengths; one scan of
@@ -555,11 +555,11 @@ __device__ __forceinline__ D group_discr(const SegArgs& a, const D& d, const uin
 // flags and no thread closes a segment for the others.  6 * 10^7 u32 in segments
 // of up to 4096 (mean 1600), m = 4: 46 instructions an element and 167 us, where a
 // segmented scan with the segments closed by the threads that hold their ends took
-// 78 and 212; 10^5 LogNormal(ln 1024, 1.5) segments, m = 2, 4, 8, 16: 363, 368,
-// 457, 745 -> 294, 306, 361, 689 us.  What bounds it now is latency: four barriers
-// a group and 24 warps to an SM (shared memory).  Windows of P / 2 and 3 P / 4, the
-// former with four CTAs: 309 and 336 against 306 us at m = 4, 448 and 398 against
-// 361 at m = 8.  The run counts as items of this kernel, to fill the idle memory
+// 78 and 212; 10^5 LogNormal(ln 1024, 1.5) segments, m = 4, 8, 16: 368, 457, 745 ->
+// 306, 361, 689 us, with the groups' ranges fetched ahead (GroupRange) 289, 349, 633.  What bounds it now is latency: four barriers
+// a group and 24 warps to an SM (shared memory).  Windows of P / 2 with
+// four CTAs: 299 against 289 us at m = 4, 439 against 349 at m = 8, 663 against 633
+// at m = 16; windows of 3 P / 4 were slower too.  The run counts as items of this kernel, to fill the idle memory
 // pipe: 545 us for both against 306 + 157.
 template <class V, class D, int M, int THREADS>
 __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, const uint32_t* cmod,
@@ -793,13 +793,28 @@ __global__ void __launch_bounds__(THREADS, 4) seg_run_count(SegArgs a, D d) {
     }
 }
 
-// Persistent; CTAs take tickets for batches of small-segment groups.
+// A CTA's groups in their pipeline: a group's ticket is drawn four groups ahead, its
+// entry loaded three, its range loaded two and published one group ahead, all by one
+// thread of the last warp, so that no group waits for that chain.  Loaded at a
+// batch's start, the chain and its two barriers were 306 against 289 us on 10^5
+// LogNormal(ln 1024, 1.5) segments (u32, m = 4, batches of two groups; in batches of
+// sixteen, which hid it before, 314: their last ones leave CTAs idle).  Without
+// tickets, the groups dealt out in turns: 307.
+struct GroupRange {
+    uint32_t h, he;   // segments [h, he)
+    uint32_t r0, r1;  // elements [r0, r1) (n < 2^32)
+    uint32_t valid;   // false: the CTA has had its last group
+};
+
+// Persistent; CTA b begins with batch b of the small-segment groups and takes tickets
+// for the batches after its first.
 template <class V, class D, int M, int THREADS>
 __global__ void __launch_bounds__(THREADS, 3)
     seg_main(SegArgs a, D d) {
     using L = SegSmem<V, M, THREADS>;
     constexpr uint32_t AU = L::kAU;
     constexpr uint32_t P = L::kTile;
+    constexpr int kPlanner = THREADS - 1;  // the thread that knows the groups to come
     static_assert(M <= 16 && M >= 2, "class bound");
     static_assert(static_cast<int>(kGroupSegs) <= THREADS, "one thread per segment");
 
@@ -811,9 +826,7 @@ __global__ void __launch_bounds__(THREADS, 3)
     GroupScratch<M, THREADS>& gs = *reinterpret_cast<GroupScratch<M, THREADS>*>(g_out + L::kGroupElems);
 
     __shared__ __align__(8) uint64_t gbar;
-    __shared__ uint32_t ticket_sh[2];
-    __shared__ uint32_t gb_h[kMaxGroupBatch], gb_he[kMaxGroupBatch];  // the batch's groups
-    __shared__ uint32_t gb_r0[kMaxGroupBatch], gb_r1[kMaxGroupBatch];
+    __shared__ GroupRange range_sh[2];  // of this group and of the next, in turns
     __shared__ uint32_t cmod[17];  // DiscrMod constants for m = 1 .. 16
 
     const int tid = threadIdx.x;
@@ -825,12 +838,64 @@ __global__ void __launch_bounds__(THREADS, 3)
     pdl_wait();
     const uint64_t S = seg_count(a);
     const uint32_t num_groups = a.hdr->num_groups;
-    // groups per ticket: the tuned batch, but no more than spreads the groups
-    // over every CTA (a few groups must not queue up on one CTA)
+    // neighbouring groups per ticket: the tuned batch, but no more than spreads the
+    // groups over every CTA (a few groups must not queue up on one CTA)
     const uint32_t batch =
         max(1u, min(a.group_batch, (num_groups + gridDim.x - 1) / gridDim.x));
-    const uint32_t num_batches = (num_groups + batch - 1) / batch;
     uint32_t uses = 0;  // of the input buffer
+
+    // kPlanner's state: the group to load an entry of, `left` more of its batch, the
+    // ticket after it; the entry; and of the group before that segments and elements
+    uint32_t g = blockIdx.x * batch, left = batch - 1u, ticket = 0;
+    uint32_t eh = 0, ee = 0, wh = 0, we = 0;
+    bool ev = false, wv = false;
+    uint64_t w0 = 0, w1 = 0;
+    auto draw = [&] { ticket = gridDim.x + atomicAdd(&a.hdr->ticket, 1u); };
+    auto load_entry = [&] {  // of group g, then the next group
+        ev = g < num_groups;
+        if (!ev) return;
+        eh = a.groups[g];
+        ee = a.groups_end[g];
+        g++;
+        if (left-- == 0u) {
+            g = ticket * batch;
+            left = batch - 1u;
+            draw();
+        }
+    };
+    auto load_range = [&] {  // of the entry
+        wv = ev;
+        if (!ev) return;
+        wh = eh;
+        we = static_cast<uint32_t>(min(static_cast<uint64_t>(ee), S));
+        we = min(max(we, wh), wh + kGroupSegs);
+        w0 = a.offsets[wh];
+        w1 = a.offsets[we];
+    };
+    auto publish = [&](uint32_t q) {
+        const bool bad = w1 < w0 || w1 - w0 >= 2u * P || w1 > a.n;  // malformed: nothing to do
+        range_sh[q].h = wh;
+        range_sh[q].he = bad ? wh : we;
+        range_sh[q].r0 = bad ? 0u : static_cast<uint32_t>(w0);
+        range_sh[q].r1 = bad ? 0u : static_cast<uint32_t>(w1);
+        range_sh[q].valid = wv;
+    };
+    // the 16-byte words of a group that one bulk copy brings
+    auto vec_end = [&](uint32_t r1, uint64_t as) {
+        const uint64_t ve = min((static_cast<uint64_t>(r1) + AU - 1u) & ~static_cast<uint64_t>(AU - 1u),
+                                a.n & ~static_cast<uint64_t>(AU - 1u));
+        return in_vec && ve > as ? ve : as;
+    };
+    auto issue_group = [&](uint32_t q) {  // thread 0 only
+        const uint64_t as = range_sh[q].r0 & ~(AU - 1u);
+        const uint32_t bytes = static_cast<uint32_t>((vec_end(range_sh[q].r1, as) - as) * sizeof(V));
+        if (bytes > 0) {
+            mbar_arrive_expect_tx(&gbar, bytes);
+            bulk_load_g2s(g_in, in + as, bytes, &gbar);
+        } else {
+            mbar_arrive(&gbar);
+        }
+    };
 
     if (tid == 0) {
         mbar_init(&gbar, 1);
@@ -838,121 +903,99 @@ __global__ void __launch_bounds__(THREADS, 3)
     }
     if (tid >= 1 && tid <= 16) cmod[tid] = DiscrMod::make(static_cast<uint32_t>(tid)).c;
     if (tid == 0) cmod[0] = 0;
+    if (g >= num_groups) return;
+    if (tid == kPlanner) {
+        draw();
+        load_entry();
+        load_range();
+        load_entry();
+        publish(0);
+        load_range();
+        load_entry();
+    }
     __syncthreads();
+    if (tid == 0) issue_group(0);
 
-    for (uint32_t it = 0;; it++) {
-        if (tid == 0) ticket_sh[it & 1u] = atomicAdd(&a.hdr->ticket, 1u);
-        __syncthreads();
-        const uint32_t t = ticket_sh[it & 1u];
-        if (t >= num_batches) break;
-        // group i of the batch: segments [h, he), elements [r0, r1); its range is
-        // fetched by one bulk copy while the previous group is written
-        const uint32_t g0 = t * batch;
-        const uint32_t gcnt = min(batch, num_groups - g0);
-        if (tid < static_cast<int>(gcnt)) {
-            const uint32_t h = a.groups[g0 + tid];
-            uint32_t he = static_cast<uint32_t>(min(static_cast<uint64_t>(a.groups_end[g0 + tid]), S));
-            he = min(max(he, h), h + kGroupSegs);
-            uint64_t r0 = a.offsets[h], r1 = a.offsets[he];
-            if (r1 < r0 || r1 - r0 >= 2u * P || r1 > a.n) {  // malformed: nothing to do
-                he = h;
-                r0 = r1 = 0u;
-            }
-            gb_h[tid] = h;
-            gb_he[tid] = he;
-            gb_r0[tid] = static_cast<uint32_t>(r0);  // n < 2^32
-            gb_r1[tid] = static_cast<uint32_t>(r1);
+    GroupPrefetch pf;
+    pf.valid = false;
+    for (uint32_t q = 0; range_sh[q].valid; q ^= 1u) {
+        const uint32_t h = range_sh[q].h, nseg = range_sh[q].he - h;
+        const uint32_t r0 = range_sh[q].r0, r1 = range_sh[q].r1;
+        if (tid == kPlanner) {
+            publish(q ^ 1u);
+            load_range();
+            load_entry();
         }
-        __syncthreads();
-        // the 16-byte words of group i that one bulk copy brings
-        auto vec_end = [&](uint32_t i, uint64_t as) {
-            const uint64_t ve =
-                min((static_cast<uint64_t>(gb_r1[i]) + AU - 1u) & ~static_cast<uint64_t>(AU - 1u),
-                    a.n & ~static_cast<uint64_t>(AU - 1u));
-            return in_vec && ve > as ? ve : as;
-        };
-        auto issue_group = [&](uint32_t i) {  // thread 0 only
-            const uint64_t as = gb_r0[i] & ~(AU - 1u);
-            const uint32_t bytes = static_cast<uint32_t>((vec_end(i, as) - as) * sizeof(V));
-            if (bytes > 0) {
-                mbar_arrive_expect_tx(&gbar, bytes);
-                bulk_load_g2s(g_in, in + as, bytes, &gbar);
-            } else {
-                mbar_arrive(&gbar);
+        const uint64_t as = r0 & ~static_cast<uint64_t>(AU - 1u);
+        const uint32_t phase = static_cast<uint32_t>(r0 - as);
+        const uint32_t end = static_cast<uint32_t>(r1 - as);
+        // ---- heads, while the group's elements are on their way
+        bool bad = false;
+        if (static_cast<uint32_t>(tid) < nseg) {
+            if (!pf.valid) {
+                pf.o0 = a.offsets[h + tid];
+                pf.o1 = a.offsets[h + tid + 1];
+                pf.m = a.seg_m != nullptr ? min(max(a.seg_m[h + tid], 1u), a.m_bound) : a.m;
             }
-        };
-        if (tid == 0) issue_group(0);
-        bool failed = false;
-        GroupPrefetch pf;
-        pf.valid = false;
-        for (uint32_t i = 0; i < gcnt; i++) {
-            const uint32_t h = gb_h[i], nseg = gb_he[i] - h;
-            const uint32_t r0 = gb_r0[i], r1 = gb_r1[i];
-            const uint64_t as = r0 & ~static_cast<uint64_t>(AU - 1u);
-            const uint32_t phase = static_cast<uint32_t>(r0 - as);
-            const uint32_t end = static_cast<uint32_t>(r1 - as);
-            // ---- heads, while the group's elements are on their way
-            bool bad = false;
-            if (static_cast<uint32_t>(tid) < nseg) {
-                if (!pf.valid) {
-                    pf.o0 = a.offsets[h + tid];
-                    pf.o1 = a.offsets[h + tid + 1];
-                    pf.m = a.seg_m != nullptr ? min(max(a.seg_m[h + tid], 1u), a.m_bound) : a.m;
-                }
-                bad = pf.o0 < r0 || pf.o1 < pf.o0 || pf.o1 > r1;
-                gs.hpos[tid] = static_cast<uint16_t>(pf.o0 - as);
-                gs.msz[tid] = static_cast<uint8_t>(pf.m);
-            }
-            if (tid == 0) gs.hpos[nseg] = static_cast<uint16_t>(end);
-            const bool ok = mbar_wait_bounded(&gbar, uses & 1u);
-            const uint64_t ve = vec_end(i, as);
-            if (ve < r1) {  // what the bulk copy did not bring (CTA-uniform)
-                for (uint64_t e = max(ve, static_cast<uint64_t>(r0)) + tid; e < r1; e += THREADS)
-                    g_in[e - as] = in[e];
-            }
-            if (__syncthreads_or(bad || !ok)) {  // a malformed group is left alone
+            bad = pf.o0 < r0 || pf.o1 < pf.o0 || pf.o1 > r1;
+            gs.hpos[tid] = static_cast<uint16_t>(pf.o0 - as);
+            gs.msz[tid] = static_cast<uint8_t>(pf.m);
+        }
+        if (tid == 0) gs.hpos[nseg] = static_cast<uint16_t>(end);
+        const bool ok = mbar_wait_bounded(&gbar, uses & 1u);
+        const uint64_t ve = vec_end(r1, as);
+        if (ve < r1) {  // what the bulk copy did not bring (CTA-uniform)
+            for (uint64_t e = max(ve, static_cast<uint64_t>(r0)) + tid; e < r1; e += THREADS)
+                g_in[e - as] = in[e];
+        }
+        if (__syncthreads_or(bad || !ok)) {  // a malformed group is left alone
+            fence_proxy_async_smem();
+            if (__syncthreads_or(!ok)) {
                 if (tid == 0) {  // only this group's copy can be in flight
                     const bool late = mbar_wait_bounded(&gbar, uses & 1u);
                     if (!late) atomicOr(&a.hdr->error, kErrTimeout);
                 }
-                failed = true;
                 break;
             }
             uses++;
-            pf.valid = i + 1 < gcnt;
-            if (pf.valid && static_cast<uint32_t>(tid) < gb_he[i + 1] - gb_h[i + 1]) {
-                const uint64_t ns = static_cast<uint64_t>(gb_h[i + 1]) + tid;
-                pf.o0 = a.offsets[ns];
-                pf.o1 = a.offsets[ns + 1];
-                pf.m = a.seg_m != nullptr ? min(max(a.seg_m[ns], 1u), a.m_bound) : a.m;
-            }
-            const uint32_t nq = ((end + THREADS * AU - 1u) / (THREADS * AU)) | 1u;
-            uint32_t qn = 0;  // heads before the thread's first position
-            if (nseg > 0u) {
-                const uint32_t lo = static_cast<uint32_t>(tid) * nq * AU;
-                for (uint32_t step = 1u << (31 - __clz(nseg)); step > 0u; step >>= 1)
-                    if (qn + step <= nseg && gs.hpos[qn + step - 1u] < lo) qn += step;
-            }
-            seg_group_cta<V, D, M, THREADS>(a, d, cmod, h, nseg, as, phase, end, g_in, g_out, gs, qn, nq);
-            // every access of the buffers precedes the copies of them
-            fence_proxy_async_smem();
-            __syncthreads();
-            if (tid == 0 && i + 1 < gcnt) issue_group(i + 1);
-            // write the range back from the output image
-            const uint32_t vs = min((phase + AU - 1u) & ~(AU - 1u), end), vt = max(vs, end & ~(AU - 1u));
-            if (out_vec) {
-                if (tid == 0 && vt > vs) {
-                    bulk_store_s2g(out + as + vs, g_out + vs, (vt - vs) * sizeof(V));
-                    bulk_commit();
-                }
-                if (static_cast<uint32_t>(tid) < vs - phase) out[r0 + tid] = g_out[phase + tid];
-                if (static_cast<uint32_t>(tid) < end - vt) out[as + vt + tid] = g_out[vt + tid];
-            } else {
-                for (uint32_t y = phase + tid; y < end; y += THREADS) out[as + y] = g_out[y];
-                __syncthreads();
-            }
+            pf.valid = false;
+            if (tid == 0 && range_sh[q ^ 1u].valid) issue_group(q ^ 1u);
+            continue;
         }
-        if (failed) break;
+        uses++;
+        const bool more = range_sh[q ^ 1u].valid;
+        pf.valid = more;
+        if (more && static_cast<uint32_t>(tid) < range_sh[q ^ 1u].he - range_sh[q ^ 1u].h) {
+            const uint64_t ns = static_cast<uint64_t>(range_sh[q ^ 1u].h) + tid;
+            pf.o0 = a.offsets[ns];
+            pf.o1 = a.offsets[ns + 1];
+            pf.m = a.seg_m != nullptr ? min(max(a.seg_m[ns], 1u), a.m_bound) : a.m;
+        }
+        const uint32_t nq = ((end + THREADS * AU - 1u) / (THREADS * AU)) | 1u;
+        uint32_t qn = 0;  // heads before the thread's first position
+        if (nseg > 0u) {
+            const uint32_t lo = static_cast<uint32_t>(tid) * nq * AU;
+            for (uint32_t step = 1u << (31 - __clz(nseg)); step > 0u; step >>= 1)
+                if (qn + step <= nseg && gs.hpos[qn + step - 1u] < lo) qn += step;
+        }
+        seg_group_cta<V, D, M, THREADS>(a, d, cmod, h, nseg, as, phase, end, g_in, g_out, gs, qn, nq);
+        // every access of the buffers precedes the copies of them
+        fence_proxy_async_smem();
+        __syncthreads();
+        if (tid == 0 && more) issue_group(q ^ 1u);
+        // write the range back from the output image
+        const uint32_t vs = min((phase + AU - 1u) & ~(AU - 1u), end), vt = max(vs, end & ~(AU - 1u));
+        if (out_vec) {
+            if (tid == 0 && vt > vs) {
+                bulk_store_s2g(out + as + vs, g_out + vs, (vt - vs) * sizeof(V));
+                bulk_commit();
+            }
+            if (static_cast<uint32_t>(tid) < vs - phase) out[r0 + tid] = g_out[phase + tid];
+            if (static_cast<uint32_t>(tid) < end - vt) out[as + vt + tid] = g_out[vt + tid];
+        } else {
+            for (uint32_t y = phase + tid; y < end; y += THREADS) out[as + y] = g_out[y];
+            __syncthreads();
+        }
     }
     if (tid == 0) bulk_wait_all();
 }

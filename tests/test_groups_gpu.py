@@ -72,3 +72,28 @@ def test_class_count_per_segment(cuda_ready):
         cls = x[a:b] % seg_m[s]
         assert np.array_equal(got[a:b], x[a:b][np.argsort(cls, kind="stable")]), s
         assert np.array_equal(gs[s], np.bincount(cls, minlength=16)), s
+
+
+@pytest.mark.parametrize("batch", [1, 3, 32])
+@pytest.mark.parametrize("groups", [1, 2, 443, 2300])
+def test_groups_a_cta(cuda_ready, batch, groups):
+    """From one group in all to several tickets a CTA, with batches that end before
+    and at the last group."""
+    torch = cuda_ready
+    rng = np.random.default_rng(groups + batch)
+    offs = np.concatenate([[0], np.cumsum(rng.integers(1500, 4097, 2 * groups))]).astype(np.uint64)
+    n = int(offs[-1])
+    x = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    eo, es, ef = oracle.partition_segmented(x, offs, 5, headflags=True)
+    try:
+        mdx.set_tuning(mdx.ELEM_U32, 8, 0, 33, run_tiles=4, group_batch=batch)
+        o, sizes, hf = mdx.partition_segmented(torch.from_numpy(x.view(np.int32)).cuda(),
+                                               torch.from_numpy(offs.view(np.int64)).cuda(), ("mod", 5),
+                                               headflags=True)
+        torch.cuda.synchronize()
+    finally:
+        mdx.load_tuning(mdx.TUNING_PATH, missing_ok=True)
+    assert mdx.workspace(0).error() == mdx.MDX_OK
+    assert np.array_equal(sizes.cpu().numpy(), es)
+    assert np.array_equal(o.cpu().numpy().view(np.uint32), eo)
+    assert np.array_equal(hf.cpu().numpy(), ef)

@@ -238,10 +238,11 @@ mdx_status mdx_partition_noalloc_error(mdx_stream_t stream);
  * together (cuda_code/MdiscrHost_tuples.cu.h:262-429 partitions a u32, a u8 and
  * a bool array by a functor of the first): column 0 is the u32 key the class
  * comes from, the others (1, 2, 4 or 8 bytes per row, up to 8 columns in all)
- * follow its rows.  Both build {key, row} 8-byte records, partition them with
- * the 8-byte-record kernels and gather the rows (4- and 8-byte records take the
- * direct paths); workspaces from the two size functions (they hold the record
- * arrays: about 16 bytes per row).  Outputs must not overlap any input.
+ * follow its rows.  Rows are moved whole through shared memory (4- and 8-byte
+ * records take the direct paths; records above 1024 bytes are partitioned as
+ * {key, row} 8-byte records and gathered); workspaces from the two size functions
+ * (they have room for the record arrays: about 16 bytes per row).  Outputs must not
+ * overlap any input.
  */
 size_t mdx_records_workspace_size(uint64_t n, uint32_t record_bytes, uint32_t m);
 mdx_status mdx_partition_records(const void* d_in, void* d_out, uint64_t n, uint32_t record_bytes,
@@ -388,7 +389,7 @@ typedef struct {
                                     scatter as two kernels; 4- and 8-byte elements) */
     uint32_t tile_threads;       /* plain path: threads of a scatter CTA, 256 (default, 0) or 512
                                     (64-byte tiles twice as long, half the per-tile steps; count +
-                                    scatter as two kernels; 4- and 8-byte elements, m <= 16;
+                                    scatter as two kernels; 4- and 8-byte elements;
                                     takes precedence over tile_bytes) */
 } mdx_tuning;
 

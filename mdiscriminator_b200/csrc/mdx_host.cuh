@@ -303,8 +303,13 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     // Element loads, which such inputs had before, kept one 4-byte request in flight where
     // a vector load has 16 bytes: 2^27 u32 at 4 bytes off, 8 / 13 / 64 classes 539 / 807 /
     // 680 us, now 293 / 330 / 425, as aligned ones; 2^26 records 8 bytes off, 8 / 16
-    // classes 492 / 497, now 283 / 288.
-    const uint32_t shift = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(d_in) % 16 / sizeof(V));
+    // classes 492 / 497, now 283 / 288.  Not the two steps of a sharded call: tiles
+    // would be counted from that address, and a scatter may be given the counted
+    // elements in a buffer of another alignment, so their chunks start at the elements.
+    const uint32_t shift =
+        step == PlainStep::kBoth
+            ? static_cast<uint32_t>(reinterpret_cast<uintptr_t>(d_in) % 16 / sizeof(V))
+            : 0u;
     const void* const base_in = static_cast<const V*>(d_in) - shift;
     const uint32_t tiles_n = static_cast<uint32_t>((n + TILE - 1) / TILE);
     const uint32_t nt = static_cast<uint32_t>((n + shift + TILE - 1) / TILE);

@@ -178,6 +178,15 @@ __device__ __forceinline__ uint64_t seg_count(const SegArgs& a) {
     return a.num_segs == kSegsOnDevice ? a.hdr->num_segs : a.num_segs;
 }
 
+// Whether segment s of S, [a0, a1), can be one of the segments that tile [0, n).  Both
+// planning kernels leave the others alone, by this one test: entries of a segment that
+// was given no room would take another's, and runs of two segments mixed under one
+// can reach past its end.
+__device__ __forceinline__ bool seg_in_place(const SegArgs& a, uint64_t s, uint64_t S, uint64_t a0,
+                                             uint64_t a1) {
+    return a0 <= a1 && a1 <= a.n && (s != 0 || a0 == 0) && (s + 1 != S || a1 == a.n);
+}
+
 // --------------------------------------------------------------- planning --
 // Block b of the planner owns segments [b*R, min((b+1)*R, S)), R = ceil(S/G).
 template <int P, int THREADS>
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
         uint32_t runs = 0, head = 0, mid = 0;
         if (s < s1) {
             const uint64_t a0 = a.offsets[s], a1 = a.offsets[s + 1];
-            if (a1 < a0 || a1 > a.n || (s == 0 && a0 != 0) || (s + 1 == S && a1 != a.n)) {
+            if (!seg_in_place(a, s, S, a0, a1)) {
                 atomicOr(&a.hdr->error, kErrSegments);
             } else if (a1 - a0 > static_cast<uint64_t>(P)) {
                 if (is_mid<P>(a, a0, a1)) {
@@ -340,7 +349,8 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
         const uint64_t s = base + tid;
         if (s < s1) {
             const uint64_t a0 = a.offsets[s], a1 = a.offsets[s + 1];
-            if (a1 >= a0 && a1 <= a.n) {
+            const bool in_place = seg_in_place(a, s, S, a0, a1);
+            if (in_place) {
                 if (a1 - a0 > static_cast<uint64_t>(P) && is_mid<P>(a, a0, a1)) {
                     const uint32_t pos = moff + a.mid_loc[s];
                     if (pos < num_mids) a.mids[pos] = static_cast<uint32_t>(s);
@@ -369,7 +379,7 @@ __global__ void __launch_bounds__(THREADS) seg_plan_emit(SegArgs a) {
             }
             // the group before segment s ends at s at the latest when s starts
             // a group, is large or is malformed
-            const bool small_ok = (a1 >= a0 && a1 <= a.n && a1 - a0 <= static_cast<uint64_t>(P));
+            const bool small_ok = in_place && a1 - a0 <= static_cast<uint64_t>(P);
             const bool is_head = small_ok && group_head<P>(a, s, a0);
             const uint32_t before = goff + a.grp_loc[s];  // groups starting before s
             if ((is_head || !small_ok) && before >= 1u && before - 1u < num_groups)

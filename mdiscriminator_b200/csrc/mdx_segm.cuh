@@ -250,7 +250,9 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
             a.grp_loc[s] = carry_g + pg + ig - head;
             a.mid_loc[s] = carry_m + pm + im - mid;
         }
-        carry_r += tr;
+        // segments that overlap can have more runs than 32 bits count: one more than
+        // there is room for says as much (groups and medium segments are at most S)
+        carry_r = min(carry_r + tr, a.max_runs + 1u);
         carry_g += tg;
         carry_m += tm;
         __syncthreads();
@@ -290,7 +292,8 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        uint32_t before = 0, all = 0;
+        uint32_t before = 0;
+        uint64_t all = 0;
 #pragma unroll
         for (int w = 0; w < W; w++) {
             before += w < warp ? wsum[q][w] : 0u;
@@ -302,7 +305,8 @@ __global__ void __launch_bounds__(THREADS) seg_plan_spans(SegArgs a) {
             if (4u * tid + u < gridDim.x) arrs[q][4u * tid + u] = run;
             run += x[q][u];
         }
-        if (tid == 0) *counts[q] = all <= bounds[q] ? all : 0u;  // over capacity: malformed
+        if (tid == 0)  // over capacity: malformed
+            *counts[q] = all <= bounds[q] ? static_cast<uint32_t>(all) : 0u;
     }
     __syncthreads();
     if (tid == 0) {

@@ -86,3 +86,20 @@ def test_head_flags_without_a_first_one(cuda_ready):
     got, status = run(torch, x, lambda d, o: mdx.mdiscr_segm(d, df, ("mod", M), d_out=o), False)
     assert status == mdx.MDX_ERR_SEGMENTS
     check(got, x, offs, {1})
+
+
+def test_more_runs_than_32_bits_count(cuda_ready):
+    """Segments that all cover the whole input, 2^20 + 1 of 2^12 runs each: their sum,
+    taken modulo 2^32, would fit the run table."""
+    torch = cuda_ready
+    n = 1 << 24
+    offs = torch.zeros(2 * ((1 << 20) + 1), dtype=torch.int64, device="cuda")
+    offs[1::2] = n
+    x = values(n, False)
+    try:
+        mdx.set_tuning(mdx.ELEM_U32, M, 0, 33, plain_two_kernel=1, run_tiles=1)
+        got, status = run(torch, x, lambda d, o: mdx.partition_segmented(d, offs, ("mod", M), out=o), False)
+    finally:
+        mdx.load_tuning(mdx.TUNING_PATH, missing_ok=True)
+    assert status == mdx.MDX_ERR_SEGMENTS
+    assert (got == -1).all()

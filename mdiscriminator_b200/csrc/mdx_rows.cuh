@@ -38,7 +38,8 @@ struct RowsColumn {
     uint32_t bytes;   // of a row
     uint32_t unit;    // 1, 2, 4, 8 or 16: bytes moved at a time
     uint32_t offset;  // of the column's tile in a tile buffer
-    uint32_t bulk;    // a whole tile comes by one bulk copy (16-byte aligned)
+    uint32_t lead;    // bytes of the column's first 16-byte word before its first row
+    uint32_t copied;  // bytes of the 16-byte words that hold a whole tile
 };
 
 struct RowsArgs {
@@ -49,7 +50,8 @@ struct RowsArgs {
     uint32_t buf_bytes;   // of a tile buffer
     uint32_t key_offset;  // of the key column's tile in a tile buffer
     uint32_t num_cols;
-    uint32_t all_bulk;    // every column is `bulk`
+    uint32_t bulk_tiles;  // whole tiles that come by bulk copies: all of them, but the last
+                          // when a column has a lead (its copy would pass the column's end)
     uint32_t end[4];      // columns (not a record): end[q] of 8 >> q bytes or more, the wider first
     RowsColumn col[kMaxCols];
 };
@@ -160,7 +162,7 @@ __device__ __forceinline__ void write_records(const RowsColumn& col, const unsig
                                               const uint32_t* stage, const TileShared<M>& sh,
                                               uint32_t rows, const RowShare& share) {
     const uint32_t bytes = col.bytes, at = share.word * static_cast<uint32_t>(sizeof(T));
-    const unsigned char* src = tile + at;
+    const unsigned char* src = tile + col.offset + at;
     unsigned char* out = col.out + at;
 #pragma unroll 4
     for (uint32_t s = share.first; s < rows; s += share.step) {
@@ -260,28 +262,34 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     }
     __syncthreads();
 
-    // i-th tile in processing order is tile t1-1-i
+    // i-th tile in processing order is tile t1-1-i.  A tile's rows come by one bulk copy
+    // per column, of the 16-byte words that hold them: a column off a 16-byte address
+    // lies `lead` bytes into its room.  Element loads with a barrier after them, which
+    // took the place of the copies there: 5 * 10^8 bytes at 4 bytes off, a call, rows of
+    // 20 bytes m = 8 412 us, now 284 (aligned 280), of 256 bytes m = 64 673 and 358
+    // (279: its rows move by 4 bytes, not 16); 2 * 10^7 rows of a key and seven columns of
+    // 8 bytes, m = 2, 1093 and 451 (446).
     auto rows_of = [&](uint32_t tile) {
         return static_cast<uint32_t>(
             min(static_cast<uint64_t>(T), a.p.n - static_cast<uint64_t>(tile) * T));
     };
-    auto issue = [&](uint32_t i) {  // thread 0: the whole-tile columns of tile i
+    auto issue = [&](uint32_t i) {  // thread 0: the columns of tile i
         const uint32_t tile = t1 - 1u - i;
         uint64_t* bar = &bars[i & 1u];
         unsigned char* buf = bufs + (i & 1u) * static_cast<size_t>(a.buf_bytes);
-        uint32_t bytes = 0;
-        if (rows_of(tile) == T)
-            for (uint32_t c = 0; c < a.num_cols; c++) bytes += a.col[c].bulk ? T * a.col[c].bytes : 0u;
-        if (bytes == 0) {
+        if (tile >= a.bulk_tiles) {
             mbar_arrive(bar);
             return;
         }
+        uint32_t bytes = 0;
+        for (uint32_t c = 0; c < a.num_cols; c++) bytes += a.col[c].copied;
         mbar_arrive_expect_tx(bar, bytes);
-        for (uint32_t c = 0; c < a.num_cols; c++)
-            if (a.col[c].bulk)
-                bulk_load_g2s(buf + a.col[c].offset,
-                              a.col[c].in + static_cast<uint64_t>(tile) * T * a.col[c].bytes,
-                              T * a.col[c].bytes, bar);
+        for (uint32_t c = 0; c < a.num_cols; c++) {
+            const RowsColumn& col = a.col[c];
+            bulk_load_g2s(buf + (col.offset - col.lead),
+                          col.in + static_cast<uint64_t>(tile) * T * col.bytes - col.lead, col.copied,
+                          bar);
+        }
     };
     if (tid == 0) issue(0);
     RowShare share{0u, 1u, 0u};
@@ -299,9 +307,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
         const uint32_t rows = rows_of(tile);
         unsigned char* buf = bufs + (i & 1u) * static_cast<size_t>(a.buf_bytes);
         const bool ok = mbar_wait_bounded(&bars[i & 1u], (i >> 1) & 1u);
-        if (rows < T || !a.all_bulk) {  // columns that no bulk copy brought
+        if (tile >= a.bulk_tiles) {  // no bulk copy brought it
             for (uint32_t c = 0; c < a.num_cols; c++) {
-                if (a.col[c].bulk && rows == T) continue;
                 const uint64_t row0 = static_cast<uint64_t>(tile) * T;
                 if constexpr (RECORD) {
                     load_rows<uint32_t, THREADS>(a.col[c], buf, row0, rows);
@@ -323,7 +330,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
             // keys, to the thread that ranks it
             for (uint32_t r = tid; r < rows; r += THREADS)
                 cls[r] = static_cast<unsigned char>(
-                    ok ? d(*reinterpret_cast<const uint32_t*>(buf + r * a.key_stride)) : 0u);
+                    ok ? d(*reinterpret_cast<const uint32_t*>(buf + a.key_offset + r * a.key_stride)) : 0u);
             __syncthreads();
 #pragma unroll
             for (int q = 0; q < ITEMS / 4; q++) {
@@ -331,18 +338,29 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 #pragma unroll
                 for (int j = 0; j < 4; j++) v[4 * q + j] = (e0 + 4 * q + j) | (((x >> (8 * j)) & 0xffu) << 16);
             }
-        } else {  // a column of keys: the thread's own, in 16-byte words (a tile is whole ones)
-            const uint4* keys = reinterpret_cast<const uint4*>(buf + a.key_offset + 4u * e0);
+        } else {  // a column of keys: the thread's own, in 16-byte words
+            const uint32_t off = (a.key_offset >> 2) & 3u;  // keys before the thread's in its first
+            const uint4* keys = reinterpret_cast<const uint4*>(buf + a.key_offset - 4u * off + 4u * e0);
+            uint32_t x[ITEMS + 4];
+            auto load = [&](int q) {
+                uint4 k = make_uint4(0u, 0u, 0u, 0u);
+                if (ok && e0 + 4 * q < rows + off) k = keys[q];
+                x[4 * q] = k.x;
+                x[4 * q + 1] = k.y;
+                x[4 * q + 2] = k.z;
+                x[4 * q + 3] = k.w;
+            };
 #pragma unroll
-            for (int q = 0; q < ITEMS / 4; q++) {
-                uint4 x = make_uint4(0u, 0u, 0u, 0u);
-                if (ok && e0 + 4 * q < rows) x = keys[q];
-                const uint32_t r = e0 + 4 * q;
-                v[4 * q] = r | (d(x.x) << 16);
-                v[4 * q + 1] = (r + 1) | (d(x.y) << 16);
-                v[4 * q + 2] = (r + 2) | (d(x.z) << 16);
-                v[4 * q + 3] = (r + 3) | (d(x.w) << 16);
+            for (int q = 0; q < ITEMS / 4; q++) load(q);
+            if (off != 0u) {  // the same for every thread of the grid
+                load(ITEMS / 4);
+#pragma unroll
+                for (int j = 0; j < ITEMS + 3; j++) x[j] = (off & 1u) ? x[j + 1] : x[j];
+#pragma unroll
+                for (int j = 0; j < ITEMS + 2; j++) x[j] = (off & 2u) ? x[j + 2] : x[j];
             }
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j) | (d(x[j]) << 16);
         }
         auto next = [&] {  // every thread has stored the rows of the other buffer
             if (tid == 0 && i + 1 < cnt) issue(i + 1);

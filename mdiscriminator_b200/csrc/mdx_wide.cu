@@ -96,7 +96,7 @@ constexpr uint32_t rows_buffer(int M) { return M > 16 ? 36864 : 20480; }
 // measured (6 * 10^8 bytes, m = 8: rows of 20, 64, 256 and 1024 bytes 929, 689, 559
 // and 505 us gathered, 347, 317, 260 and 221 whole).
 constexpr uint32_t kMaxRowBytes = 1024;
-static_assert(16 * kMaxRowBytes <= rows_buffer(2) && kMaxRowBytes / 4 <= rows_threads(2), "tile of 16");
+static_assert(16 * kMaxRowBytes + 16 <= rows_buffer(2) && kMaxRowBytes / 4 <= rows_threads(2), "tile of 16");
 
 template <class D, int M, int ITEMS, bool RECORD>
 mdx_status launch_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
@@ -134,26 +134,35 @@ mdx_status launch_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
 template <class D, int M, bool RECORD>
 mdx_status run_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
     constexpr uint32_t TS = rows_threads(M);
-    uint32_t row_bytes = 0;
-    for (uint32_t c = 0; c < a.num_cols; c++) row_bytes += a.col[c].bytes;
+    uint32_t row_bytes = 0, room = rows_buffer(M);
+    bool leads = false;
+    for (uint32_t c = 0; c < a.num_cols; c++) {
+        row_bytes += a.col[c].bytes;
+        a.col[c].lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a.col[c].in) % 16);
+        if (a.col[c].lead != 0) {  // its tile takes a 16-byte word more
+            leads = true;
+            room -= 16;
+        }
+    }
     // eight rows a thread where that many (three quarters of them) fit the buffer,
     // else four; shorter tiles when that gives every SM two of them
-    const uint32_t fit = rows_buffer(M) / row_bytes;
+    const uint32_t fit = room / row_bytes;
     const bool eight = fit >= 6 * TS;
     uint32_t T = std::min(fit & ~15u, TS * (eight ? 8u : 4u));
     while (T > 256 && a.p.n / T < 296) T = (T / 2) & ~15u;
     a.tile_rows = T;
     uint32_t off = 0;
-    a.all_bulk = 1;
     for (uint32_t c = 0; c < a.num_cols; c++) {
-        a.col[c].offset = off;
-        off += T * a.col[c].bytes;  // T is a multiple of 16: 16-byte aligned
-        a.col[c].bulk = reinterpret_cast<uintptr_t>(a.col[c].in) % 16 == 0;
-        a.all_bulk = a.all_bulk && a.col[c].bulk;
+        RowsColumn& col = a.col[c];
+        col.offset = off + col.lead;
+        col.copied = (col.lead + T * col.bytes + 15u) & ~15u;  // T is a multiple of 16
+        off += col.copied;
     }
-    a.key_offset = RECORD ? 0u : a.col[a.end[0]].offset;  // the first of the 4-byte columns
+    a.key_offset = a.col[RECORD ? 0 : a.end[0]].offset;  // the first of the 4-byte columns
     a.buf_bytes = (off + 127u) & ~127u;
     a.p.num_tiles = static_cast<uint32_t>((a.p.n + T - 1) / T);
+    a.bulk_tiles = static_cast<uint32_t>(a.p.n / T);
+    if (leads && a.bulk_tiles == a.p.num_tiles) a.bulk_tiles--;
     return eight ? launch_rows<D, M, 8, RECORD>(a, d, max_stride, st)
                  : launch_rows<D, M, 4, RECORD>(a, d, max_stride, st);
 }

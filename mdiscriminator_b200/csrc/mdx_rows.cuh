@@ -40,6 +40,7 @@ struct RowsColumn {
     uint32_t offset;  // of the column's tile in a tile buffer
     uint32_t lead;    // bytes of the column's first 16-byte word before its first row
     uint32_t copied;  // bytes of the 16-byte words that hold a whole tile
+    uint32_t stride;  // bytes of a whole tile
 };
 
 struct RowsArgs {
@@ -48,6 +49,7 @@ struct RowsArgs {
     uint32_t key_stride;  // bytes between keys
     uint32_t tile_rows;   // rows of a tile, a multiple of 16
     uint32_t buf_bytes;   // of a tile buffer
+    uint32_t copied;      // bytes that a whole tile's copies bring
     uint32_t key_offset;  // of the key column's tile in a tile buffer
     uint32_t num_cols;
     uint32_t bulk_tiles;  // whole tiles that come by bulk copies: all of them, but the last
@@ -281,14 +283,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
             mbar_arrive(bar);
             return;
         }
-        uint32_t bytes = 0;
-        for (uint32_t c = 0; c < a.num_cols; c++) bytes += a.col[c].copied;
-        mbar_arrive_expect_tx(bar, bytes);
-        for (uint32_t c = 0; c < a.num_cols; c++) {
+        mbar_arrive_expect_tx(bar, a.copied);
+        for (uint32_t c = 0; c < (RECORD ? 1u : a.num_cols); c++) {
             const RowsColumn& col = a.col[c];
-            bulk_load_g2s(buf + (col.offset - col.lead),
-                          col.in + static_cast<uint64_t>(tile) * T * col.bytes - col.lead, col.copied,
-                          bar);
+            bulk_load_g2s(buf + col.offset - col.lead,
+                          col.in - col.lead + static_cast<uint64_t>(tile) * col.stride, col.copied, bar);
         }
     };
     if (tid == 0) issue(0);
@@ -341,26 +340,32 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
         } else {  // a column of keys: the thread's own, in 16-byte words
             const uint32_t off = (a.key_offset >> 2) & 3u;  // keys before the thread's in its first
             const uint4* keys = reinterpret_cast<const uint4*>(buf + a.key_offset - 4u * off + 4u * e0);
-            uint32_t x[ITEMS + 4];
-            auto load = [&](int q) {
-                uint4 k = make_uint4(0u, 0u, 0u, 0u);
-                if (ok && e0 + 4 * q < rows + off) k = keys[q];
-                x[4 * q] = k.x;
-                x[4 * q + 1] = k.y;
-                x[4 * q + 2] = k.z;
-                x[4 * q + 3] = k.w;
-            };
+            const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+            if (off == 0u) {  // the same for every thread of the grid
 #pragma unroll
-            for (int q = 0; q < ITEMS / 4; q++) load(q);
-            if (off != 0u) {  // the same for every thread of the grid
-                load(ITEMS / 4);
+                for (int q = 0; q < ITEMS / 4; q++) {
+                    const uint4 x = ok && e0 + 4 * q < rows ? keys[q] : none;
+                    const uint32_t r = e0 + 4 * q;
+                    v[4 * q] = r | (d(x.x) << 16);
+                    v[4 * q + 1] = (r + 1) | (d(x.y) << 16);
+                    v[4 * q + 2] = (r + 2) | (d(x.z) << 16);
+                    v[4 * q + 3] = (r + 3) | (d(x.w) << 16);
+                }
+            } else {
+                uint32_t x[ITEMS + 4];
 #pragma unroll
-                for (int j = 0; j < ITEMS + 3; j++) x[j] = (off & 1u) ? x[j + 1] : x[j];
+                for (int q = 0; q <= ITEMS / 4; q++) {
+                    const uint4 k = ok && e0 + 4 * q < rows + off ? keys[q] : none;
+                    x[4 * q] = k.x;
+                    x[4 * q + 1] = k.y;
+                    x[4 * q + 2] = k.z;
+                    x[4 * q + 3] = k.w;
+                }
 #pragma unroll
-                for (int j = 0; j < ITEMS + 2; j++) x[j] = (off & 2u) ? x[j + 2] : x[j];
+                for (int j = 0; j < ITEMS; j++)
+                    v[j] = (e0 + j) |
+                           (d(off == 1u ? x[j + 1] : off == 2u ? x[j + 2] : x[j + 3]) << 16);
             }
-#pragma unroll
-            for (int j = 0; j < ITEMS; j++) v[j] = (e0 + j) | (d(x[j]) << 16);
         }
         auto next = [&] {  // every thread has stored the rows of the other buffer
             if (tid == 0 && i + 1 < cnt) issue(i + 1);

@@ -84,12 +84,28 @@ inline mdx_status key_order(const unsigned char* keys, uint64_t stride, uint64_t
                          ws + w.plain, w.L.total, reinterpret_cast<mdx_stream_t>(st));
 }
 
-// The row kernels' tiles: 256 threads and two buffers of 20 KB, four CTAs to an SM;
-// above 16 classes 512 threads and two of 36 KB, two CTAs, so that the byte counters'
-// scan is shared by twice the rows (2 * 10^7 rows of a key and 1, 2 and 8 bytes, a
-// call: m = 6 187 us with 256 threads, 192 with 512; m = 32 260 and 205).
+// The row kernels' tiles: 256 threads and two buffers of 20 KB, four CTAs to an SM
+// (three at 9..16 classes with eight rows a thread: buffers of 18 KB, which make room
+// for the fourth, were slower, 304 -> 315 us for 5 * 10^8 bytes of 20-byte rows); above
+// 16 classes 512 threads and two of 36 KB, two CTAs, so that the byte counters' scan is
+// shared by twice the rows (when it was taken, 2 * 10^7 rows of a key and 1, 2 and 8
+// bytes, a call: m = 6 187 us with 256 threads, 192 with 512; m = 32 260 and 205).
 constexpr int rows_threads(int M) { return M > 16 ? 512 : 256; }
-constexpr uint32_t rows_buffer(int M) { return M > 16 ? 36864 : 20480; }
+constexpr uint32_t rows_buffer(int M) { return M > 32 ? 26624 : M > 16 ? 36864 : 20480; }
+// At 33..64 classes the counters leave two CTAs 26 KB a buffer, enough for whole tiles
+// (eight rows a thread) of rows of up to 6 bytes.  A tile of longer rows is cut by the
+// buffer and pays for the same scan, so one CTA with two of 72 KB is better there.  A
+// call at m = 64, one CTA with 36 KB (the only form before), two with 26 KB, one with
+// 72 KB: 2 * 10^7 keys alone 198, 110, 198 us; with a column of 4 bytes 166, 152, 166
+// (3 * 10^6: 26.8, 31.0, 26.8), with seven of one byte 314, 298, 250; 5 * 10^8 bytes of
+// rows of 20 bytes 415, 369, 353, of 64 bytes 324, 303, 260, of 1000 bytes 386, 337, 200.
+constexpr uint32_t kTwoCtaRowBytes = 6;
+constexpr uint32_t rows_buffer(int M, uint32_t row_bytes) {
+    return M > 32 && row_bytes > kTwoCtaRowBytes ? 73728 : rows_buffer(M);
+}
+constexpr int rows_ctas(int M, int items) { return M > 16 ? 2 : M > 8 && items == 8 ? 3 : 4; }
+constexpr size_t kSmBytes = 228 * 1024;  // of an SM
+constexpr size_t cta_bytes(int M) { return 1024 + 256 + 36 * M; }  // reserved, and the kernel's variables
 
 // The row kernels take every record a tile of 16 of which fits the buffer and whose
 // words do not outnumber the threads; the gathered route is behind at every width
@@ -103,11 +119,15 @@ mdx_status launch_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
     constexpr int TS = rows_threads(M);
     auto scatter = rows_scatter_kernel<D, M, TS, ITEMS, RECORD>;
     using SL = RowsSmem<M, TS, ITEMS>;
+    static_assert(rows_ctas(M, ITEMS) * (SL::bytes(rows_buffer(M)) + cta_bytes(M)) <= kSmBytes,
+                  "CTAs of an SM");
     const size_t smem = SL::bytes(a.buf_bytes);
-    // the shared-memory limit is set for the largest buffers, once per kernel
+    // as many CTAs as the buffers leave room for: looked up for the two sizes they have
+    // at most, not for each tile's own (short inputs have short tiles)
+    const uint32_t most = a.buf_bytes <= rows_buffer(M) ? rows_buffer(M) : rows_buffer(M, kMaxRowBytes);
     int blocks = 0, sms = 0;
-    if (host::occupancy(reinterpret_cast<const void*>(scatter), SL::bytes(rows_buffer(M)), &blocks,
-                        &sms, TS) != cudaSuccess)
+    if (host::occupancy(reinterpret_cast<const void*>(scatter), SL::bytes(most), &blocks, &sms, TS) !=
+        cudaSuccess)
         return MDX_ERR_CUDA;
     uint32_t G = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
     G = std::min(std::min(G, a.p.num_tiles), std::min(max_stride, host::kMaxChunks));
@@ -134,10 +154,11 @@ mdx_status launch_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
 template <class D, int M, bool RECORD>
 mdx_status run_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
     constexpr uint32_t TS = rows_threads(M);
-    uint32_t row_bytes = 0, room = rows_buffer(M);
+    uint32_t row_bytes = 0;
+    for (uint32_t c = 0; c < a.num_cols; c++) row_bytes += a.col[c].bytes;
+    uint32_t room = rows_buffer(M, row_bytes);
     bool leads = false;
     for (uint32_t c = 0; c < a.num_cols; c++) {
-        row_bytes += a.col[c].bytes;
         a.col[c].lead = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(a.col[c].in) % 16);
         if (a.col[c].lead != 0) {  // its tile takes a 16-byte word more
             leads = true;
@@ -155,9 +176,11 @@ mdx_status run_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
     for (uint32_t c = 0; c < a.num_cols; c++) {
         RowsColumn& col = a.col[c];
         col.offset = off + col.lead;
-        col.copied = (col.lead + T * col.bytes + 15u) & ~15u;  // T is a multiple of 16
+        col.stride = T * col.bytes;  // T is a multiple of 16
+        col.copied = (col.lead + col.stride + 15u) & ~15u;
         off += col.copied;
     }
+    a.copied = off;
     a.key_offset = a.col[RECORD ? 0 : a.end[0]].offset;  // the first of the 4-byte columns
     a.buf_bytes = (off + 127u) & ~127u;
     a.p.num_tiles = static_cast<uint32_t>((a.p.n + T - 1) / T);

@@ -18,7 +18,8 @@ def order_of(keys, m):
 
 def tile_rows(row_bytes, leads, m):
     """Rows of a tile when there are many: see run_rows."""
-    threads, buf = (512, 36864) if m > 16 else (256, 20480)
+    threads = 512 if m > 16 else 256
+    buf = (26624 if row_bytes <= 6 else 73728) if m > 32 else 36864 if m > 16 else 20480
     fit = (buf - 16 * leads) // row_bytes
     return min(fit & ~15, threads * (8 if fit >= 6 * threads else 4))
 

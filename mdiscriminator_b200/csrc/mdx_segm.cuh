@@ -416,10 +416,19 @@ struct SegSmem {
     // input buffer and an output image, each for a range of < 2P elements plus
     // 16-byte alignment slack (the next group's copy overlaps the current
     // group's write-out; the other resident CTAs cover the rest of its latency)
-    static constexpr int kGroupElems =
-        static_cast<int>(group_window<kTile>()) + kTile + 2 * static_cast<int>(kAU);
+    // A group's range is shorter than 2P.  Above 8 classes the scratch leaves three CTAs
+    // to an SM buffers of 7/4 P: a longer group gives up its last segment to a group of
+    // its own (both parts lie within P).  With buffers of 2P and two CTAs, groups of many
+    // short segments, which latency bounds, were slower than before the class counts
+    // were scanned without flags: 3 * 10^7 u32 in segments of 2 and of up to 32, m = 16,
+    // a call 2855 and 1155 us, 2185 and 895 now (2103 and 899 with flags); log-normal
+    // with median 1024, through head flags, 241 and 221; 2^20 elements in segments of
+    // 4000, whose groups are all cut, 24 and 27.
+    static constexpr int kGroupMost = M > 8 ? kTile / 4 * 7 : static_cast<int>(group_window<kTile>()) + kTile;
+    static constexpr int kGroupElems = kGroupMost + 2 * static_cast<int>(kAU);
     static constexpr size_t kGroupBytes = 2ull * kGroupElems * sizeof(V);
     static constexpr size_t kBytes = 128 + kGroupBytes + group_scratch_bytes<M, THREADS>();  // seg_main
+    static constexpr size_t kSmBytes = 228 * 1024, kReserved = 1024 + 128;  // of an SM, of a CTA
 };
 
 // seg_run_scatter: TMA slot + tile stage + count matrix
@@ -438,14 +447,20 @@ template <int M, int THREADS>
 struct GroupScratch {
     static constexpr int NB = M > 4 ? M / 4 : 1;  // words of byte counts
     static constexpr int NH = M / 2;              // words of 16-bit counts
-    uint32_t hcnt[kGroupSegs][NB];     // its owner thread's class counts before the head
-    uint32_t hpre[kGroupSegs][NH];     // the group's class counts before the head
-    uint32_t hcur[kGroupSegs][NH];     // first position of each class of the segment
+    // per segment; above 8 classes [word][segment], so that neighbouring segments' words
+    // lie in different banks (segments of 2, m = 16: 2855 -> 2546 us), below
+    // [segment][word], which one access takes (m = 4: 118 against 120 us)
+    uint32_t hcnt[NB * kGroupSegs];    // its owner thread's class counts before the head
+    uint32_t hpre[NH * kGroupSegs];    // the group's class counts before the head
+    uint32_t hcur[NH * kGroupSegs];    // first position of each class of the segment
     uint32_t col[NH][THREADS];         // class counts before each thread's elements; before
                                        // that byte counters (M = 16), after it cursors (M > 4)
     uint32_t wagg[NH][THREADS / 32];
     uint16_t hpos[kGroupSegs + 2];     // head of each segment; [nseg] = the group's end
     uint8_t msz[kGroupSegs];           // the segment's class count (per-segment m)
+    static __device__ __forceinline__ uint32_t at(int words, int w, uint32_t seg) {
+        return M > 8 ? w * kGroupSegs + seg : seg * words + w;
+    }
 };
 
 template <int M, int THREADS>
@@ -607,7 +622,7 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                     const uint32_t y = y0 + e;
                     while (nxt == y && qn < nseg) {
 #pragma unroll
-                        for (int q = 0; q < NB; q++) gs.hcnt[qn][q] = cnt.word(gs, q);
+                        for (int q = 0; q < NB; q++) gs.hcnt[GS::at(NB, q, qn)] = cnt.word(gs, q);
                         dc = group_discr(a, d, cmod, gs.msz[qn]);
                         nxt = gs.hpos[++qn];
                     }
@@ -659,7 +674,7 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
 #pragma unroll
             for (int i = 0; i < NH; i++) {
                 const uint32_t w = __shfl_sync(0xffffffffu, wpre[i], t >> 5);
-                p[i] = inside ? w + gs.col[i][t] + widen_pair<M>(gs.hcnt[q][i / 2], i) : tot[i];
+                p[i] = inside ? w + gs.col[i][t] + widen_pair<M>(gs.hcnt[GS::at(NB, i / 2, q)], i) : tot[i];
             }
         };
         before(tid, hq, p0);
@@ -673,8 +688,8 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                 const uint32_t n0 = n & 0xffffu, n1 = n >> 16;
                 const uint32_t o0 = off, o1 = off + n0;
                 off = o1 + n1;
-                gs.hpre[tid][i] = p0[i];
-                gs.hcur[tid][i] = (hq + o0) | ((hq + o1) << 16);
+                gs.hpre[GS::at(NH, i, tid)] = p0[i];
+                gs.hcur[GS::at(NH, i, tid)] = (hq + o0) | ((hq + o1) << 16);
                 if (a.seg_sizes != nullptr) {
                     if (2u * i < a.m) a.seg_sizes[s * a.m + 2 * i] = n0;
                     if (2u * i + 1u < a.m) a.seg_sizes[s * a.m + 2 * i + 1] = n1;
@@ -700,7 +715,8 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
         if (qn > 0u) {
 #pragma unroll
             for (int i = 0; i < NH; i++)
-                cur.set(gs, i, gs.hcur[qn - 1u][i] + (inc[i] - gs.hpre[qn - 1u][i]));
+                cur.set(gs, i, gs.hcur[GS::at(NH, i, qn - 1u)] +
+                                   (inc[i] - gs.hpre[GS::at(NH, i, qn - 1u)]));
         }
         for (uint32_t j = 0; j < nq; j++) {
             const uint32_t y0 = lo + j * VE;
@@ -716,7 +732,7 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                     const uint32_t y = y0 + e;
                     while (nxt == y && qn < nseg) {
 #pragma unroll
-                        for (int i = 0; i < NH; i++) cur.set(gs, i, gs.hcur[qn][i]);
+                        for (int i = 0; i < NH; i++) cur.set(gs, i, gs.hcur[GS::at(NH, i, qn)]);
                         dc = group_discr(a, d, cmod, gs.msz[qn]);
                         nxt = gs.hpos[++qn];
                     }
@@ -831,6 +847,7 @@ __global__ void __launch_bounds__(THREADS, 3)
     constexpr int kPlanner = THREADS - 1;  // the thread that knows the groups to come
     static_assert(M <= 16 && M >= 2, "class bound");
     static_assert(static_cast<int>(kGroupSegs) <= THREADS, "one thread per segment");
+    static_assert(3 * (L::kBytes + L::kReserved) <= L::kSmBytes, "three CTAs to an SM");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
@@ -862,8 +879,10 @@ __global__ void __launch_bounds__(THREADS, 3)
     // ticket after it; the entry; and of the group before that segments and elements
     uint32_t g = blockIdx.x * batch, left = batch - 1u, ticket = 0;
     uint32_t eh = 0, ee = 0, wh = 0, we = 0;
-    bool ev = false, wv = false;
-    uint64_t w0 = 0, w1 = 0;
+    bool ev = false, wv = false, cut = false;  // cut: what is left is the group's last segment
+    uint64_t w0 = 0, w1 = 0, wl = 0;           // its elements; where its last segment begins
+    constexpr uint32_t kMost = L::kGroupMost;
+    constexpr bool kCut = kMost < 2u * P;
     auto draw = [&] { ticket = gridDim.x + atomicAdd(&a.hdr->ticket, 1u); };
     auto load_entry = [&] {  // of group g, then the next group
         ev = g < num_groups;
@@ -885,14 +904,26 @@ __global__ void __launch_bounds__(THREADS, 3)
         we = min(max(we, wh), wh + kGroupSegs);
         w0 = a.offsets[wh];
         w1 = a.offsets[we];
+        if constexpr (kCut) wl = a.offsets[max(we, 1u) - 1u];
     };
-    auto publish = [&](uint32_t q) {
-        const bool bad = w1 < w0 || w1 - w0 >= 2u * P || w1 > a.n;  // malformed: nothing to do
+    auto publish = [&](uint32_t q) {  // true: the group's last segment is still to come
+        cut = kCut && !cut && wv && w1 - w0 > kMost && w1 - w0 < 2u * P && we - wh > 1u;
+        const uint64_t end = cut ? wl : w1;
+        const bool bad = end < w0 || end - w0 > kMost || end > a.n;  // malformed: nothing to do
         range_sh[q].h = wh;
-        range_sh[q].he = bad ? wh : we;
+        range_sh[q].he = bad ? wh : cut ? we - 1u : we;
         range_sh[q].r0 = bad ? 0u : static_cast<uint32_t>(w0);
-        range_sh[q].r1 = bad ? 0u : static_cast<uint32_t>(w1);
+        range_sh[q].r1 = bad ? 0u : static_cast<uint32_t>(end);
         range_sh[q].valid = wv;
+        if (cut) {
+            wh = we - 1u;
+            w0 = wl;
+        }
+        return cut;
+    };
+    auto fetch = [&] {
+        load_range();
+        load_entry();
     };
     // the 16-byte words of a group that one bulk copy brings
     auto vec_end = [&](uint32_t r1, uint64_t as) {
@@ -923,9 +954,7 @@ __global__ void __launch_bounds__(THREADS, 3)
         load_entry();
         load_range();
         load_entry();
-        publish(0);
-        load_range();
-        load_entry();
+        if (!publish(0)) fetch();
     }
     __syncthreads();
     if (tid == 0) issue_group(0);
@@ -936,9 +965,7 @@ __global__ void __launch_bounds__(THREADS, 3)
         const uint32_t h = range_sh[q].h, nseg = range_sh[q].he - h;
         const uint32_t r0 = range_sh[q].r0, r1 = range_sh[q].r1;
         if (tid == kPlanner) {
-            publish(q ^ 1u);
-            load_range();
-            load_entry();
+            if (!publish(q ^ 1u)) fetch();
         }
         const uint64_t as = r0 & ~static_cast<uint64_t>(AU - 1u);
         const uint32_t phase = static_cast<uint32_t>(r0 - as);

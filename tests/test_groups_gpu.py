@@ -97,3 +97,44 @@ def test_groups_a_cta(cuda_ready, batch, groups):
     assert np.array_equal(sizes.cpu().numpy(), es)
     assert np.array_equal(o.cpu().numpy().view(np.uint32), eo)
     assert np.array_equal(hf.cpu().numpy(), ef)
+
+
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("m", [8, 9, 16])
+def test_groups_longer_than_the_buffers(cuda_ready, m, rec):
+    """Above 8 classes a group of more than 7/4 windows gives up its last segment: ranges
+    around that, the last segment as long as it can be, heads around it, a class count
+    per segment."""
+    torch = cuda_ready
+    rng = np.random.default_rng(m)
+    P = 2048 if rec else 4096
+    most = P // 4 * 7
+    lengths = []
+    for total in (most - 1, most, most + 1, most + 9, 2 * P - 1):
+        for parts in ([total - P, P], [3, 0, total - P - 3, P], [0, 1, total - P - 1, P, 0],
+                      [5] * 40 + [total - P - 200, P], [P - 1, total - P + 1]):
+            lengths += parts + [-sum(parts) % P]  # the next group starts a window
+    lengths = np.array(lengths * 3)
+    offs = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint64)
+    n = int(offs[-1])
+    x = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    seg_m = rng.integers(1, m + 1, lengths.size).astype(np.int32)
+    cls = x % np.repeat(seg_m, lengths).astype(np.uint32)
+    if rec:
+        x = x.astype(np.uint64) | (np.arange(n, dtype=np.uint64) << np.uint64(32))
+    eo, es, ef = oracle.partition_segmented(x, offs, m, headflags=True)
+    d = torch.from_numpy(x.view(np.int64 if rec else np.int32)).cuda()
+    do = torch.from_numpy(offs.view(np.int64)).cuda()
+    o, sizes, hf = mdx.partition_segmented(d, do, ("mod", m), headflags=True)
+    torch.cuda.synchronize()
+    assert mdx.workspace(0).error() == mdx.MDX_OK
+    assert np.array_equal(sizes.cpu().numpy(), es)
+    assert np.array_equal(o.cpu().numpy().view(x.dtype), eo)
+    assert np.array_equal(hf.cpu().numpy(), ef)
+    o, sizes = mdx.partition_segmented_multi(d, do, torch.from_numpy(seg_m).cuda(), m)
+    torch.cuda.synchronize()
+    assert mdx.workspace(0).error() == mdx.MDX_OK
+    seg = np.repeat(np.arange(lengths.size), lengths)
+    assert np.array_equal(o.cpu().numpy().view(x.dtype), x[np.lexsort((cls, seg))])
+    counts = np.bincount(seg * m + cls, minlength=lengths.size * m).reshape(-1, m)
+    assert np.array_equal(sizes.cpu().numpy(), counts)

@@ -33,6 +33,9 @@ constexpr int kStages = 2;  // TMA ring of the one-kernel path
 // two tiles has no earlier step to overlap the second one's copy with: two slots
 // (n = 1.5 * 10^6 records of 8 bytes, m = 16, 1.2 tiles a CTA: scatter 11.2 us with
 // one, 10.7 with two; twice as many records: the call 20.7 with one, 22.5 with two).
+// Only where CTAs do have a second tile and the slot does not cost a third: two slots
+// leave an SM fewer CTAs at 17 to 32 classes (2^20 records of 8 bytes, m = 32, 512 tiles:
+// 592 CTAs with one slot, 444 with two, 14.5 and 16.5 us a call).
 constexpr uint32_t kTwoSlotTiles = 2;  // tiles a CTA up to which the ring has two slots
 constexpr size_t kHeaderBytes = 256;  // done, error, ... (see WsHeader)
 constexpr size_t kAlign = 256;
@@ -320,12 +323,17 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
         return MDX_ERR_CUDA;
     size_t smem = SL::bytes(1);
     if constexpr (kBase) {
-        if (step == PlainStep::kBoth &&
-            nt <= kTwoSlotTiles * static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms)) {
-            scatter = plain_scatter_tma_kernel<V, D, M, TS, 2, OutFlat<V>, BPT>;
-            smem = SL::bytes(2);
-            if (occupancy(reinterpret_cast<const void*>(scatter), smem, &blocks, &sms, TS) != cudaSuccess)
+        const uint32_t one = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
+        if (step == PlainStep::kBoth && nt > one && nt <= kTwoSlotTiles * one) {
+            auto two_slots = plain_scatter_tma_kernel<V, D, M, TS, 2, OutFlat<V>, BPT>;
+            int b = 0;
+            if (occupancy(reinterpret_cast<const void*>(two_slots), SL::bytes(2), &b, &sms, TS) != cudaSuccess)
                 return MDX_ERR_CUDA;
+            if (nt <= kTwoSlotTiles * static_cast<uint32_t>(b) * static_cast<uint32_t>(sms)) {
+                scatter = two_slots;
+                smem = SL::bytes(2);
+                blocks = b;
+            }
         }
     }
     if (tun.plain_ctas_per_sm > 0 && static_cast<int>(tun.plain_ctas_per_sm) < blocks)

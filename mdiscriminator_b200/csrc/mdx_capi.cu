@@ -360,7 +360,8 @@ mdx_status mdx_set_tuning(mdx_elem elem, uint32_t m, uint32_t log2_n_lo, uint32_
         return MDX_ERR_INVALID;
     TuningTable& tt = tuning_table();
     std::lock_guard<std::mutex> lk(tt.mu);
-    for (uint32_t b = log2_n_lo; b <= log2_n_hi; b++) {
+    const uint32_t up = elem == MDX_ELEM_REC16 ? kRec16Log2 : 0u;
+    for (uint32_t b = std::min(log2_n_lo + up, 33u); b <= std::min(log2_n_hi + up, 33u); b++) {
         Tuning& x = tt.t[elem == MDX_ELEM_REC8 ? 1 : 0][bound_index(class_bound(m))][b];
         x.plain_ctas_per_sm = t->plain_ctas_per_sm;
         x.run_tiles = t->run_tiles ? t->run_tiles : kRunTiles;

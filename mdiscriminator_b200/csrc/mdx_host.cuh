@@ -251,10 +251,16 @@ inline int bound_index(uint32_t M) {
     while ((2u << i) < M && i < 6) i++;
     return i;
 }
+// 16-byte records share the entries of u32 values, those of the same bytes (and so of
+// as many tiles): 2 more in log2 n.  Those of the same number, where a quarter of the
+// tiles is spread over the CTAs, cost 2^20 records in class order, m = 4, 15.7 us a call
+// for 14.3.
+constexpr uint32_t kRec16Log2 = 2;
 inline Tuning tuning_for(mdx_elem e, uint32_t M, uint64_t n) {
     TuningTable& tt = tuning_table();
     std::lock_guard<std::mutex> lk(tt.mu);
-    return tt.t[e == MDX_ELEM_REC8 ? 1 : 0][bound_index(M)][log2_ceil(n)];
+    return tt.t[e == MDX_ELEM_REC8 ? 1 : 0][bound_index(M)]
+               [log2_ceil(e == MDX_ELEM_REC16 ? n << kRec16Log2 : n)];
 }
 
 // Steps of a plain call: both kernels, or (distributed partition) the count
@@ -316,7 +322,8 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     const void* const base_in = static_cast<const V*>(d_in) - shift;
     const uint32_t tiles_n = static_cast<uint32_t>((n + TILE - 1) / TILE);
     const uint32_t nt = static_cast<uint32_t>((n + shift + TILE - 1) / TILE);
-    const Tuning tun = tuning_for(sizeof(V) == 8 ? MDX_ELEM_REC8 : MDX_ELEM_U32, M, n);
+    const Tuning tun = tuning_for(
+        sizeof(V) == 16 ? MDX_ELEM_REC16 : sizeof(V) == 8 ? MDX_ELEM_REC8 : MDX_ELEM_U32, M, n);
     auto scatter = plain_scatter_tma_kernel<V, D, M, TS, 1, OutFlat<V>, BPT>;
     int blocks = 0, sms = 0;
     if (occupancy(reinterpret_cast<const void*>(scatter), SL::bytes(1), &blocks, &sms, TS) != cudaSuccess)

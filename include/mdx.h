@@ -369,7 +369,8 @@ mdx_status mdx_server_destroy(mdx_server server);
  * Entries are kept per (element layout, class bound = smallest power of two
  * >= m, ceil(log2 n)); mdx_set_tuning sets every n bucket in
  * [log2_n_lo, log2_n_hi].  Zero fields keep the built-in default.  16-byte records
- * share the plain entries of 4-byte values with as many bytes (log2 n larger by 2).
+ * share the plain entries of 4-byte values with as many bytes (log2 n larger by 2);
+ * above 16 classes they always take two kernels and 512 threads.
  */
 typedef struct {
     uint32_t plain_ctas_per_sm;  /* plain path: CTAs per SM of the chunk grid (0: as many as fit) */

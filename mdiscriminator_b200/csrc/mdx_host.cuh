@@ -290,6 +290,9 @@ constexpr uint32_t kFusedPoolPct = 10;  // share of every chunk drained by ticke
 static_assert(kFusedBarOffset >= kDistSkipOffset + 4 && kFusedBarOffset + 16 <= kHeaderBytes,
               "barrier words inside the header");
 
+template <class V, int M>
+constexpr bool kWideRec16 = sizeof(V) == 16 && M > 16;  // see run_plain
+
 // BPT: bytes of a tile per thread (64: the tiles of every path; 32: tiles
 // half as long); TS: threads of a scatter CTA (256, or 512 for tiles twice
 // as long).  Geometries other than 64 bytes x 256 threads run the two-kernel
@@ -413,7 +416,7 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
             return cudaLaunchKernelEx(&cfg, small, b, d, o) == cudaSuccess ? MDX_OK : MDX_ERR_CUDA;
         }
     }
-    if constexpr (kBase) {  // the one-kernel path has the base geometry only
+    if constexpr (kBase && !kWideRec16<V, M>) {  // the one-kernel path has the base geometry only
         if (step == PlainStep::kBoth && dist == nullptr && ev_mid == nullptr && allow_fused &&
             tun.plain_two_kernel == 0) {
             // one cooperative kernel: count, grid barrier, scatter (mdx_fused.cuh)
@@ -553,6 +556,16 @@ mdx_status run_plain(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
                                                           d_headflags, ws, L, stream, ev_mid, step,
                                                           dist, allow_fused);
         }
+    }
+    // 16-byte records above 16 classes: a thread has four, and the scan of its counters
+    // costs as much as for sixteen values, so tiles of 512 threads and two kernels,
+    // whatever the knobs (2^25 records, a call: m = 32 292 us with 256 threads, 356 in
+    // one kernel, 285 with 512; m = 64 360, 399, 311; the ballots per class bit that the
+    // counters replaced 312 and 325)
+    if constexpr (kWideRec16<V, M>) {
+        if (dist == nullptr && step == PlainStep::kBoth && n > kSmallTiles * 1024)
+            return run_plain_g<V, D, M, 64, 512>(d_in, d_out, n, d, m, d_sizes, d_headflags, ws, L,
+                                                 stream, ev_mid, step, dist, allow_fused);
     }
     return run_plain_g<V, D, M, 64, kThreads>(d_in, d_out, n, d, m, d_sizes, d_headflags, ws, L,
                                               stream, ev_mid, step, dist, allow_fused);

@@ -37,10 +37,10 @@ if os.path.dirname(HERE) not in sys.path:
 
 import mdiscriminator_b200 as mdx  # noqa: E402
 
-# n buckets: (timed n of 4-byte values, ceil(log2 n) range the winner is
-# installed for); 8-byte records are timed at half the count (same bytes).  Where a
-# grid has few tiles a CTA the geometry that wins changes from one power of two to
-# the next, so those have a bucket each, timed at three quarters of their range.
+# n buckets: (timed n, ceil(log2 n) range the winner is installed for); the longest
+# arrays of 8-byte records have half the count (see timed_count).  Where a grid has few
+# tiles a CTA the geometry that wins changes from one power of two to the next, so
+# those have a bucket each, timed at three quarters of their range.
 BUCKETS = [(1 << 17, (0, 18)), (3 << 18, (19, 20)), (3 << 19, (21, 21)), (3 << 20, (22, 22)),
            (3 << 21, (23, 23)), (3 << 22, (24, 24)), (3 << 23, (25, 25)), (1 << 28, (26, 33))]
 
@@ -51,6 +51,15 @@ BUCKETS = [(1 << 17, (0, 18)), (3 << 18, (19, 20)), (3 << 19, (21, 21)), (3 << 2
 # picked here.
 PLAIN_CANDIDATES = [(1, 0, 0, 64, 256), (1, 3, 0, 64, 256), (1, 2, 0, 64, 256),
                     (1, 0, 0, 64, 512), (1, 1, 0, 64, 512)]
+
+
+PLAIN_KNOBS = ("plain_ctas_per_sm", "plain_two_kernel", "pool_pct", "tile_bytes", "tile_threads")
+
+
+def timed_count(elem, n, bucket):
+    """Elements that a bucket is timed at, which lie in it: n, or for 8-byte records in
+    the last one half as many (the same bytes)."""
+    return n // 2 if elem == mdx.ELEM_REC8 and bucket == BUCKETS[-1][1] else n
 
 
 def timeit(graph, torch, reps=9):
@@ -89,19 +98,29 @@ def main(argv=None):
     ap = argparse.ArgumentParser()
     ap.add_argument("--out", default=mdx.TUNING_PATH)
     ap.add_argument("--quick", action="store_true", help="fewer candidates and sizes")
+    ap.add_argument("--elem", choices=("u32", "rec8"), help="this layout only; the table at --out "
+                    "keeps its other entries")
+    ap.add_argument("--up-to", type=int, default=33, help="buckets up to this log2 n only, likewise")
+    ap.add_argument("--plain", action="store_true", help="the plain path's knobs only, likewise")
     args = ap.parse_args(argv)
+    kept = {"entries": [], "timings": [], "runs": []}
+    if args.elem or args.plain or args.up_to < 33:
+        with open(args.out) as f:
+            kept = json.load(f)
     import torch
     dev = torch.device("cuda", 0)
     g = torch.Generator(device=dev).manual_seed(1)
     entries = []
     bounds = [2, 4, 8, 16] if args.quick else [2, 4, 8, 16, 32, 64]
-    buckets = BUCKETS[1:] if args.quick else BUCKETS
+    buckets = [b for b in (BUCKETS[1:] if args.quick else BUCKETS) if b[1][1] <= args.up_to]
     t0 = time.time()
     for elem in (mdx.ELEM_U32, mdx.ELEM_REC8):
         ename = "u32" if elem == mdx.ELEM_U32 else "rec8"
+        if args.elem not in (None, ename):
+            continue
         dtype = torch.int32 if elem == mdx.ELEM_U32 else torch.int64
-        for n4, (lo, hi) in buckets:
-            n = n4 if elem == mdx.ELEM_U32 else n4 // 2
+        for n0, (lo, hi) in buckets:
+            n = timed_count(elem, n0, (lo, hi))
             d = torch.randint(0, 1 << 31, (n,), device=dev, dtype=torch.int64, generator=g).to(dtype)
             out = torch.empty_like(d)
             ws = mdx.new_workspace(mdx.workspace_size(n, elem, 64), dev)
@@ -128,8 +147,8 @@ def main(argv=None):
                                tile_threads=best[5])
             del d, out, ws
         seg_bounds = [2, 4, 8, 16]
-        for n4, (lo, hi) in buckets:
-            n_target = min(n4 if elem == mdx.ELEM_U32 else n4 // 2, 1 << 27)
+        for n0, (lo, hi) in [] if args.plain else buckets:
+            n_target = min(timed_count(elem, n0, (lo, hi)), 1 << 27)
             offs = lognormal_offsets(n_target, 3)
             n = int(offs[-1])
             S = len(offs) - 1
@@ -170,13 +189,22 @@ def main(argv=None):
                                mid_tiles=best[3])
             del d, out, ws
     # one entry per key: the segmented entry (it carries the plain knob too)
-    merged = {}
-    for e in entries:
-        key = (e["elem"], e["m"], tuple(e["log2_n"]))
-        if key not in merged or e["path"] == "segmented":
-            merged[key] = e
-    table = {"device": torch.cuda.get_device_name(0), "tuned_in_s": round(time.time() - t0, 1),
-             "entries": list(merged.values()), "timings": entries}
+    def key_of(e):
+        return e["elem"], e["m"], tuple(e["log2_n"])
+
+    merged = {key_of(e): e for e in kept["entries"]}
+    for e in entries:  # a key's segmented entry comes after its plain one
+        old = merged.get(key_of(e), e)
+        merged[key_of(e)] = {**old, **{k: e[k] for k in PLAIN_KNOBS}} \
+            if args.plain and old["path"] == "segmented" else e
+    tuned = {(key_of(e), e["path"]) for e in entries}
+    table = {"device": torch.cuda.get_device_name(0),
+             "runs": kept["runs"] + [{"elem": args.elem or "all",
+                                      "path": "plain" if args.plain else "all",
+                                      "up_to_log2_n": args.up_to,
+                                      "seconds": round(time.time() - t0, 1)}],
+             "entries": list(merged.values()),
+             "timings": [e for e in kept["timings"] if (key_of(e), e["path"]) not in tuned] + entries}
     with open(args.out, "w") as f:
         json.dump(table, f, indent=1)
     print(f"wrote {len(merged)} entries to {args.out} in {time.time() - t0:.0f} s")

@@ -368,7 +368,7 @@ mdx_status mdx_server_destroy(mdx_server server);
  * its block shapes at compile time with -D macros swept by cuda_code/run.py).
  * Entries are kept per (element layout, class bound = smallest power of two
  * >= m, ceil(log2 n)); mdx_set_tuning sets every n bucket in
- * [log2_n_lo, log2_n_hi].  Zero fields keep the built-in default.  16-byte records
+ * [log2_n_lo, log2_n_hi].  Zero fields take the default stated with them.  16-byte records
  * share the plain entries of 4-byte values with as many bytes (log2 n larger by 2);
  * above 16 classes they always take two kernels and 512 threads.
  */
@@ -376,8 +376,9 @@ typedef struct {
     uint32_t plain_ctas_per_sm;  /* plain path: CTAs per SM of the chunk grid (0: as many as fit) */
     uint32_t run_tiles;          /* segmented: tiles per run of a large segment (default 8) */
     uint32_t group_batch;        /* segmented: small-segment groups per work item (default 8, at most 32) */
-    uint32_t plain_two_kernel;   /* plain path: 1 = count and scatter as two kernels; 0 (default) =
-                                    one cooperative kernel where the input allows TMA */
+    uint32_t plain_two_kernel;   /* plain path: 1 = count and scatter as two kernels (also where
+                                    nothing was set); 0 = one cooperative kernel where the
+                                    input allows TMA */
     uint32_t pool_pct;           /* one-kernel plain path: % of every chunk's tiles that the CTAs
                                     share by ticket at the end of each phase (0: default 10;
                                     100: none) */

@@ -222,12 +222,17 @@ inline bool make_row_map(CUtensorMap* map, const void* base, uint64_t n, size_t 
 
 // ------------------------------------------------------------------ tuning --
 // Run-time knobs per (element width, class bound, log2 n), installed by
-// mdx_set_tuning (the package loads the autotuner's table at import).
+// mdx_set_tuning (the package loads the autotuner's table at import).  These are what
+// callers without a table run with, those of the C ABI and the C++ templates: two
+// kernels, which are as fast as the one-kernel form or faster at every class count and
+// size measured (4-, 8- and 16-byte elements, 2^17 to 2^29 bytes; 2^27 u32, m = 2, 8,
+// 16, 64, a call: 276, 288, 360, 507 us in one kernel, 267, 279, 304, 459 in two; 2^26
+// records of 8 bytes 271, 281, 329, 464 and 263, 273, 278, 402).
 struct Tuning {
     uint32_t plain_ctas_per_sm = 0;  // 0: as many as fit
     uint32_t run_tiles = kRunTiles;
     uint32_t group_batch = kGroupBatch;
-    uint32_t plain_two_kernel = 0;  // 1: count and scatter as two kernels
+    uint32_t plain_two_kernel = 1;  // 1: count and scatter as two kernels; 0: the one-kernel form
     uint32_t pool_pct = 0;          // one-kernel path: % of every chunk drained by ticket (0: default)
     uint32_t mid_tiles = 0;         // segmented: medium segments up to this many tiles (0, 1: none)
     uint32_t tile_bytes = 0;        // plain path: tile bytes per thread (0, 64: 64; 32: 32)

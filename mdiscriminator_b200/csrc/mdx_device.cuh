@@ -206,12 +206,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ------------------------------------------------------------- warp helpers --
-__device__ __forceinline__ uint32_t lanemask_lt() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -229,14 +223,6 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t x) {
 }
 
 // Acquire / release accesses at GPU scope for cross-CTA publication.
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -354,8 +354,12 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     if (tun.plain_ctas_per_sm > 0 && static_cast<int>(tun.plain_ctas_per_sm) < blocks)
         blocks = static_cast<int>(tun.plain_ctas_per_sm);
     uint32_t G = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
-    if (G > tiles_n) G = tiles_n;  // the tables hold a chunk for each of the n elements' tiles
+    if (G > tiles_n) G = tiles_n;
     if (G > kMaxChunks) G = kMaxChunks;
+    // the counts have room for a chunk per 64-byte tile of 256 threads; a whole call keeps
+    // no prefixes, so those of the shorter tiles, twice as many, may take theirs too
+    const size_t room = ((step == PlainStep::kBoth ? L.tile_cnt : L.ready) - L.chunk_cnt) / (4 * M);
+    if (G > (room & ~size_t{3})) G = static_cast<uint32_t>(room & ~size_t{3});
 
     PlainArgs a;
     a.in = base_in;
@@ -565,7 +569,7 @@ mdx_status run_plain(const void* d_in, void* d_out, uint64_t n, D d, uint32_t m,
     // 16-byte records above 16 classes: a thread has four, and the scan of its counters
     // costs as much as for sixteen values, so tiles of 512 threads and two kernels,
     // whatever the knobs (2^25 records, a call: m = 32 292 us with 256 threads, 356 in
-    // one kernel, 285 with 512; m = 64 360, 399, 311; the ballots per class bit that the
+    // one kernel, 288 with 512; m = 64 360, 399, 316; the ballots per class bit that the
     // counters replaced 312 and 325)
     if constexpr (kWideRec16<V, M>) {
         if (dist == nullptr && step == PlainStep::kBoth && n > kSmallTiles * 1024)

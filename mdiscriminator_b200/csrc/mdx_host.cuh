@@ -33,9 +33,11 @@ constexpr int kStages = 2;  // TMA ring of the one-kernel path
 // two tiles has no earlier step to overlap the second one's copy with: two slots
 // (n = 1.5 * 10^6 records of 8 bytes, m = 16, 1.2 tiles a CTA: scatter 11.2 us with
 // one, 10.7 with two; twice as many records: the call 20.7 with one, 22.5 with two).
-// Only where CTAs do have a second tile and the slot does not cost a third: two slots
-// leave an SM fewer CTAs at 17 to 32 classes (2^20 records of 8 bytes, m = 32, 512 tiles:
-// 592 CTAs with one slot, 444 with two, 14.5 and 16.5 us a call).
+// Not where the CTAs that two slots leave an SM need a round of tiles more (2^20 records
+// of 8 bytes, m = 32, 512 tiles: 592 CTAs with one slot, 444 with two, 14.5 and 16.5 us a
+// call).  A single round takes them too: larger CTAs are spread over more SMs when they
+// are scheduled beside the count's (2^20 u32, 256 tiles, replayed: m = 13 sorted by
+// class 14.5 us with one slot, 12.4 with two, m = 32 12.4 and 11.0).
 constexpr uint32_t kTwoSlotTiles = 2;  // tiles a CTA up to which the ring has two slots
 constexpr size_t kHeaderBytes = 256;  // done, error, ... (see WsHeader)
 constexpr size_t kAlign = 256;
@@ -339,12 +341,13 @@ mdx_status run_plain_g(const void* d_in, void* d_out, uint64_t n, D d, uint32_t 
     size_t smem = SL::bytes(1);
     if constexpr (kBase) {
         const uint32_t one = static_cast<uint32_t>(blocks) * static_cast<uint32_t>(sms);
-        if (step == PlainStep::kBoth && nt > one && nt <= kTwoSlotTiles * one) {
+        if (step == PlainStep::kBoth && nt <= kTwoSlotTiles * one) {
             auto two_slots = plain_scatter_tma_kernel<V, D, M, TS, 2, OutFlat<V>, BPT>;
             int b = 0;
             if (occupancy(reinterpret_cast<const void*>(two_slots), SL::bytes(2), &b, &sms, TS) != cudaSuccess)
                 return MDX_ERR_CUDA;
-            if (nt <= kTwoSlotTiles * static_cast<uint32_t>(b) * static_cast<uint32_t>(sms)) {
+            const uint32_t two = static_cast<uint32_t>(b) * static_cast<uint32_t>(sms);
+            if ((nt + two - 1) / two == (nt + one - 1) / one) {
                 scatter = two_slots;
                 smem = SL::bytes(2);
                 blocks = b;

@@ -62,10 +62,16 @@ def timed_count(elem, n, bucket):
     return n // 2 if elem == mdx.ELEM_REC8 and bucket == BUCKETS[-1][1] else n
 
 
+def tie(ms):
+    """What a candidate has to be below of the best one before it: replays of a few
+    microseconds come in steps of two, those of a tenth of a millisecond and more are
+    told apart to 1 %."""
+    return 0.96 if ms < 0.1 else 0.99
+
+
 def timeit(graph, torch, reps=9):
     """Median time of one of ten replays of a captured call (no host time between
-    its launches).  Replays of a few microseconds come in steps of two, so a
-    candidate has to be clearly faster to replace the one before it."""
+    its launches)."""
     for _ in range(10):
         graph.launch()
     torch.cuda.synchronize()
@@ -136,7 +142,7 @@ def main(argv=None):
                     ms = timeit(mdx.capture_partition(d, ("mask", M), out, sizes, ws=ws), torch)
                     if ws.error() != mdx.MDX_OK:
                         raise SystemExit(f"device error while tuning {ename} m={M}")
-                    if best is None or ms < 0.96 * best[0]:  # ties stay with the first
+                    if best is None or ms < tie(best[0]) * best[0]:  # ties stay with the first
                         best = (ms, k, two, pool, tb, tt)
                 entries.append({"elem": ename, "m": M, "log2_n": [lo, hi], "path": "plain",
                                 "plain_ctas_per_sm": best[1], "plain_two_kernel": best[2],

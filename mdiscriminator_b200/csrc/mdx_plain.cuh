@@ -453,8 +453,8 @@ __device__ __forceinline__ void scatter_cursors(const PlainArgs& a, uint32_t k, 
 // is shared by twice the elements (N = 2^28 u32, m = 2, 4, 8, 16, 64: scatter
 // 346, 359, 367, 404, 707 us with 256 threads, 335, 343, 353, 391, 597 with 512;
 // a device copy of the same bytes takes 337).  Up to 16 classes that is 2 to 3 % of the
-// whole call, less than the tuner asks of a candidate, so its table has 256 there but
-// for m = 4 with 8-byte records.
+// whole call: the table has 512 there for records at m = 4 and 8 only, its 4-byte
+// entries up to 16 classes being of a run that asked a candidate to be 4 % faster.
 // SLOTS: tiles in flight per CTA (1 or 2).
 template <class V, class D, int M, int THREADS, int SLOTS, class OUT = OutFlat<V>, int BPT = 64>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)  // 32 warps per SM: <= 64 registers

@@ -273,7 +273,8 @@ mdx_status mdx_partition_columns(const mdx_column* cols, uint32_t num_cols, uint
  *      d_counts (device).
  *   2. the caller all-gathers the counts of every rank into d_all_counts
  *      ([R][m], rank-major; one tiny collective, e.g. an NCCL all-gather);
- *   3. mdx_dist_scatter (same workspace, same n_local): each element is stored
+ *   3. mdx_dist_scatter (same workspace, same n_local, the counted elements, in the
+ *      same buffer or another): each element is stored
  *      straight into the chunk that owns its output position -- through
  *      out_chunks[q], a HOST array of R device pointers, peers' chunks mapped
  *      into this process (mdx_ipc_*) -- by the same kernel that ranks it; the

@@ -16,9 +16,9 @@
 // without intermediates.  The {key, row} records, partitioned as 8-byte elements
 // and followed by a gather of the rows, that this replaces cost 48 bytes of
 // traffic a row beyond that, and the gather's reads touched every sector once for
-// each class.  3 * 10^7 rows of 20 bytes, m = 8: 924 -> 347 us a call (scatter 235,
-// count 108; read twice and written once at the copy rate: 275).  2 * 10^7 rows of
-// a key and columns of 1, 2 and 8 bytes, m = 6: 415 -> 153 us (floor 104).  Rows of
+// each class.  3 * 10^7 rows of 20 bytes, m = 8: 924 -> 345 us a call (scatter about
+// 235, count 108; read twice and written once at the copy rate: 275).  2 * 10^7 rows of
+// a key and columns of 1, 2 and 8 bytes, m = 6: 415 -> 148 us (floor 104).  Rows of
 // 32 bytes and more are bound by memory, narrower ones by the instructions a row
 // costs (ranks, two table lookups, a load and a store per column).
 #pragma once
@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     // per column, of the 16-byte words that hold them: a column off a 16-byte address
     // lies `lead` bytes into its room.  Element loads with a barrier after them, which
     // took the place of the copies there: 5 * 10^8 bytes at 4 bytes off, a call, rows of
-    // 20 bytes m = 8 412 us, now 284 (aligned 280), of 256 bytes m = 64 673 and 358
-    // (279: its rows move by 4 bytes, not 16); 2 * 10^7 rows of a key and seven columns of
-    // 8 bytes, m = 2, 1093 and 451 (446).
+    // 20 bytes m = 8 412 us, now 274 (aligned 271), of 256 bytes 363 and 226 (212: its
+    // rows move by 4 bytes, not 16); 2 * 10^7 rows of a key and seven columns of 8 bytes,
+    // m = 2, 1093 and 452 (446).
     auto rows_of = [&](uint32_t tile) {
         return static_cast<uint32_t>(
             min(static_cast<uint64_t>(T), a.p.n - static_cast<uint64_t>(tile) * T));

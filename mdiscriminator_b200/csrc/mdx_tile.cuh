@@ -850,10 +850,10 @@ __device__ __forceinline__ bool tile_scatter_bytes(const D& d, const V (&v)[ITEM
     } else if (full) {
         // Records whose neighbours share a class: stored in the threads' own order, lanes
         // of one class meet in two banks.  3 * 10^7 records of 8 bytes in runs of 300, a
-        // call: m = 32 175 us without the look and 154 with it, m = 64 200 and 167; the
-        // one-kernel form on sorted records, m = 32, 194 and 169.  Random classes pay 1.8
-        // and 0.3 % for the look.  4-byte values go without: their sixteen a thread share
-        // a class less often, and such inputs were no slower than before.
+        // call: m = 32 175 us without the look and 154 with it (256 threads), m = 64 200
+        // and 167; the one-kernel form on sorted records, m = 32, 194 and 169.  Random
+        // classes pay 1.8 and 0.3 % for the look.  4-byte values go without: their sixteen
+        // a thread share a class less often, and in runs they were no slower than before.
         constexpr bool kSpread = !CLUSTERED && sizeof(V) >= 8;
         constexpr uint32_t kLast = 8 * ((ITEMS - 1) & 3);
         const bool one = kSpread && (lr[(ITEMS - 1) >> 2] >> kLast) == ITEMS - 1;

@@ -52,8 +52,8 @@ struct RowsArgs {
     uint32_t copied;      // bytes that a whole tile's copies bring
     uint32_t key_offset;  // of the key column's tile in a tile buffer
     uint32_t num_cols;
-    uint32_t bulk_tiles;  // whole tiles that come by bulk copies: all of them, but the last
-                          // when a column has a lead (its copy would pass the column's end)
+    uint32_t bulk_tiles;  // whole tiles that come by bulk copies: all of them, but when a
+                          // column has a lead not the last (its copy could pass the end)
     uint32_t end[4];      // columns (not a record): end[q] of 8 >> q bytes or more, the wider first
     RowsColumn col[kMaxCols];
 };

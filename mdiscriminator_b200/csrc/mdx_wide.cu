@@ -184,8 +184,8 @@ mdx_status run_rows(RowsArgs a, D d, uint32_t max_stride, cudaStream_t st) {
     a.key_offset = a.col[RECORD ? 0 : a.end[0]].offset;  // the first of the 4-byte columns
     a.buf_bytes = (off + 127u) & ~127u;
     a.p.num_tiles = static_cast<uint32_t>((a.p.n + T - 1) / T);
-    a.bulk_tiles = static_cast<uint32_t>(a.p.n / T);
-    if (leads && a.bulk_tiles == a.p.num_tiles) a.bulk_tiles--;
+    // a copy of whole words ends up to 15 bytes past its tile: 16 rows of any column on
+    a.bulk_tiles = static_cast<uint32_t>((a.p.n - (leads ? std::min<uint64_t>(a.p.n, 16) : 0)) / T);
     return eight ? launch_rows<D, M, 8, RECORD>(a, d, max_stride, st)
                  : launch_rows<D, M, 4, RECORD>(a, d, max_stride, st);
 }

@@ -70,3 +70,26 @@ def test_columns(cuda_ready, widths, m):
             for e, g in zip(expect, got):
                 assert np.array_equal(g.cpu().numpy(), e), (n, off, e.dtype)
             assert np.array_equal(sizes.cpu().numpy(), es)
+
+
+@pytest.mark.parametrize("m", [2, 16, 64])
+def test_numbers_of_rows_after_the_last_whole_tile(cuda_ready, m):
+    """Fewer rows of a one-byte column than a 16-byte word holds, and more."""
+    torch = cuda_ready
+    tile = tile_rows(5, 2, m)
+    for n in (5, 15, 16, 17, 300 * tile + 1, 300 * tile + 15, 300 * tile + 16, 300 * tile + 17):
+        rng = np.random.default_rng(n + m)
+        keys = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+        perm, es = order_of(keys, m)
+        other = rng.integers(0, 256, n, dtype=np.uint8)
+        for at in (1, 15):
+            base = torch.zeros(n + 3, dtype=torch.int32, device="cuda")[3:]
+            base.copy_(torch.from_numpy(keys.view(np.int32)))
+            col = torch.zeros(n + at, dtype=torch.uint8, device="cuda")[at:]
+            col.copy_(torch.from_numpy(other))
+            got, sizes = mdx.partition_columns([base, col], ("mod", m))
+            torch.cuda.synchronize()
+            assert mdx.workspace(0).error() == mdx.MDX_OK
+            assert np.array_equal(got[0].cpu().numpy().view(np.uint32), keys[perm]), (n, at)
+            assert np.array_equal(got[1].cpu().numpy(), other[perm]), (n, at)
+            assert np.array_equal(sizes.cpu().numpy(), es)

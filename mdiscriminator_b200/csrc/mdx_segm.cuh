@@ -421,8 +421,8 @@ struct SegSmem {
     // its own (both parts lie within P).  With buffers of 2P and two CTAs, groups of many
     // short segments, which latency bounds, were slower than before the class counts
     // were scanned without flags: 3 * 10^7 u32 in segments of 2 and of up to 32, m = 16,
-    // a call 2855 and 1155 us, 2185 and 895 now (2103 and 899 with flags); log-normal
-    // with median 1024, through head flags, 241 and 221; 2^20 elements in segments of
+    // a call 2855 and 1155 us, 2126 and 820 now (2103 and 899 with flags); log-normal
+    // with median 1024, through head flags, 240 and 219; 2^20 elements in segments of
     // 4000, whose groups are all cut, 24 and 27.
     static constexpr int kGroupMost = M > 8 ? kTile / 4 * 7 : static_cast<int>(group_window<kTile>()) + kTile;
     static constexpr int kGroupElems = kGroupMost + 2 * static_cast<int>(kAU);
@@ -447,19 +447,50 @@ template <int M, int THREADS>
 struct GroupScratch {
     static constexpr int NB = M > 4 ? M / 4 : 1;  // words of byte counts
     static constexpr int NH = M / 2;              // words of 16-bit counts
-    // per segment; above 8 classes [word][segment], so that neighbouring segments' words
-    // lie in different banks (segments of 2, m = 16: 2855 -> 2546 us), below
-    // [segment][word], which one access takes (m = 4: 118 against 120 us)
-    uint32_t hcnt[NB * kGroupSegs];    // its owner thread's class counts before the head
-    uint32_t hpre[NH * kGroupSegs];    // the group's class counts before the head
-    uint32_t hcur[NH * kGroupSegs];    // first position of each class of the segment
+    // per segment, N words each (load, store)
+    alignas(16) uint32_t hcnt[NB * kGroupSegs];  // its owner thread's class counts before the head
+    alignas(16) uint32_t hpre[NH * kGroupSegs];  // the group's class counts before the head
+    alignas(16) uint32_t hcur[NH * kGroupSegs];  // first position of each class of the segment
     uint32_t col[NH][THREADS];         // class counts before each thread's elements; before
                                        // that byte counters (M = 16), after it cursors (M > 4)
     uint32_t wagg[NH][THREADS / 32];
     uint16_t hpos[kGroupSegs + 2];     // head of each segment; [nseg] = the group's end
     uint8_t msz[kGroupSegs];           // the segment's class count (per-segment m)
-    static __device__ __forceinline__ uint32_t at(int words, int w, uint32_t seg) {
-        return M > 8 ? w * kGroupSegs + seg : seg * words + w;
+    // Above 8 classes in 16-byte words, the two of eight u32 swapped in every other four
+    // segments, so that neighbouring segments' words lie in different banks (3 * 10^7
+    // u32 in segments of two and of up to 32, m = 16: 2185 and 895 us a call with every
+    // word of its own, [word][segment], 2126 and 820 so).
+    template <int N>
+    static __device__ __forceinline__ uint32_t word(uint32_t seg, int q) {
+        return N == 8 ? 2u * seg + (q ^ (seg >> 2 & 1u)) : N / 4 * seg + q;
+    }
+    template <int N>
+    static __device__ __forceinline__ void load(const uint32_t* a, uint32_t seg, uint32_t (&x)[N]) {
+        if constexpr (M > 8) {
+#pragma unroll
+            for (int q = 0; q < N / 4; q++) {
+                const uint4 v = reinterpret_cast<const uint4*>(a)[word<N>(seg, q)];
+                x[4 * q] = v.x;
+                x[4 * q + 1] = v.y;
+                x[4 * q + 2] = v.z;
+                x[4 * q + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int w = 0; w < N; w++) x[w] = a[seg * N + w];
+        }
+    }
+    template <int N>
+    static __device__ __forceinline__ void store(uint32_t* a, uint32_t seg, const uint32_t (&x)[N]) {
+        if constexpr (M > 8) {
+#pragma unroll
+            for (int q = 0; q < N / 4; q++)
+                reinterpret_cast<uint4*>(a)[word<N>(seg, q)] =
+                    make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int w = 0; w < N; w++) a[seg * N + w] = x[w];
+        }
     }
 };
 
@@ -621,8 +652,10 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                 for (uint32_t e = 0; e < VE; e++) {
                     const uint32_t y = y0 + e;
                     while (nxt == y && qn < nseg) {
+                        uint32_t own[NB];
 #pragma unroll
-                        for (int q = 0; q < NB; q++) gs.hcnt[GS::at(NB, q, qn)] = cnt.word(gs, q);
+                        for (int q = 0; q < NB; q++) own[q] = cnt.word(gs, q);
+                        GS::store(gs.hcnt, qn, own);
                         dc = group_discr(a, d, cmod, gs.msz[qn]);
                         nxt = gs.hpos[++qn];
                     }
@@ -671,10 +704,12 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
         auto before = [&](uint32_t q, uint32_t y, uint32_t (&p)[NH]) {  // counts before head q at y
             const bool inside = y < end && q < nseg;
             const uint32_t t = inside ? y / k : 0u;
+            uint32_t own[NB];
+            GS::load(gs.hcnt, inside ? q : 0u, own);
 #pragma unroll
             for (int i = 0; i < NH; i++) {
                 const uint32_t w = __shfl_sync(0xffffffffu, wpre[i], t >> 5);
-                p[i] = inside ? w + gs.col[i][t] + widen_pair<M>(gs.hcnt[GS::at(NB, i / 2, q)], i) : tot[i];
+                p[i] = inside ? w + gs.col[i][t] + widen_pair<M>(own[i / 2], i) : tot[i];
             }
         };
         before(tid, hq, p0);
@@ -682,14 +717,14 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
         const uint64_t s = static_cast<uint64_t>(h) + tid;
         uint32_t off = 0;
         if (mine) {
+            uint32_t cur[NH];
 #pragma unroll
             for (int i = 0; i < NH; i++) {
                 const uint32_t n = p1[i] - p0[i];  // each 16-bit field is no smaller
                 const uint32_t n0 = n & 0xffffu, n1 = n >> 16;
                 const uint32_t o0 = off, o1 = off + n0;
                 off = o1 + n1;
-                gs.hpre[GS::at(NH, i, tid)] = p0[i];
-                gs.hcur[GS::at(NH, i, tid)] = (hq + o0) | ((hq + o1) << 16);
+                cur[i] = (hq + o0) | ((hq + o1) << 16);
                 if (a.seg_sizes != nullptr) {
                     if (2u * i < a.m) a.seg_sizes[s * a.m + 2 * i] = n0;
                     if (2u * i + 1u < a.m) a.seg_sizes[s * a.m + 2 * i + 1] = n1;
@@ -699,6 +734,8 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                     if (n1 > 0u) a.headflags[as + hq + o1] = n1;
                 }
             }
+            GS::store(gs.hpre, tid, p0);
+            GS::store(gs.hcur, tid, cur);
         }
     }
     // the output image is about to be rewritten: the previous group's bulk store
@@ -713,10 +750,11 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
         GroupCursors<M, THREADS> cur;
         cur.init(gs);
         if (qn > 0u) {
+            uint32_t first[NH], before[NH];
+            GS::load(gs.hcur, qn - 1u, first);
+            GS::load(gs.hpre, qn - 1u, before);
 #pragma unroll
-            for (int i = 0; i < NH; i++)
-                cur.set(gs, i, gs.hcur[GS::at(NH, i, qn - 1u)] +
-                                   (inc[i] - gs.hpre[GS::at(NH, i, qn - 1u)]));
+            for (int i = 0; i < NH; i++) cur.set(gs, i, first[i] + (inc[i] - before[i]));
         }
         for (uint32_t j = 0; j < nq; j++) {
             const uint32_t y0 = lo + j * VE;
@@ -731,8 +769,10 @@ __device__ __forceinline__ void seg_group_cta(const SegArgs& a, const D& d, cons
                 for (uint32_t e = 0; e < VE; e++) {
                     const uint32_t y = y0 + e;
                     while (nxt == y && qn < nseg) {
+                        uint32_t first[NH];
+                        GS::load(gs.hcur, qn, first);
 #pragma unroll
-                        for (int i = 0; i < NH; i++) cur.set(gs, i, gs.hcur[GS::at(NH, i, qn)]);
+                        for (int i = 0; i < NH; i++) cur.set(gs, i, first[i]);
                         dc = group_discr(a, d, cmod, gs.msz[qn]);
                         nxt = gs.hpos[++qn];
                     }
